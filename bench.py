@@ -1,13 +1,13 @@
 """Benchmark: particle-steps/s of the particle side of a PIC step on B200.
 
-One step = 5 fused LSRK4 stages (velocity, monomial interpolation, Lorentz
+One step = 5 LSRK4 stages in one kernel (velocity, monomial interpolation, Lorentz
 force, RK update, element relocation) + one deposition of rho and j onto the
 DG nodes (+ the element sort of the store). Default workload: config2 --
 32x32x128 cubes x 6 jittered tets (786,432 tets), order 3 (Np = 20,
 15.7M nodes), 16M electrons in an r < 0.25 cm beam, shape-function
 deposition with radius 0.08 cm, static Bz + 8 seeded Fourier modes of E and
-B; FP64 plain form. Inputs are far larger than L2 (3.5 GB of particle state
-moved per stage), so no L2 flush is needed between steps.
+B; FP64 plain form. Inputs are far larger than L2 (2.7 GB of particle state
+moved per step), so no L2 flush is needed between steps.
 
 Usage: python bench.py [--gpus N] [--steps K] [--warmup W] [--impl reference]
 With N > 1 (torchrun), every rank advances its own 16M particles (weak
@@ -167,7 +167,6 @@ MEASURED_TRAFFIC = {
         "tc_deposit_kernel<0, 0>": 1486009600 + 119841792,
         "tc_deposit_kernel<1, 1>": 1075521536 + 520001792,
         "deposit_groups_kernel<1, 1, 2>": 166834674176 + 130093312,
-        "lsrk_stage_mixed_kernel<3>": 2012872448 + 1545450240,
     }
 }
 
@@ -249,11 +248,12 @@ def form_accuracy(m, s, fields, dt, torch, steps=5):
         x, p, el = s.x.clone(), s.p.clone(), s.el.clone()
         kx = torch.zeros_like(x)
         kp = torch.zeros_like(p)
-        for t in range(stages):
-            _lib.check(m.lib.prt_lsrk_stage(
-                m.pusher.handle, m.workspace, x.shape[1], x.data_ptr(), p.data_ptr(),
-                s.q.data_ptr(), s.m.data_ptr(), el.data_ptr(), kx.data_ptr(), kp.data_ptr(), fp,
-                LSRK4_A[t % 5], LSRK4_B[t % 5], dt, c, prec, stream))
+        coef = m.pusher.field_coefficients(fp, prec)
+        _lib.check(m.lib.prt_lsrk_steps(
+            m.pusher.handle, m.workspace, x.shape[1], x.data_ptr(), p.data_ptr(),
+            s.q.data_ptr(), s.m.data_ptr(), el.data_ptr(), kx.data_ptr(), kp.data_ptr(),
+            coef.data_ptr(), fp, prec, (C.c_double * 5)(*LSRK4_A), (C.c_double * 5)(*LSRK4_B),
+            5, stages, dt, c, None, None, None, stream))
         return x, p, el, kp
 
     kp64 = run(0, 1)[3]
@@ -925,7 +925,9 @@ def main():
     avg_gather64 = gms64 / max(gk64, 1)
     achieved64 = 15.0 * pairs / (avg_gather64 * 1e-3) / 1e12
     sms, sk = kernel["lsrk_stage"]
-    stage_gbs = 216.0 * n / (sms / max(sk, 1) * 1e-3) / 1e9
+    # per step: x, p read and written (96 B), q, m (16), element (8), the
+    # residuals written (48)
+    stage_gbs = 168.0 * n / (sms / max(sk, 1) * 1e-3) / 1e9
     algorithmic = (f"15 flops x {pairs} (particle, distinct node position) pairs within the "
                    f"radius per launch ({node_pairs} (particle, node) pairs over all DG nodes; "
                    f"coincident nodes are evaluated once; {evaluated} pairs evaluated after "
@@ -949,11 +951,12 @@ def main():
                             "rate (cuBLAS SGEMM, TF32 off, measured in this run): the work "
                             "the CUDA-core form of this deposition does per pair"},
                 "normalize_pass_ms": avg_norm,
-                "secondary": {"bound": "hbm", "kernel": "lsrk_stage_mixed_kernel<3>",
+                "secondary": {"bound": "hbm", "kernel": "lsrk_steps_kernel (five stages, FP32 field "
+                                                        "coefficients)",
                               "achieved": stage_gbs, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                               "frac": stage_gbs / peaks["hbm_gbs"],
-                              "traffic": measured_traffic(args, "lsrk_stage_mixed_kernel<3>"),
-                              "algorithmic": "216 B per particle per stage",
+                              "traffic": None,
+                              "algorithmic": "168 B per particle per step",
                               "peak_source": src}}
     fp64_block = {
         "value": value64, "unit": METRIC, "ms_per_step": ms64 / args.steps,
@@ -972,8 +975,8 @@ def main():
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "f16/i8 tensor + f32 + f64 (mixed: split-FP16 tensor-core shape scores, "
                      "23-bit integer weights (three digits) summed exactly on the int8 tensor cores, FP64 "
-                     "per-node combine and normalisation; split-BF16 tensor-core Lagrange "
-                     "values; FP64 state/force/locate)",
+                     "per-node combine and normalisation; FP32 fields from per-element "
+                     "monomial coefficients; FP64 state/force/locate)",
             "data": "synthetic (seeded mesh, particles and fields of the workload)",
             "config": {"workload": f"{args.workload}: {w.mesh.element_count} tets order "
                                    f"{w.order}, {n} particles/GPU, shape radius "
@@ -983,7 +986,7 @@ def main():
                        "particles_per_gpu": n, "elements": w.mesh.element_count,
                        "nodes": nn, "order": w.order, "form": "mixed",
                        "depositor": args.depositor,
-                       "l2": f"inputs larger than L2 ({216 * n / 1e9:.1f} GB particle state per stage)",
+                       "l2": f"inputs larger than L2 ({168 * n / 1e9:.1f} GB particle state per step)",
                        "parallelism": f"particles sharded over {world} GPU(s) (z slabs of "
                                       "the beam), NCCL all-reduce of the integer digit sums "
                                       "per node position" if world > 1 else "1 GPU"},
@@ -996,8 +999,9 @@ def main():
             "accuracy_mixed_vs_fp64": accuracy}
     # libprt's own kernels in the timed region of the headline form (CUB's
     # radix-sort kernels not counted): per sort iota + 5 permutation gathers
-    # (x, p, q, m, ids; the residuals are dead at a step boundary); per RK
-    # stage one fused kernel; per deposition bin keys, bin starts, payload,
+    # (x, p, q, m, ids; the residuals are dead at a step boundary); per step one
+    # kernel for the five RK stages (and one per call for the field
+    # coefficients, not counted); per deposition bin keys, bin starts, payload,
     # the tile work estimate, charges, charge scale, charge digits, the
     # deposition pass and the expansion to nodes (9), and with the
     # normalising depositor position weights, their maximum, scale and

@@ -204,6 +204,35 @@ int prt_lsrk_stage(const prt_pusher *pusher, prt_workspace *ws, int64_t n,
                    double rk_b, double dt, double vacuum_c, int32_t precision,
                    void *stream);
 
+/* Per-element monomial coefficients of the six nodal fields (NULL: zero), the
+ * form in which prt_lsrk_steps reads them:
+ * coefficients[e][k][j] = sum_i fields[k][e Np + i] W[i][j], with
+ * l_i = sum_j W[i][j] m_j the element's Lagrange polynomials
+ * (push_monomial.hpp:155-210), rows padded with zeros to an even count. FP64,
+ * or for PRT_PRECISION_MIXED rounded to FP32 with rows padded to a multiple of
+ * four; _bytes gives the size. The buffer must be 16-byte aligned. */
+int prt_field_coefficients_bytes(const prt_pusher *pusher, int32_t precision, int64_t *bytes);
+int prt_field_coefficients(const prt_pusher *pusher, const double *const fields[6],
+                           int32_t precision, void *coefficients, void *stream);
+
+/* `stages` low-storage RK stages of prt_lsrk_stage in one launch, with the
+ * fields standing still (PicMethod.advance_state under the 2N-storage RK
+ * update, cloud.py:172-186, 554-603): stage t uses rk_a[t % rk_count] and
+ * rk_b[t % rk_count] (HOST arrays, rk_count <= 8). With `coefficients` (from
+ * prt_field_coefficients of the same precision) the fields come from those
+ * and `fields` may be NULL; without, from the nodal `fields` in FP64.
+ * A first stage with rk_a[0] = 0 does not read kx and kp; they are written at
+ * the end. tape_x, tape_p [stages + 1][3][n] and tape_el [stages + 1][n] (all
+ * or none NULL) receive the state after stage t in slot t + 1. */
+int prt_lsrk_steps(const prt_pusher *pusher, prt_workspace *ws, int64_t n,
+                   double *positions, double *momenta, const double *charges,
+                   const double *masses, uint32_t *elements, double *kx,
+                   double *kp, const void *coefficients,
+                   const double *const fields[6], int32_t precision,
+                   const double *rk_a, const double *rk_b, int32_t rk_count,
+                   int32_t stages, double dt, double vacuum_c, double *tape_x,
+                   double *tape_p, uint32_t *tape_el, void *stream);
+
 /* ----------------------------------------------------------- deposition --- */
 
 /* polynomial_shape_function(radius, dimensions, alpha) (tools.hpp:514-556,

@@ -148,6 +148,11 @@ SIGNATURES = {
     "prt_forces": (_i32, [_vp, _i64, _vp, _vp, _vp, _vp, C.POINTER(_vp), _vp, _vp, _vp]),
     "prt_lsrk_stage": (_i32, [_vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                               C.POINTER(_vp), _d, _d, _d, _d, _i32, _vp]),
+    "prt_field_coefficients_bytes": (_i32, [_vp, _i32, _i64p]),
+    "prt_field_coefficients": (_i32, [_vp, C.POINTER(_vp), _i32, _vp, _vp]),
+    "prt_lsrk_steps": (_i32, [_vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
+                              C.POINTER(_vp), _i32, _dp, _dp, _i32, _i32, _d, _d, _vp, _vp,
+                              _vp, _vp]),
     "prt_deposit_shape": (_i32, [_vp, _vp, _i32, ShapeFunctionDesc, _dp, _i64, _vp, _vp,
                                  _vp, _vp, _vp, _vp, _i32, C.POINTER(DepositStats), _vp]),
     "prt_deposit_shape_noalloc": (_i32, [_vp, ShapeFunctionDesc, _i64, _vp, _vp, _vp, _vp,

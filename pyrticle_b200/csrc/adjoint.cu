@@ -63,26 +63,26 @@ __global__ void __launch_bounds__(256, ORDER >= 4 ? 2 : 3)
                              double b, double dt, double c, DevStatus *st) {
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   unsigned ctr[4] = {0, 0, 0, 0};
+  const uint32_t e = i < n ? el_in[i] : PRT_INVALID;
+  double xx[3] = {0, 0, 0}, pp[3] = {0, 0, 0};
   if (i < n) {
-    const uint32_t e = el_in[i];
-    double xx[3] = {x_in[i], x_in[n + i], x_in[2 * n + i]};
-    double pp[3] = {p_in[i], p_in[n + i], p_in[2 * n + i]};
-    uint32_t ne = e;
-    if (e != PRT_INVALID) {
-      int err = 0;
-      const uint32_t r = stage_particle<ORDER>(M, L, F, e, xx, pp, q[i], mass[i], kx, kp, n,
-                                               i, a, b, dt, c, ctr, &err);
-      if (err)
-        record_error(st, err, i);
-      else
-        ne = r;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      xx[d] = x_in[d * n + i];
+      pp[d] = p_in[d * n + i];
     }
+  }
+  int err = 0;
+  const uint32_t ne = stage_particle<ORDER>(M, L, F, e != PRT_INVALID, e, xx, pp, q, mass, kx,
+                                            kp, n, i, a, b, dt, c, ctr, &err);
+  if (i < n) {
+    if (err) record_error(st, err, i);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       x_out[d * n + i] = xx[d];
       p_out[d * n + i] = pp[d];
     }
-    el_out[i] = ne;
+    el_out[i] = err ? e : ne;
   }
   flush_counters(st, ctr);
 }

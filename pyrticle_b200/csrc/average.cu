@@ -135,14 +135,22 @@ __global__ void __launch_bounds__(256)
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   unsigned ctr[4] = {0, 0, 0, 0};
   const uint32_t e = i < n ? el[i] : PRT_INVALID;
-  if (e != PRT_INVALID) {
-    double xx[3] = {x[i], x[n + i], x[2 * n + i]};
-    double pp[3] = {p[i], p[n + i], p[2 * n + i]};
-    double v[3];
+  const bool live = e != PRT_INVALID;
+  double xx[3] = {0, 0, 0}, pp[3] = {0, 0, 0}, r[3];
+  if (live) {
+    double v[3], f[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      xx[d] = x[d * n + i];
+      pp[d] = p[d * n + i];
+      f[d] = forces[d * n + i];
+    }
     velocity_exact(pp[0], pp[1], pp[2], mass[i], c, v[0], v[1], v[2]);
-    const double f[3] = {forces[i], forces[n + i], forces[2 * n + i]};
-    int err = 0;
-    const uint32_t ne = update_particle(M, e, f, v, xx, pp, kx, kp, n, i, a, b, dt, ctr, &err);
+    update_particle(f, v, xx, pp, kx, kp, n, i, a, b, dt);
+  }
+  int err = 0;
+  const uint32_t ne = relocate(M, live, xx, pp, e, ctr, &err, r);
+  if (live) {
     if (err) record_error(st, err, i);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {

@@ -300,11 +300,53 @@ extern "C" int prt_get_velocities(int64_t n, const double *p, const double *m, d
   return PRT_OK;
 }
 
+// Particles of a warp that share their element bin (sorted stores) walk its
+// list together, every lane testing its own point against one element at a
+// uniform address; the others are searched by the warp one after the other
+// (search_lists). From eight sharers on the common walk is the cheaper one:
+// 300,000 positions took 99 us sorted and 393 us unsorted with every lane on
+// its own, 165 and 218 us with the warp's search alone.
+constexpr int SHARED_BIN = 8;
 __global__ void find_global_kernel(DevMesh M, long long n, const double *__restrict__ x,
                                    uint32_t *__restrict__ el) {
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  el[i] = find_global(M, x[i], x[n + i], x[2 * n + i]);
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const bool valid = i < n;
+  double xx[3] = {0, 0, 0};
+  uint32_t row = 0, e = PRT_INVALID;
+  if (valid) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) xx[d] = x[d * n + i];
+    row = element_bin(M, xx);
+  }
+  bool open = valid;
+  unsigned todo = __ballot_sync(0xffffffffu, valid);
+  while (todo) {
+    const uint32_t rs = __shfl_sync(0xffffffffu, row, __ffs(todo) - 1);
+    const bool peer = valid && row == rs;
+    const unsigned peers = __ballot_sync(0xffffffffu, peer);
+    todo &= ~peers;
+    if (__popc(peers) < SHARED_BIN) continue;
+    if (peer) {
+      const uint32_t s = __ldg(M.bin_starts + rs), t = __ldg(M.bin_starts + rs + 1);
+      for (uint32_t k = s; k < t; k += 4) {
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+          if (k + u >= t) break;
+          const uint32_t c = __ldg(M.bin_elements + k + u);
+          double r[3];
+          const bool in = in_element(M, c, xx[0], xx[1], xx[2], r);
+          if (open && in) {
+            e = c;
+            open = false;
+          }
+        }
+        if (!__any_sync(peers, open)) break;
+      }
+      open = false;
+    }
+  }
+  const uint32_t g = search_lists(M, open, row, M.bin_starts, M.bin_elements, xx);
+  if (valid) el[i] = open ? g : e;
 }
 
 extern "C" int prt_find_containing_elements(const prt_mesh *mesh, int64_t n,
@@ -321,22 +363,28 @@ extern "C" int prt_find_containing_elements(const prt_mesh *mesh, int64_t n,
 __global__ void update_elements_kernel(DevMesh M, long long n, double *__restrict__ x,
                                        const double *__restrict__ p,
                                        uint32_t *__restrict__ el, DevStatus *st) {
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   unsigned ctr[4] = {0, 0, 0, 0};
-  uint32_t prev = i < n ? el[i] : PRT_INVALID;
-  if (prev != PRT_INVALID) {
-    double x0 = x[i], x1 = x[n + i], x2 = x[2 * n + i];
-    int err = 0;
-    bool wrapped;
-    uint32_t ne = relocate(M, x0, x1, x2, p[i], p[n + i], p[2 * n + i], prev, ctr, &err,
-                           &wrapped);
+  const uint32_t prev = i < n ? el[i] : PRT_INVALID;
+  const bool live = prev != PRT_INVALID;
+  double xx[3] = {0, 0, 0}, pp[3] = {0, 0, 0}, r[3];
+  if (live) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      xx[d] = x[d * n + i];
+      pp[d] = p[d * n + i];
+    }
+  }
+  int err = 0;
+  bool wrapped;
+  const uint32_t ne = relocate(M, live, xx, pp, prev, ctr, &err, r, &wrapped);
+  if (live) {
     if (err) {
       record_error(st, err, i);
     } else {
       if (wrapped) {
-        x[i] = x0;
-        x[n + i] = x1;
-        x[2 * n + i] = x2;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) x[d * n + i] = xx[d];
       }
       el[i] = ne;
     }
@@ -414,12 +462,19 @@ __global__ void __launch_bounds__(256, ORDER >= 4 ? 2 : PRT_STAGE_MIN_BLOCKS)
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   unsigned ctr[4] = {0, 0, 0, 0};
   const uint32_t e = i < n ? el[i] : PRT_INVALID;
-  if (e != PRT_INVALID) {
-    double xx[3] = {x[i], x[n + i], x[2 * n + i]};
-    double pp[3] = {p[i], p[n + i], p[2 * n + i]};
-    int err = 0;
-    const uint32_t ne = stage_particle<ORDER>(M, L, F, e, xx, pp, q[i], mass[i], kx, kp, n, i,
-                                              a, b, dt, c, ctr, &err);
+  const bool live = e != PRT_INVALID;
+  double xx[3] = {0, 0, 0}, pp[3] = {0, 0, 0};
+  if (live) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      xx[d] = x[d * n + i];
+      pp[d] = p[d * n + i];
+    }
+  }
+  int err = 0;
+  const uint32_t ne = stage_particle<ORDER>(M, L, F, live, e, xx, pp, q, mass, kx, kp, n, i, a,
+                                            b, dt, c, ctr, &err);
+  if (live) {
     if (err) record_error(st, err, i);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {

@@ -90,28 +90,28 @@ static Lagrange<ORDER> make_lagrange(const prt_pusher *P) {
   return L;
 }
 
-// RK update and relocation from a force f at (x, p): k = a k + dt (v(p), f),
-// (x, p) += b k (residuals kx, kp [3][n] at index i, read and written before
-// the relocation), then the new containing element (PRT_INVALID if the
-// particle left the mesh; *err on a locate error).
-__device__ __forceinline__ uint32_t update_particle(const DevMesh &M, uint32_t e,
-                                                    const double f[3], const double v[3],
-                                                    double xx[3], double pp[3],
-                                                    double *__restrict__ kx,
-                                                    double *__restrict__ kp, long long n,
-                                                    long long i, double a, double b,
-                                                    double dt, unsigned ctr[4], int *err) {
+// RK update of one particle: k = a k + dt f, y += b k (rounded as written).
+__device__ __forceinline__ void rk_update(double a, double b, double dt, double f, double &k,
+                                          double &y) {
+  k = __dadd_rn(__dmul_rn(a, k), __dmul_rn(dt, f));
+  y = __dadd_rn(y, __dmul_rn(b, k));
+}
+
+// The same from a force f and velocity v, with the residuals kx, kp [3][n] at
+// index i.
+__device__ __forceinline__ void update_particle(const double f[3], const double v[3],
+                                                double xx[3], double pp[3],
+                                                double *__restrict__ kx,
+                                                double *__restrict__ kp, long long n,
+                                                long long i, double a, double b, double dt) {
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const double kxd = __dadd_rn(__dmul_rn(a, kx[d * n + i]), __dmul_rn(dt, v[d]));
-    const double kpd = __dadd_rn(__dmul_rn(a, kp[d * n + i]), __dmul_rn(dt, f[d]));
+    double kxd = kx[d * n + i], kpd = kp[d * n + i];
+    rk_update(a, b, dt, v[d], kxd, xx[d]);
+    rk_update(a, b, dt, f[d], kpd, pp[d]);
     kx[d * n + i] = kxd;
     kp[d * n + i] = kpd;
-    xx[d] = __dadd_rn(xx[d], __dmul_rn(b, kxd));
-    pp[d] = __dadd_rn(pp[d], __dmul_rn(b, kpd));
   }
-  bool wrapped;
-  return relocate(M, xx[0], xx[1], xx[2], pp[0], pp[1], pp[2], e, ctr, err, &wrapped);
 }
 
 // Lorentz force F = q E + v x (q B) in the reference's operation order
@@ -129,24 +129,22 @@ __device__ __forceinline__ void lorentz_force(double charge, const double ef[6],
   f[2] = __dadd_rn(elf[2], __dsub_rn(__dmul_rn(v[0], qb[1]), __dmul_rn(v[1], qb[0])));
 }
 
-// The stage after the interpolation: Lorentz force from the fields ef at x,
-// RK update, relocation (shared by the FP64 stage and the mixed-precision
-// stage, whose fields come from the tensor cores).
-__device__ __forceinline__ uint32_t stage_from_fields(const DevMesh &M, uint32_t e,
-                                                      const double ef[6], double xx[3],
-                                                      double pp[3], double charge, double mass,
-                                                      double *__restrict__ kx,
-                                                      double *__restrict__ kp, long long n,
-                                                      long long i, double a, double b,
-                                                      double dt, double c, unsigned ctr[4],
-                                                      int *err) {
+// The stage after the interpolation: Lorentz force from the fields ef at x
+// and the RK update; the caller relocates (a warp at a time, common.cuh).
+__device__ __forceinline__ void stage_from_fields(const double ef[6], double xx[3],
+                                                  double pp[3], double charge, double mass,
+                                                  double *__restrict__ kx,
+                                                  double *__restrict__ kp, long long n,
+                                                  long long i, double a, double b, double dt,
+                                                  double c) {
   double v[3], f[3];
   velocity_exact(pp[0], pp[1], pp[2], mass, c, v[0], v[1], v[2]);
   lorentz_force(charge, ef, v, f);
-  return update_particle(M, e, f, v, xx, pp, kx, kp, n, i, a, b, dt, ctr, err);
+  update_particle(f, v, xx, pp, kx, kp, n, i, a, b, dt);
 }
 
-// One low-storage RK stage for one live particle in element e:
+// One low-storage RK stage of a warp's particles (live: this lane has one, in
+// element e):
 //   v = v(p), F = q E(x) + v x (q B(x)), k = a k + dt (v, F), (x, p) += b k,
 // then relocation. Updates xx, pp in place and the residuals kx, kp [3][n]
 // at index i (read and written before the relocation, which keeps them out
@@ -154,15 +152,20 @@ __device__ __forceinline__ uint32_t stage_from_fields(const DevMesh &M, uint32_t
 // particle left the mesh); *err is set on a locate error.
 template <int ORDER>
 __device__ __forceinline__ uint32_t stage_particle(const DevMesh &M, const Lagrange<ORDER> &L,
-                                                   const Fields6 &F, uint32_t e, double xx[3],
-                                                   double pp[3], double charge, double mass,
+                                                   const Fields6 &F, bool live, uint32_t e,
+                                                   double xx[3], double pp[3],
+                                                   const double *__restrict__ q,
+                                                   const double *__restrict__ mass,
                                                    double *__restrict__ kx,
                                                    double *__restrict__ kp, long long n,
                                                    long long i, double a,
                                                    double b, double dt, double c,
                                                    unsigned ctr[4], int *err) {
-  double ef[6];
-  interpolate_fields<ORDER>(M, L, F, e, xx[0], xx[1], xx[2], ef);
-  return stage_from_fields(M, e, ef, xx, pp, charge, mass, kx, kp, n, i, a, b, dt, c, ctr,
-                           err);
+  if (live) {
+    double ef[6];
+    interpolate_fields<ORDER>(M, L, F, e, xx[0], xx[1], xx[2], ef);
+    stage_from_fields(ef, xx, pp, q[i], mass[i], kx, kp, n, i, a, b, dt, c);
+  }
+  double r[3];
+  return relocate(M, live, xx, pp, e, ctr, err, r);
 }

@@ -283,9 +283,12 @@ __global__ void __launch_bounds__(MX_BLOCK)
       double ef[6];
 #pragma unroll
       for (int k = 0; k < 6; ++k) ef[k] = (double)ef32[k];
-      int err = 0;
-      const uint32_t ne = stage_from_fields(M, e, ef, xx, pp, q[i], mass[i], kx, kp, n, i, a,
-                                            b, dt, c, ctr, &err);
+      stage_from_fields(ef, xx, pp, q[i], mass[i], kx, kp, n, i, a, b, dt, c);
+    }
+    int err = 0;
+    double r[3];
+    const uint32_t ne = relocate(M, live, xx, pp, e, ctr, &err, r);
+    if (live) {
       if (err) record_error(st, err, i);
 #pragma unroll
       for (int d = 0; d < 3; ++d) {

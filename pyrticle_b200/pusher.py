@@ -73,6 +73,36 @@ class MonomialParticlePusher(Pusher):
             kp.data_ptr(), fptrs, a, b, dt, c, precision,
             C.c_void_p(torch.cuda.current_stream().cuda_stream)), "prt_lsrk_stage")
 
+    def field_coefficients(self, fptrs, precision=0):
+        """Per-element monomial coefficients of the fields behind ``fptrs``
+        (prt_field_coefficients), a device buffer for ``lsrk_steps``."""
+        nbytes = C.c_int64()
+        _lib.check(self.lib.prt_field_coefficients_bytes(self.handle, precision,
+                                                         C.byref(nbytes)),
+                   "prt_field_coefficients_bytes")
+        out = torch.empty((nbytes.value,), dtype=torch.uint8, device=self.method.dev)
+        _lib.check(self.lib.prt_field_coefficients(
+            self.handle, fptrs, precision, out.data_ptr(),
+            C.c_void_p(torch.cuda.current_stream().cuda_stream)), "prt_field_coefficients")
+        return out
+
+    def fused_stages(self):
+        """Whether whole steps may run through ``lsrk_steps``: not where a
+        subclass or an instance brings a stage of its own."""
+        return getattr(self.lsrk_stage, "__func__", None) is MonomialParticlePusher.lsrk_stage
+
+    def lsrk_steps(self, state, fptrs, coefficients, kx, kp, rk_a, rk_b, stages, dt, c,
+                   precision=0):
+        """``stages`` RK stages of the whole store in one launch
+        (prt_lsrk_steps), from ``coefficients`` or else the nodal fields."""
+        m = self.method
+        _lib.check(self.lib.prt_lsrk_steps(
+            self.handle, m.workspace, len(state), state.x.data_ptr(), state.p.data_ptr(),
+            state.q.data_ptr(), state.m.data_ptr(), state.el.data_ptr(), kx.data_ptr(),
+            kp.data_ptr(), None if coefficients is None else coefficients.data_ptr(), fptrs,
+            precision, rk_a, rk_b, len(rk_a), stages, dt, c, None, None, None,
+            C.c_void_p(torch.cuda.current_stream().cuda_stream)), "prt_lsrk_steps")
+
     def field_pointers(self, fields):
         """Pointer array for six device field components (None = zero)."""
         arr = (C.c_void_p * 6)()
