@@ -166,7 +166,6 @@ MEASURED_TRAFFIC = {
     "config2": {
         "tc_deposit_kernel<0, 0>": 1486009600 + 119841792,
         "tc_deposit_kernel<1, 1>": 1075521536 + 520001792,
-        "deposit_groups_kernel<1, 1, 2>": 166834674176 + 130093312,
     }
 }
 
@@ -961,10 +960,10 @@ def main():
     fp64_block = {
         "value": value64, "unit": METRIC, "ms_per_step": ms64 / args.steps,
         "kernel_ms_per_step": {k: v[0] / args.steps for k, v in kernel64.items()},
-        "roofline": {"bound": "fp64", "kernel": "deposit_groups_kernel (deposition, FP64)",
+        "roofline": {"bound": "fp64", "kernel": "deposit_blocks_kernel (deposition, FP64)",
                      "achieved": achieved64, "peak": fp64, "unit": "TFLOP/s",
                      "frac": achieved64 / fp64,
-                     "traffic": measured_traffic(args, "deposit_groups_kernel<1, 1, 2>"),
+                     "traffic": None,
                      "peak_source": "cuBLAS DGEMM 8192^3 measured in this run",
                      "algorithmic": algorithmic + f"; {avg_gather64:.3f} ms per launch"},
         "form": ("plain form: FP64 throughout" +

@@ -147,6 +147,7 @@ extern "C" int prt_mesh_destroy(prt_mesh *m) {
                         P.wide_starts, P.wide_spheres};
   for (const void *p : ptrs)
     if (p) cudaFree((void *)p);
+  prt_free_tiles(&m->positions.tiles);
   delete m;
   return PRT_OK;
 }

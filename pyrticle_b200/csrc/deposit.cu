@@ -13,19 +13,19 @@
 // positions, which needs no floating-point atomics and is deterministic:
 //
 //   1. set-up (host, once per mesh): merge coincident nodes into positions,
-//      order them along a Morton curve, cut the order into warp groups
-//      (<= 32 positions at Morton cells of ~24) and wide groups (<= 64, two
-//      positions per lane), each with its bounding sphere;
+//      order them along a Morton curve, cut them by recursive bisection into
+//      tiles of 32 in blocks of four (the FP64 sums' targets, tiles.cuh), and
+//      cut the Morton order into position groups (<= 32, and wide ones <= 64
+//      for mixed_simt) with bounding spheres;
 //   2. per call: bin the particles (bin width radius/2), radix sort by bin,
 //      pack a 64-byte payload per particle in bin order; estimate each
-//      group's work (the particles of its bin rows) and launch the groups
+//      block's work (the particles of its bin rows) and launch the blocks
 //      heaviest first;
-//   3. one warp per group, warps independent: the warp streams the
-//      particles of the bin rows within the radius of its box straight from
-//      L2, culls them against the box grown by the radius, appends the
-//      survivors to a private shared-memory ring (ballot), and every 32
-//      entries the lanes walk the batch with a branch-free weight, two
-//      positions per lane; rho, j accumulate in a fixed order;
+//   3. a block per four tiles stages the particles near its box in shared
+//      memory and each warp sums those near its tile (tiles.cuh), in a fixed
+//      order; mixed_simt: one warp per wide group, which streams the particles
+//      of the bin rows within the radius of its box, culls them into a ring
+//      and walks it two positions per lane;
 //   4. expand: every node takes its position's values.
 //
 // The chosen form's tensor-core deposition (deposit_tc.cu) shares steps 1,
@@ -45,7 +45,9 @@
 #include <vector>
 
 #include "binning.cuh"
+#include "bisect.cuh"
 #include "gather.cuh"
+#include "tiles.cuh"
 
 namespace prt_dep {
 
@@ -184,35 +186,20 @@ using namespace prt_dep;
 
 constexpr int WARPS = BLOCK / 32;
 
-// resident CTAs per SM the group kernel is compiled for (register budget)
-#ifndef PRT_GATHER_MIN_BLOCKS
-#define PRT_GATHER_MIN_BLOCKS 6
-#endif
-// the same for the two-positions-per-lane form (twice the accumulators)
-#ifndef PRT_GATHER_MIN_BLOCKS_WIDE
-#define PRT_GATHER_MIN_BLOCKS_WIDE 4
-#endif
 // mixed form, wide groups: 6 CTAs (80 registers, no spills) measured best
 // with the heaviest groups first: 8 CTAs cost ~20% on dense bunches
 // (config4) and 4 CTAs ~15% on config2
 #ifndef PRT_MIXED_MIN_BLOCKS_WIDE
 #define PRT_MIXED_MIN_BLOCKS_WIDE 6
 #endif
-// positions per lane of the FP64 and mixed deposition (2: wide groups)
-#ifndef PRT_FP64_PPL
-#define PRT_FP64_PPL 2
-#endif
+// positions per lane of the mixed_simt deposition (2: wide groups)
 #ifndef PRT_MIXED_PPL
 #define PRT_MIXED_PPL 2
 #endif
-// unrolling of the full-batch loops (two entries per step)
-#ifndef PRT_FP64_UNROLL
-#define PRT_FP64_UNROLL 4
-#endif
+// unrolling of its full-batch loop
 #ifndef PRT_MIXED_UNROLL
 #define PRT_MIXED_UNROLL 4
 #endif
-constexpr int FP64_UNROLL = PRT_FP64_UNROLL;
 // launch the position groups heaviest first (1) or in Morton order (0)
 #ifndef PRT_DEPOSIT_HEAVY_FIRST
 #define PRT_DEPOSIT_HEAVY_FIRST 1
@@ -352,23 +339,26 @@ __device__ __forceinline__ void warp_box(const double *__restrict__ pos, uint32_
     }
 }
 
-// Work estimate per position group: the particles in the bin rows of its
-// sphere grown by the radius (periodic images ignored), keyed for a
+// Work estimate per position group or block of tiles (bounding spheres [.][4]
+// or boxes [.][6]): the particles in the bin rows of it grown by the radius (periodic images ignored), keyed for a
 // descending sort so that the heaviest groups start first and the light
 // ones fill the tail of the launch. Each group is still walked by one warp,
 // so the order changes no result.
-__global__ void group_work_kernel(long long ngroups, const double *__restrict__ gspheres,
+template <bool BOXES>
+__global__ void group_work_kernel(long long ngroups, const double *__restrict__ bounds,
                                   BinGrid G, const uint32_t *__restrict__ starts,
                                   double radius, uint32_t *__restrict__ work,
                                   uint32_t *__restrict__ ids) {
   const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (g >= ngroups) return;
-  const double r = gspheres[4 * g + 3] + radius;
   int lo[3], hi[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    lo[d] = max(0, min(G.dims[d] - 1, bin_floor(G, d, gspheres[4 * g + d] - r)));
-    hi[d] = max(0, min(G.dims[d] - 1, bin_floor(G, d, gspheres[4 * g + d] + r)));
+    // (a block of tiles: the box of its first)
+    const double c = bounds[(BOXES ? 6 * BW : 4) * g + d];
+    const double r = (BOXES ? bounds[6 * BW * g + 3 + d] : bounds[4 * g + 3]) + radius;
+    lo[d] = max(0, min(G.dims[d] - 1, bin_floor(G, d, c - r)));
+    hi[d] = max(0, min(G.dims[d] - 1, bin_floor(G, d, c + r)));
   }
   unsigned long long wsum = 0;
   for (int bz = lo[2]; bz <= hi[2]; ++bz)
@@ -380,178 +370,234 @@ __global__ void group_work_kernel(long long ngroups, const double *__restrict__ 
   ids[g] = (uint32_t)g;
 }
 
-// One warp per position group (<= 32 positions, one per lane), warps fully
-// independent (no block-level barrier). The warp streams the particles of
-// the bin rows within its sphere grown by the radius straight from L2/L1:
-// each lane tests one particle on the payload's first 32-byte sector
-// (x, y, z, q N); the survivors' weights are fetched and appended to the
-// warp's shared-memory ring (warp ballot); every 32 entries the lanes walk
-// the batch, two particles per iteration. Coordinates are relative to the
-// group centre c: r^2 = |u|^2 + |w|^2 - 2 u.w with u = x_position - c,
-// w = x_particle - c. Output out[4][npos]: rho, j_x, j_y, j_z per position.
-// In COUNT mode counters[0] receives the (particle, position) pairs within
-// the radius, counters[1] the (particle, node) pairs (positions weighted by
-// their node count) and counters[2] the evaluated pairs.
-template <bool ALPHA2, bool COUNT, int PPL = 1>
-__global__ void __launch_bounds__(BLOCK, PPL == 1 ? PRT_GATHER_MIN_BLOCKS : PRT_GATHER_MIN_BLOCKS_WIDE)
-    deposit_groups_kernel(const double *__restrict__ pos, long long ngroups,
-                          const uint32_t *__restrict__ gstarts,
-                          const double *__restrict__ gspheres,
-                          const uint32_t *__restrict__ run_starts, BinGrid G,
-                          DepParticles P, ShapeParams S, long long npos,
-                          double *__restrict__ out, unsigned long long *__restrict__ counters,
-                          const uint32_t *__restrict__ order = nullptr) {
-  // ring entries: (wx, wy), (wz, |w|^2), (q N, q N vx), (q N vy, q N vz)
-  __shared__ double2 ring[WARPS][4][RING];
-
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const long long gi = blockIdx.x * (long long)WARPS + wid;
-  if (gi >= ngroups) return;  // whole warp
-  const long long g = order ? (long long)order[gi] : gi;
-  const uint32_t p0 = gstarts[g];
-  const int npg = (int)(gstarts[g + 1] - p0);
-  double2(*R)[RING] = ring[wid];
-
-  const double c0 = gspheres[4 * g], c1 = gspheres[4 * g + 1], c2 = gspheres[4 * g + 2];
-  // lane holds positions p0 + lane + 32 h, h < PPL. With u = x_position - c
-  // and w = x_particle - c: a - r^2/a = (a - |u|^2/a) - |w|^2/a + (2/a) u.w,
-  // so per pair the weight base is three FMAs and an add: B + e + V . w
-  double V0[PPL], V1[PPL], V2[PPL], B[PPL];
-  bool live[PPL];
-  unsigned mult[PPL];
+// The plain deposition's sums (tiles.cuh): targets are node positions (or
+// brick points), sources the particles of the bin rows near a tile. FP64
+// operations per evaluated pair: four for a - r^2/a, one for its square, four
+// for rho and j (15 flops; the clamp is an integer maximum).
+struct TileSums {
+  double *__restrict__ out[4];
+};
+// The per-lane targets and sums of a warp's tile.
+template <int PER, bool ALPHA2, bool COUNT>
+struct DepositTargets {
+  double V[3][PER], B[PER], sum[4][PER];
+  unsigned hits[PER];
+  double alpha;
+  // rows PER tg .. of tile t, relative to c; rows past the tile's (npt) are
+  // never within the radius
+  __device__ __forceinline__ void load(const TilesDev &T, long long p0, int npt, int tg,
+                                       const double c[3], const ShapeWeight &S) {
+    alpha = S.alpha;
 #pragma unroll
-  for (int h = 0; h < PPL; ++h) {
-    live[h] = lane + 32 * h < npg;
-    V0[h] = V1[h] = V2[h] = B[h] = 0;
-    mult[h] = 0;
-    if (live[h]) {
-      const long long u = p0 + lane + 32 * h;
-      const double u0 = pos[3 * u] - c0, u1 = pos[3 * u + 1] - c1, u2 = pos[3 * u + 2] - c2;
-      B[h] = S.radius - (u0 * u0 + u1 * u1 + u2 * u2) * S.inv_radius;
-      V0[h] = 2 * u0 * S.inv_radius;
-      V1[h] = 2 * u1 * S.inv_radius;
-      V2[h] = 2 * u2 * S.inv_radius;
-      if (COUNT) mult[h] = run_starts[u + 1] - run_starts[u];
+    for (int h = 0; h < PER; ++h) {
+      const int row = PER * tg + h;
+      double u[3] = {0, 0, 0}, u2 = 0;
+      if (row < npt) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          u[d] = T.pos[3 * (p0 + row) + d] - c[d];
+          u2 = fma(u[d], u[d], u2);
+        }
+      }
+      B[h] = row < npt ? S.radius - u2 * S.inv_radius : -1e300;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) V[d][h] = 2 * u[d] * S.inv_radius;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) sum[k][h] = 0;
+      hits[h] = 0;
     }
   }
-
-  double r0[PPL], x0[PPL], y0[PPL], z0[PPL], r1[PPL], x1[PPL], y1[PPL], z1[PPL];
+  __device__ __forceinline__ void operator()(double w0, double w1, double w2, double e,
+                                             const double *v) {
 #pragma unroll
-  for (int h = 0; h < PPL; ++h) r0[h] = x0[h] = y0[h] = z0[h] = r1[h] = x1[h] = y1[h] = z1[h] = 0;
-  unsigned long long npairs = 0, nnode = 0, nevals = 0;
-
-  // shape weight from tr = a - r^2/a (zero beyond the radius)
-  // alpha = 2: (tr + |tr|)^2 = 4 max(tr, 0)^2 exactly (one add with an
-  // absolute-value operand and one multiply); the sums are scaled by 1/4 at
-  // the end, also exactly, so the result equals that of max(tr, 0)^2
-  auto weight = [&](double tr) -> double {
-    if (ALPHA2) {
-      const double t2 = tr + fabs(tr);
-      return t2 * t2;
+    for (int h = 0; h < PER; ++h) {
+      const double tr = fma(V[0][h], w0, fma(V[1][h], w1, fma(V[2][h], w2, B[h] + e)));
+      const double sw = shape_power<ALPHA2>(tr, alpha);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) sum[k][h] = fma(v[k], sw, sum[k][h]);
+      if (COUNT) hits[h] += __double2hiint(tr) >= 0;
     }
-    return tr > 0 ? pow(tr, S.alpha) : 0.0;
-  };
-  const double wscale = ALPHA2 ? 0.25 : 1.0;
-  // one ring entry against the lane's positions
-  auto pair = [&](const double2 p, const double2 q, const double2 wq, const double2 wv,
-                  double *r, double *x, double *y, double *z) {
+  }
+  // adds the tile's pairs, node pairs and evaluated pairs to counters[0..2]
+  __device__ __forceinline__ void count(const TilesDev &T, const uint32_t *run_starts,
+                                        long long p0, int npt, int tg,
+                                        unsigned long long evaluated,
+                                        unsigned long long *counters) const {
+    unsigned long long pairs = 0, nodes = 0;
 #pragma unroll
-    for (int h = 0; h < PPL; ++h) {
-      const double tr = fma(V0[h], p.x, fma(V1[h], p.y, fma(V2[h], q.x, B[h] + q.y)));
-      const double sw = weight(tr);
-      r[h] = fma(wq.x, sw, r[h]);
-      x[h] = fma(wq.y, sw, x[h]);
-      y[h] = fma(wv.x, sw, y[h]);
-      z[h] = fma(wv.y, sw, z[h]);
-      if (COUNT) {
-        const unsigned in = live[h] && tr >= 0;
-        npairs += in;
-        nnode += in * mult[h];
+    for (int h = 0; h < PER; ++h) {
+      pairs += hits[h];
+      if (hits[h] && run_starts) {
+        const uint32_t u = T.rows[p0 + PER * tg + h];
+        nodes += hits[h] * (unsigned long long)(run_starts[u + 1] - run_starts[u]);
       }
     }
-  };
-  int head = 0, count = 0;
-  // walks `k` ring entries from head (warp-uniform k)
-  auto drain = [&](int k) {
-    for (int i = 0; i < k; ++i) {
-      const int e = (head + i) & (RING - 1);
-      pair(R[0][e], R[1][e], R[2][e], R[3][e], r0, x0, y0, z0);
-    }
-    if (COUNT && lane == 0) nevals += (unsigned long long)k * (unsigned)npg;
-    head = (head + k) & (RING - 1);
-    count -= k;
-  };
-  // a full batch of 32 from head (0 or 32): constant offsets, two entries
-  // per step into two sets of accumulators
-  auto drain_full = [&]() {
-    const double2 *E0 = &R[0][head], *E1 = &R[1][head], *E2 = &R[2][head], *E3 = &R[3][head];
-#pragma unroll FP64_UNROLL
-    for (int i = 0; i < 32; i += 2) {
-      pair(E0[i], E1[i], E2[i], E3[i], r0, x0, y0, z0);
-      pair(E0[i + 1], E1[i + 1], E2[i + 1], E3[i + 1], r1, x1, y1, z1);
-    }
-    if (COUNT && lane == 0) nevals += 32ull * (unsigned)npg;
-    head = (head + 32) & (RING - 1);
-    count -= 32;
-  };
-
-  const double cc[3] = {c0, c1, c2};
-  double blo[3], bhi[3];
-  warp_box<PPL>(pos, p0, npg, lane, cc, blo, bhi);
-  const double2 *__restrict__ pay = reinterpret_cast<const double2 *>(P.payload);
-  stream_box(G, P, cc, blo, bhi, S.radius, lane,
-             [&](bool in, uint32_t k, double w0, double w1, double w2) {
-               const unsigned bal = __ballot_sync(0xffffffffu, in);
-               if (in) {
-                 const double d2 = w0 * w0 + w1 * w1 + w2 * w2;
-                 const double2 zq = pay[4 * (size_t)k + 1];
-                 const double2 jv = pay[4 * (size_t)k + 2], jt = pay[4 * (size_t)k + 3];
-                 const int slot =
-                     (head + count + __popc(bal & ((1u << lane) - 1u))) & (RING - 1);
-                 R[0][slot] = make_double2(w0, w1);
-                 R[1][slot] = make_double2(w2, -d2 * S.inv_radius);
-                 R[2][slot] = make_double2(zq.y, jv.x);
-                 R[3][slot] = make_double2(jv.y, jt.x);
-               }
-               count += __popc(bal);
-               __syncwarp();
-               if (count >= 32) {
-                 drain_full();
-                 __syncwarp();
-               }
-             });
-  if (count > 0) drain(count);
-  if (COUNT) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      npairs += __shfl_down_sync(0xffffffffu, npairs, o);
-      nnode += __shfl_down_sync(0xffffffffu, nnode, o);
+      pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+      nodes += __shfl_xor_sync(0xffffffffu, nodes, o);
     }
-    if (lane == 0) {
-      if (npairs) atomicAdd(&counters[0], npairs);
-      if (nnode) atomicAdd(&counters[1], nnode);
-      if (nevals) atomicAdd(&counters[2], nevals);
+    if ((threadIdx.x & 31) == 0 && evaluated) {
+      atomicAdd(&counters[0], pairs);
+      atomicAdd(&counters[1], nodes);
+      atomicAdd(&counters[2], evaluated * (unsigned)npt);
     }
   }
+};
+
+constexpr int BLOCK_PER = 4;  // targets per lane
+// Four tiles per block.
+template <bool ALPHA2, bool COUNT>
+__global__ void __launch_bounds__(32 * BW, 3)
+    deposit_blocks_kernel(TilesDev T, const uint32_t *__restrict__ run_starts, BinGrid G,
+                          DepParticles P, ShapeWeight S, TileSums O,
+                          unsigned long long *__restrict__ counters,
+                          const uint32_t *__restrict__ order) {
+  constexpr int PER = BLOCK_PER, LANES = 32 / PER;
+  __shared__ BlockStage<4> stage;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int tg = lane % LANES, grp = lane / LANES;
+  const long long blk = order ? (long long)order[blockIdx.x] : (long long)blockIdx.x;
+  const long long t = BW * blk + wid;
+  const bool have = t < T.tiles;
+  const long long p0 = t * TILE;
+  const int npt = have ? (int)min((long long)TILE, T.count - p0) : 0;
+  BlockBox X;
 #pragma unroll
-  for (int h = 0; h < PPL; ++h)
-    if (live[h]) {
-      const long long u = p0 + lane + 32 * h;
-      out[u] = (r0[h] + r1[h]) * wscale;
-      out[npos + u] = (x0[h] + x1[h]) * wscale;
-      out[2 * npos + u] = (y0[h] + y1[h]) * wscale;
-      out[3 * npos + u] = (z0[h] + z1[h]) * wscale;
+  for (int d = 0; d < 3; ++d) {
+    double lo = INFINITY, hi = -INFINITY;
+    for (long long k = BW * blk; k < min(T.tiles, BW * blk + BW); ++k) {
+      lo = fmin(lo, T.boxes[6 * k + d] - T.boxes[6 * k + 3 + d]);
+      hi = fmax(hi, T.boxes[6 * k + d] + T.boxes[6 * k + 3 + d]);
     }
+    X.c[d] = 0.5 * (lo + hi);
+    X.h[d] = 0.5 * (hi - lo) + 1e-5 * S.radius;
+    X.mid[d] = have ? (float)(T.boxes[6 * t + d] - X.c[d]) : 0;
+    X.hf[d] = have ? (float)(T.boxes[6 * t + 3 + d] + 1e-5 * S.radius) : -1e30f;
+  }
+  stage_begin(stage);
+  DepositTargets<PER, ALPHA2, COUNT> D;
+  D.load(T, p0, npt, tg, X.c, S);
+  const uint32_t evaluated =
+      evaluate_particles<PER, 4>(stage, G, P, X, S.radius, S.inv_radius, D);
+  if (COUNT) D.count(T, run_starts, p0, npt, tg, evaluated, counters);
+  reduce_groups<PER, 4>(D.sum);
+  const int row = PER * tg + grp;
+  if (row < npt) {
+    const long long u = T.rows[p0 + row];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (O.out[k]) O.out[k][u] = D.sum[k][0];
+  }
 }
 
-// Mixed-precision form of deposit_groups_kernel: the same culling and order,
-// with the particle-to-position geometry and the shape weight in FP32
+// A tile per block, its four warps sharing the tile's particles (each streams
+// every fourth batch, adds up at the end): for jobs with too few tiles to fill
+// the SMs, where a block of four tiles would run one after the other on an
+// otherwise idle SM.
+constexpr int TILE_WARPS = 4;
+template <bool ALPHA2, bool COUNT>
+__global__ void __launch_bounds__(32 * TILE_WARPS, 3)
+    deposit_split_kernel(TilesDev T, const uint32_t *__restrict__ run_starts, BinGrid G,
+                         DepParticles P, ShapeWeight S, TileSums O,
+                         unsigned long long *__restrict__ counters) {
+  constexpr int PER = 4, LANES = 32 / PER, RING = 64;
+  // ring entries: (wx, wy), (wz, -|w|^2/a), (q N, q N vx), (q N vy, q N vz)
+  __shared__ double2 ring[TILE_WARPS][4][RING];
+  __shared__ Segments segments[TILE_WARPS];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int tg = lane % LANES, grp = lane / LANES;
+  const long long t = blockIdx.x;
+  const long long p0 = t * TILE;
+  const int npt = (int)min((long long)TILE, T.count - p0);
+  double c[3], hfd[3];
+  float hf[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    c[d] = T.boxes[6 * t + d];
+    hfd[d] = T.boxes[6 * t + 3 + d] + 1e-5 * S.radius;
+    hf[d] = (float)hfd[d];
+  }
+  DepositTargets<PER, ALPHA2, COUNT> D;
+  D.load(T, p0, npt, tg, c, S);
+  double2(*R)[RING] = ring[wid];
+  int head = 0, count = 0;
+  unsigned long long evaluated = 0;
+  // the 32 entries from head: PER at a time, one per group of lanes
+  auto drain = [&]() {
+#pragma unroll 1
+    for (int i = 0; i < 32; i += PER) {
+      const int e = head + i + grp;
+      const double2 w01 = R[0][e], w2e = R[1][e], qx = R[2][e], yz = R[3][e];
+      const double v[4] = {qx.x, qx.y, yz.x, yz.y};
+      D(w01.x, w01.y, w2e.x, w2e.y, v);
+    }
+    head ^= 32;
+    count -= 32;
+  };
+  const float rc4 = near_limit(S.radius);
+  const double2 *__restrict__ pay = reinterpret_cast<const double2 *>(P.payload);
+  stream_particles(G, P, c, hfd, S.radius, segments[wid], wid, TILE_WARPS,
+                   [&](bool valid, uint32_t k, double w0, double w1, double w2, double q) {
+                     const bool in = valid && near_box(w0, w1, w2, hf, rc4);
+                     const unsigned bal = __ballot_sync(0xffffffffu, in);
+                     if (in) {
+                       const double2 jv = pay[4 * (size_t)k + 2], jt = pay[4 * (size_t)k + 3];
+                       const int slot =
+                           (head + count + __popc(bal & ((1u << lane) - 1u))) & (RING - 1);
+                       R[0][slot] = make_double2(w0, w1);
+                       R[1][slot] =
+                           make_double2(w2, -(w0 * w0 + w1 * w1 + w2 * w2) * S.inv_radius);
+                       R[2][slot] = make_double2(q, jv.x);
+                       R[3][slot] = make_double2(jv.y, jt.x);
+                     }
+                     count += __popc(bal);
+                     if (COUNT) evaluated += __popc(bal);
+                     __syncwarp();
+                     if (count >= 32) {
+                       drain();
+                       __syncwarp();
+                     }
+                   });
+  if (count > 0) {
+    // the rest, filled up with entries beyond every radius
+    if (lane >= count) {
+      const int e = head + lane;
+      R[0][e] = R[2][e] = R[3][e] = make_double2(0, 0);
+      R[1][e] = make_double2(0, -1e300);
+    }
+    __syncwarp();
+    drain();
+  }
+  if (COUNT) D.count(T, run_starts, p0, npt, tg, evaluated, counters);
+  reduce_groups<PER, 4>(D.sum);
+  const int row = PER * tg + grp;
+  __syncwarp();
+  // (the ring is done with: four sums per row)
+  double *part = reinterpret_cast<double *>(&ring[wid][0][0]);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) part[32 * k + row] = D.sum[k][0];
+  __syncthreads();
+  if (wid != 0 || lane >= npt) return;
+  const long long u = T.rows[p0 + lane];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    double v = 0;
+#pragma unroll
+    for (int w = 0; w < TILE_WARPS; ++w)
+      v += reinterpret_cast<const double *>(&ring[w][0][0])[32 * k + lane];
+    if (O.out[k]) O.out[k][u] = v;
+  }
+}
+
+// The mixed_simt deposition: one warp per wide position group (<= 64
+// positions), with the particle-to-position geometry and the shape weight in FP32
 // (coordinates relative to the group centre, taken from the FP64 positions)
 // and the contributions summed in FP32 over each batch of 32 ring entries,
 // then combined into FP64 per-position accumulators. A ring entry is 32
 // bytes: (wx, wy, wz, |w|^2), (qN, qN vx, qN vy, qN vz).
 template <bool ALPHA2, int PPL = 1>
-__global__ void __launch_bounds__(BLOCK, PPL == 1 ? PRT_GATHER_MIN_BLOCKS : PRT_MIXED_MIN_BLOCKS_WIDE)
+__global__ void __launch_bounds__(BLOCK, PPL == 1 ? 6 : PRT_MIXED_MIN_BLOCKS_WIDE)
     deposit_groups_mixed_kernel(const double *__restrict__ pos, long long ngroups,
                                 const uint32_t *__restrict__ gstarts,
                                 const double *__restrict__ gspheres, BinGrid G,
@@ -575,8 +621,7 @@ __global__ void __launch_bounds__(BLOCK, PPL == 1 ? PRT_GATHER_MIN_BLOCKS : PRT_
 
   const double c0 = gspheres[4 * g], c1 = gspheres[4 * g + 1], c2 = gspheres[4 * g + 2];
   // lane holds positions p0 + lane + 32 h, h < PPL; the weight base
-  // a - r^2/a = B + e + V . w as in deposit_groups_kernel, B and V rounded
-  // to FP32 from FP64
+  // a - r^2/a = B + e + V . w (tiles.cuh), B and V rounded to FP32 from FP64
   float V0[PPL], V1[PPL], V2[PPL], B[PPL];
   bool live[PPL];
 #pragma unroll
@@ -851,6 +896,87 @@ int upload_vec(const std::vector<T> &v, const T **dst) {
 
 }  // namespace
 
+// ------------------------------------------------------------------- tiles
+
+int prt_build_tiles(const double *points, long long count, const uint32_t *ids, TileSet *out) {
+  const int TILE_ = prt_dep::TILE;
+  std::vector<uint32_t> rows((size_t)count);
+  std::iota(rows.begin(), rows.end(), 0u);
+  // blocks of four tiles first, so that a block's tiles lie together
+  const long long block = prt_dep::BW * TILE_;
+  prt_dep::bisect_parallel(points, rows, (uint32_t)block);
+  for (long long b = 0; b < count; b += block)
+    prt_dep::bisect(points, rows, (uint32_t)b, (uint32_t)std::min(count, b + block), TILE_, 0.0,
+                    nullptr);
+  const long long nt = (count + TILE_ - 1) / TILE_;
+  std::vector<double> pos(3 * (size_t)count), boxes(6 * (size_t)nt);
+  for (long long t = 0; t < nt; ++t) {
+    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (long long r = t * TILE_; r < std::min<long long>(count, (t + 1) * TILE_); ++r)
+      for (int a = 0; a < 3; ++a) {
+        const double x = points[3 * (size_t)rows[r] + a];
+        pos[3 * (size_t)r + a] = x;
+        lo[a] = std::min(lo[a], x);
+        hi[a] = std::max(hi[a], x);
+      }
+    for (int a = 0; a < 3; ++a) {
+      boxes[6 * (size_t)t + a] = 0.5 * (lo[a] + hi[a]);
+      boxes[6 * (size_t)t + 3 + a] = 0.5 * (hi[a] - lo[a]);
+    }
+  }
+  if (ids)
+    for (uint32_t &r : rows) r = ids[r];
+  out->tiles = nt;
+  out->count = count;
+  int rc;
+  if ((rc = upload_vec(rows, &out->rows))) return rc;
+  if ((rc = upload_vec(pos, &out->pos))) return rc;
+  return upload_vec(boxes, &out->boxes);
+}
+
+void prt_free_tiles(TileSet *T) {
+  const void *ptrs[] = {T->rows, T->pos, T->boxes};
+  for (const void *p : ptrs)
+    if (p) cudaFree((void *)p);
+  *T = TileSet();
+}
+
+template <bool ALPHA2, bool COUNT>
+static void launch_tiles(bool split, const TileSet &T, const uint32_t *run_starts,
+                         const BinGrid &G, const DepParticles &P, const ShapeWeight &W,
+                         const TileSums &O, unsigned long long *counters, const uint32_t *order,
+                         cudaStream_t s) {
+  if (split)
+    deposit_split_kernel<ALPHA2, COUNT><<<(unsigned)T.tiles, 32 * TILE_WARPS, 0, s>>>(
+        tiles_dev(T), run_starts, G, P, W, O, counters);
+  else
+    deposit_blocks_kernel<ALPHA2, COUNT><<<(unsigned)((T.tiles + BW - 1) / BW), 32 * BW, 0, s>>>(
+        tiles_dev(T), run_starts, G, P, W, O, counters, order);
+}
+
+// tiles whose blocks of four give every SM a block: below it a tile takes a
+// block of its own (10,000 particles on 577 tiles: 81 us for the deposition
+// against 160 with two positions per lane)
+constexpr long long SPLIT_TILES = 4 * 148;
+
+int prt_dep::launch_deposit_tiles(const TileSet &T, const uint32_t *run_starts, const BinGrid &G,
+                                  const DepParticles &P, const ShapeParams &S,
+                                  double *const out[4], unsigned long long *counters,
+                                  const uint32_t *order, cudaStream_t s) {
+  const ShapeWeight W = {S.radius, S.inv_radius, S.alpha};
+  TileSums O;
+  for (int k = 0; k < 4; ++k) O.out[k] = out[k];
+  const bool split = T.tiles < SPLIT_TILES;
+  if (S.alpha == 2)
+    counters ? launch_tiles<true, true>(split, T, run_starts, G, P, W, O, counters, order, s)
+             : launch_tiles<true, false>(split, T, run_starts, G, P, W, O, counters, order, s);
+  else
+    counters ? launch_tiles<false, true>(split, T, run_starts, G, P, W, O, counters, order, s)
+             : launch_tiles<false, false>(split, T, run_starts, G, P, W, O, counters, order, s);
+  PRT_CHECK_CUDA(cudaGetLastError());
+  return PRT_OK;
+}
+
 // ------------------------------------------------------------ position set
 
 unsigned long long prt_next_target_uid() {
@@ -926,6 +1052,7 @@ int prt_mesh_build_positions(prt_mesh *m, const prt_mesh_desc *d) {
   if ((rc = upload_vec(node_to_pos, &P.node_to_pos))) return rc;
   if ((rc = upload_vec(run_starts, &P.run_starts))) return rc;
   if ((rc = upload_vec(order, &P.run_nodes))) return rc;
+  if ((rc = prt_build_tiles(pos.data(), npos, nullptr, &P.tiles))) return rc;
 
   // warp groups: runs of at most 32 positions, cut wherever the Morton cell
   // of about PRT_GROUP_TARGET positions changes, so that no group straddles
@@ -1210,15 +1337,20 @@ extern "C" int prt_deposit_shape(const prt_mesh *mesh, prt_workspace *ws, int32_
     const uint32_t *gs;
     const double *gsp;
     // heaviest groups first (group_work_kernel + a descending radix sort)
-    auto heavy_first = [&](long long ngr, const double *sph, const uint32_t **order) -> int {
+    auto heavy_first = [&](long long ngr, const double *bounds, bool boxes,
+                           const uint32_t **order) -> int {
       *order = nullptr;
       if (!PRT_DEPOSIT_HEAVY_FIRST || ngr < 2) return PRT_OK;
       int rc2;
       uint32_t *buf = (uint32_t *)ws_buffer(ws, PRT_WS_GROUP_ORDER, 16 * (size_t)ngr, &rc2);
       if (!buf) return rc2;
       uint32_t *wk = buf, *ids = buf + ngr, *wk_out = buf + 2 * ngr, *ids_out = buf + 3 * ngr;
-      group_work_kernel<<<prt_grid_blocks(ngr, 256), 256, 0, s>>>(ngr, sph, G, P.starts,
-                                                                  S.radius, wk, ids);
+      if (boxes)
+        group_work_kernel<true><<<prt_grid_blocks(ngr, 256), 256, 0, s>>>(ngr, bounds, G, P.starts,
+                                                                          S.radius, wk, ids);
+      else
+        group_work_kernel<false><<<prt_grid_blocks(ngr, 256), 256, 0, s>>>(
+            ngr, bounds, G, P.starts, S.radius, wk, ids);
       PRT_CHECK_CUDA(cudaGetLastError());
       size_t tb = 0;
       PRT_CHECK_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, wk, wk_out, ids,
@@ -1234,7 +1366,7 @@ extern "C" int prt_deposit_shape(const prt_mesh *mesh, prt_workspace *ws, int32_
     if (precision != PRT_PRECISION_FP64) {
       constexpr int W = PRT_MIXED_PPL;
       const unsigned nb = groups_for(W, ng, gs, gsp);
-      if ((rc = heavy_first(ng, gsp, &order))) return rc;
+      if ((rc = heavy_first(ng, gsp, false, &order))) return rc;
       if (a2)
         deposit_groups_mixed_kernel<true, W><<<nb, BLOCK, 0, s>>>(PS.pos, ng, gs, gsp, G, P, S,
                                                                   PS.count, vals, order);
@@ -1242,23 +1374,13 @@ extern "C" int prt_deposit_shape(const prt_mesh *mesh, prt_workspace *ws, int32_
         deposit_groups_mixed_kernel<false, W><<<nb, BLOCK, 0, s>>>(PS.pos, ng, gs, gsp, G, P, S,
                                                                    PS.count, vals, order);
     } else {
-      constexpr int W = PRT_FP64_PPL;
-      const unsigned nb = groups_for(W, ng, gs, gsp);
-      if ((rc = heavy_first(ng, gsp, &order))) return rc;
-      if (counter) {
-        if (a2)
-          deposit_groups_kernel<true, true, W><<<nb, BLOCK, 0, s>>>(
-              PS.pos, ng, gs, gsp, PS.run_starts, G, P, S, PS.count, vals, counter, order);
-        else
-          deposit_groups_kernel<false, true, W><<<nb, BLOCK, 0, s>>>(
-              PS.pos, ng, gs, gsp, PS.run_starts, G, P, S, PS.count, vals, counter, order);
-      } else if (a2) {
-        deposit_groups_kernel<true, false, W><<<nb, BLOCK, 0, s>>>(
-            PS.pos, ng, gs, gsp, PS.run_starts, G, P, S, PS.count, vals, nullptr, order);
-      } else {
-        deposit_groups_kernel<false, false, W><<<nb, BLOCK, 0, s>>>(
-            PS.pos, ng, gs, gsp, PS.run_starts, G, P, S, PS.count, vals, nullptr, order);
-      }
+      // (all blocks resident at once: their order does not matter)
+      if (PS.tiles.tiles >= SPLIT_TILES &&
+          (rc = heavy_first((PS.tiles.tiles + BW - 1) / BW, PS.tiles.boxes, true, &order)))
+        return rc;
+      double *const out[4] = {vals, vals + PS.count, vals + 2 * PS.count, vals + 3 * PS.count};
+      if ((rc = launch_deposit_tiles(PS.tiles, PS.run_starts, G, P, S, out, counter, order, s)))
+        return rc;
     }
     PRT_CHECK_CUDA(cudaGetLastError());
   }
@@ -1391,16 +1513,10 @@ extern "C" int prt_deposit_shape_noalloc(const prt_mesh *mesh, prt_shape_functio
   S.inv_radius = 1.0 / shape.radius;
   S.alpha = shape.alpha;
   for (int d = 0; d < 3; ++d) S.reach[d] = shape.radius;
-  const unsigned nb = (unsigned)((PS.groups + WARPS - 1) / WARPS);
-  if (shape.alpha == 2)
-    deposit_groups_kernel<true, false><<<nb, BLOCK, 0, s>>>(
-        PS.pos, PS.groups, PS.group_starts, PS.group_spheres, PS.run_starts, G, P, S, PS.count,
-        posvals, nullptr);
-  else
-    deposit_groups_kernel<false, false><<<nb, BLOCK, 0, s>>>(
-        PS.pos, PS.groups, PS.group_starts, PS.group_spheres, PS.run_starts, G, P, S, PS.count,
-        posvals, nullptr);
-  PRT_CHECK_CUDA(cudaGetLastError());
+  double *const out[4] = {posvals, posvals + PS.count, posvals + 2 * PS.count,
+                          posvals + 3 * PS.count};
+  if ((rc = launch_deposit_tiles(PS.tiles, PS.run_starts, G, P, S, out, nullptr, nullptr, s)))
+    return rc;
   if (rho || j) {
     expand_kernel<<<prt_grid_blocks(nn, 256), 256, 0, s>>>(nn, PS.count, PS.node_to_pos,
                                                            posvals, rho, j);

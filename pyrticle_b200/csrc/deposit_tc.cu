@@ -79,6 +79,7 @@
 #include <vector>
 
 #include "binning.cuh"
+#include "bisect.cuh"
 
 namespace {
 
@@ -1219,53 +1220,6 @@ struct TcPtrs {
   double *vals;
   const uint32_t *perm;
 };
-
-// Recursive bisection of the positions idx[b, e) into compact parts:
-// along the longest axis of the part's box, at a multiple of g rows (so that
-// all parts but the last of a branch hold exactly g), until a part holds at
-// most g positions and, when wmax > 0, is at most wmax wide along every axis.
-// Appends each final part's start (depth first: neighbouring parts are
-// neighbours in space) to `cuts` when given.
-void bisect(const double *P, std::vector<uint32_t> &idx, uint32_t b, uint32_t e, uint32_t g,
-            double wmax, std::vector<uint32_t> *cuts) {
-  struct Part {
-    uint32_t b, e;
-  };
-  std::vector<Part> stack{{b, e}};
-  while (!stack.empty()) {
-    const Part t = stack.back();
-    stack.pop_back();
-    const uint32_t n = t.e - t.b;
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (uint32_t i = t.b; i < t.e; ++i)
-      for (int a = 0; a < 3; ++a) {
-        lo[a] = std::min(lo[a], P[3 * (size_t)idx[i] + a]);
-        hi[a] = std::max(hi[a], P[3 * (size_t)idx[i] + a]);
-      }
-    int ax = 0;
-    for (int a = 1; a < 3; ++a)
-      if (hi[a] - lo[a] > hi[ax] - lo[ax]) ax = a;
-    const bool wide = wmax > 0 && hi[ax] - lo[ax] > wmax;
-    if (n <= 1 || (n <= g && !wide)) {
-      if (cuts) cuts->push_back(t.b);
-      continue;
-    }
-    uint32_t nl;
-    if (n > g) {
-      nl = g * std::max<uint32_t>(1, (uint32_t)std::lround((double)n / (2.0 * g)));
-      if (nl >= n) nl = g * ((n - 1) / g);
-    } else {
-      nl = n / 2;
-    }
-    std::nth_element(idx.begin() + t.b, idx.begin() + t.b + nl, idx.begin() + t.e,
-                     [&](uint32_t x, uint32_t y) {
-                       const double px = P[3 * (size_t)x + ax], py = P[3 * (size_t)y + ax];
-                       return px != py ? px < py : x < y;
-                     });
-    stack.push_back({t.b + nl, t.e});
-    stack.push_back({t.b, t.b + nl});
-  }
-}
 
 // The tiles of a target for a shape radius, kept in the workspace while
 // target and radius stay the same: parts of <= 128 positions from recursive

@@ -32,6 +32,19 @@ enum {
   PRT_WS_SLOTS
 };
 
+// Targets cut into tiles of exactly 32 (the last one partial) by recursive
+// bisection: tile t holds the rows 32 t .. 32 t + 31.
+struct TileSet {
+  long long tiles = 0, count = 0;
+  const uint32_t *rows = nullptr;  // [count] the target of each row
+  const double *pos = nullptr;     // [count][3], row order
+  const double *boxes = nullptr;   // [tiles][6]: centre, half extents
+};
+// Cuts the host points [count][3] into tiles and uploads them; point i is
+// target ids[i] (NULL: i). Freed with prt_free_tiles.
+int prt_build_tiles(const double *points, long long count, const uint32_t *ids, TileSet *out);
+void prt_free_tiles(TileSet *tiles);
+
 // Distinct node positions (coincident DG nodes merged), in Morton order:
 // the targets of the mesh deposition.
 struct PositionSet {
@@ -45,6 +58,8 @@ struct PositionSet {
   long long groups = 0;
   const uint32_t *group_starts = nullptr; // [groups + 1]
   const double *group_spheres = nullptr;  // [groups][4]: centre xyz, radius
+  // the FP64 deposition's tiles
+  TileSet tiles;
   // wide warp groups for the deposition (two positions per lane): runs of
   // <= 64 positions that never straddle a Morton cell of about twice the
   // group target
