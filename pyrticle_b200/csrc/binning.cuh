@@ -36,8 +36,6 @@ struct DepParticles {
   const uint32_t *__restrict__ starts;  // [nbins + 1]
 };
 
-enum Weight { W_SHAPE2 = 0, W_SHAPE_POW = 1, W_TRILINEAR = 2 };
-
 struct ShapeParams {
   double radius, radius2, inv_radius, alpha;
   double reach[3];  // candidate reach per axis (radius, or h for trilinear)

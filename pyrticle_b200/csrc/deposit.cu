@@ -959,14 +959,49 @@ static void launch_tiles(bool split, const TileSet &T, const uint32_t *run_start
 // against 160 with two positions per lane)
 constexpr long long SPLIT_TILES = 4 * 148;
 
-int prt_dep::launch_deposit_tiles(const TileSet &T, const uint32_t *run_starts, const BinGrid &G,
-                                  const DepParticles &P, const ShapeParams &S,
+// The groups (or blocks of tiles) ordered heaviest first: group_work_kernel
+// and a descending radix sort.
+static int heavy_first(prt_workspace *ws, long long n, const double *bounds, bool boxes,
+                       const BinGrid &G, const DepParticles &P, double radius,
+                       const uint32_t **order, cudaStream_t s) {
+  *order = nullptr;
+  if (!PRT_DEPOSIT_HEAVY_FIRST || n < 2) return PRT_OK;
+  int rc;
+  uint32_t *buf = (uint32_t *)ws_buffer(ws, PRT_WS_GROUP_ORDER, 16 * (size_t)n, &rc);
+  if (!buf) return rc;
+  uint32_t *wk = buf, *ids = buf + n, *wk_out = buf + 2 * n, *ids_out = buf + 3 * n;
+  if (boxes)
+    group_work_kernel<true><<<prt_grid_blocks(n, 256), 256, 0, s>>>(n, bounds, G, P.starts, radius,
+                                                                    wk, ids);
+  else
+    group_work_kernel<false><<<prt_grid_blocks(n, 256), 256, 0, s>>>(n, bounds, G, P.starts,
+                                                                     radius, wk, ids);
+  PRT_CHECK_CUDA(cudaGetLastError());
+  size_t tb = 0;
+  PRT_CHECK_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, wk, wk_out, ids, ids_out,
+                                                           (int)n, 0, 32, s));
+  void *tmp = ws_buffer(ws, PRT_WS_CUB, tb, &rc);
+  if (!tmp) return rc;
+  PRT_CHECK_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp, tb, wk, wk_out, ids, ids_out,
+                                                           (int)n, 0, 32, s));
+  *order = ids_out;
+  return PRT_OK;
+}
+
+int prt_dep::launch_deposit_tiles(prt_workspace *ws, const TileSet &T, const uint32_t *run_starts,
+                                  const BinGrid &G, const DepParticles &P, const ShapeParams &S,
                                   double *const out[4], unsigned long long *counters,
-                                  const uint32_t *order, cudaStream_t s) {
+                                  cudaStream_t s) {
   const ShapeWeight W = {S.radius, S.inv_radius, S.alpha};
   TileSums O;
   for (int k = 0; k < 4; ++k) O.out[k] = out[k];
   const bool split = T.tiles < SPLIT_TILES;
+  // (a split job's blocks are all resident at once: no order)
+  const uint32_t *order = nullptr;
+  int rc;
+  if (ws && !split &&
+      (rc = heavy_first(ws, (T.tiles + BW - 1) / BW, T.boxes, true, G, P, S.radius, &order, s)))
+    return rc;
   if (S.alpha == 2)
     counters ? launch_tiles<true, true>(split, T, run_starts, G, P, W, O, counters, order, s)
              : launch_tiles<true, false>(split, T, run_starts, G, P, W, O, counters, order, s);
@@ -1336,37 +1371,11 @@ extern "C" int prt_deposit_shape(const prt_mesh *mesh, prt_workspace *ws, int32_
     long long ng;
     const uint32_t *gs;
     const double *gsp;
-    // heaviest groups first (group_work_kernel + a descending radix sort)
-    auto heavy_first = [&](long long ngr, const double *bounds, bool boxes,
-                           const uint32_t **order) -> int {
-      *order = nullptr;
-      if (!PRT_DEPOSIT_HEAVY_FIRST || ngr < 2) return PRT_OK;
-      int rc2;
-      uint32_t *buf = (uint32_t *)ws_buffer(ws, PRT_WS_GROUP_ORDER, 16 * (size_t)ngr, &rc2);
-      if (!buf) return rc2;
-      uint32_t *wk = buf, *ids = buf + ngr, *wk_out = buf + 2 * ngr, *ids_out = buf + 3 * ngr;
-      if (boxes)
-        group_work_kernel<true><<<prt_grid_blocks(ngr, 256), 256, 0, s>>>(ngr, bounds, G, P.starts,
-                                                                          S.radius, wk, ids);
-      else
-        group_work_kernel<false><<<prt_grid_blocks(ngr, 256), 256, 0, s>>>(
-            ngr, bounds, G, P.starts, S.radius, wk, ids);
-      PRT_CHECK_CUDA(cudaGetLastError());
-      size_t tb = 0;
-      PRT_CHECK_CUDA(cub::DeviceRadixSort::SortPairsDescending(nullptr, tb, wk, wk_out, ids,
-                                                               ids_out, (int)ngr, 0, 32, s));
-      void *tmp = ws_buffer(ws, PRT_WS_CUB, tb, &rc2);
-      if (!tmp) return rc2;
-      PRT_CHECK_CUDA(cub::DeviceRadixSort::SortPairsDescending(tmp, tb, wk, wk_out, ids,
-                                                               ids_out, (int)ngr, 0, 32, s));
-      *order = ids_out;
-      return PRT_OK;
-    };
     const uint32_t *order = nullptr;
     if (precision != PRT_PRECISION_FP64) {
       constexpr int W = PRT_MIXED_PPL;
       const unsigned nb = groups_for(W, ng, gs, gsp);
-      if ((rc = heavy_first(ng, gsp, false, &order))) return rc;
+      if ((rc = heavy_first(ws, ng, gsp, false, G, P, S.radius, &order, s))) return rc;
       if (a2)
         deposit_groups_mixed_kernel<true, W><<<nb, BLOCK, 0, s>>>(PS.pos, ng, gs, gsp, G, P, S,
                                                                   PS.count, vals, order);
@@ -1374,12 +1383,8 @@ extern "C" int prt_deposit_shape(const prt_mesh *mesh, prt_workspace *ws, int32_
         deposit_groups_mixed_kernel<false, W><<<nb, BLOCK, 0, s>>>(PS.pos, ng, gs, gsp, G, P, S,
                                                                    PS.count, vals, order);
     } else {
-      // (all blocks resident at once: their order does not matter)
-      if (PS.tiles.tiles >= SPLIT_TILES &&
-          (rc = heavy_first((PS.tiles.tiles + BW - 1) / BW, PS.tiles.boxes, true, &order)))
-        return rc;
       double *const out[4] = {vals, vals + PS.count, vals + 2 * PS.count, vals + 3 * PS.count};
-      if ((rc = launch_deposit_tiles(PS.tiles, PS.run_starts, G, P, S, out, counter, order, s)))
+      if ((rc = launch_deposit_tiles(ws, PS.tiles, PS.run_starts, G, P, S, out, counter, s)))
         return rc;
     }
     PRT_CHECK_CUDA(cudaGetLastError());
@@ -1515,7 +1520,7 @@ extern "C" int prt_deposit_shape_noalloc(const prt_mesh *mesh, prt_shape_functio
   for (int d = 0; d < 3; ++d) S.reach[d] = shape.radius;
   double *const out[4] = {posvals, posvals + PS.count, posvals + 2 * PS.count,
                           posvals + 3 * PS.count};
-  if ((rc = launch_deposit_tiles(PS.tiles, PS.run_starts, G, P, S, out, nullptr, nullptr, s)))
+  if ((rc = launch_deposit_tiles(nullptr, PS.tiles, PS.run_starts, G, P, S, out, nullptr, s)))
     return rc;
   if (rho || j) {
     expand_kernel<<<prt_grid_blocks(nn, 256), 256, 0, s>>>(nn, PS.count, PS.node_to_pos,

@@ -1,23 +1,25 @@
 // grid.cu -- deposition onto brick grids and the element-local remap onto
 // the DG nodes (dep_grid_base.hpp:175-382, dep_grid.hpp:220-358, grid.hpp).
 //
-// Deposition is the same deterministic gather as the mesh depositor (see
-// deposit.cu): particles binned and sorted, one CTA per tile of 8 x 4 x 4
-// brick points, one point per thread, the staged particles culled against
-// the tile's bounding sphere. Weights: the shape function at the point (the
-// reference's grid depositor) or trilinear weights (cell-centred hat
-// functions, clamped at the brick edge so that they always sum to one).
+// Weights: the shape function at the point (the reference's grid depositor):
+// the FP64 pair sums by tiles (tiles.cuh), whose targets are the bricks'
+// points; or trilinear weights (cell-centred hat functions, clamped at the
+// brick edge so that they always sum to one): particles binned and sorted, one
+// CTA per tile of 8 x 4 x 4 brick points, one point per thread, the staged
+// particles culled against the tile's bounding sphere.
 // Jiggly bricks (grid.hpp:345-449) take their points from three jittered
-// point origins; the tile boxes grow by the largest jitter.
+// point origins (shape weights only).
 
 #include <cub/cub.cuh>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "binning.cuh"
+#include "tiles.cuh"
 
 namespace {
 
@@ -29,18 +31,10 @@ using namespace prt_dep;
 
 // ---------------------------------------------------------------- targets
 
-// Per brick of a jiggly grid: the three point origins and, per axis, the
-// largest distance of a point from its cell centre.
-struct JiggleDev {
-  double origins[3][3];
-  double pad[3];
-};
-
 // Tile of 8 x 4 x 4 points of one brick; one group (the tile box).
 struct BrickTarget {
   const prt_brick *__restrict__ bricks;
   const long long *__restrict__ tile_starts;  // [bricks+1] cumulative tile counts
-  const JiggleDev *__restrict__ jiggle;       // [bricks] or NULL (regular points)
   int brick_count;
   int check_tag;
 
@@ -79,14 +73,6 @@ struct BrickTarget {
     int b, idx[3];
     valid(tile, t, b, idx);
     const prt_brick &B = bricks[b];
-    if (jiggle) {
-      // jiggly_brick::point (grid.hpp:386-396)
-      const double *o = jiggle[b].origins[(idx[0] + idx[1] + idx[2]) % 3];
-      x0 = o[0] + idx[0] * B.stepwidths[0];
-      x1 = o[1] + idx[1] * B.stepwidths[1];
-      x2 = o[2] + idx[2] * B.stepwidths[2];
-      return;
-    }
     x0 = B.origin[0] + B.stepwidths[0] / 2 + idx[0] * B.stepwidths[0];
     x1 = B.origin[1] + B.stepwidths[1] / 2 + idx[1] * B.stepwidths[1];
     x2 = B.origin[2] + B.stepwidths[2] / 2 + idx[2] * B.stepwidths[2];
@@ -101,10 +87,6 @@ struct BrickTarget {
       int last = min(i0[d] + cnt, B.dims[d]) - 1;
       lo[d] = B.origin[d] + B.stepwidths[d] / 2 + i0[d] * B.stepwidths[d];
       hi[d] = B.origin[d] + B.stepwidths[d] / 2 + last * B.stepwidths[d];
-      if (jiggle) {
-        lo[d] -= jiggle[b].pad[d];
-        hi[d] += jiggle[b].pad[d];
-      }
     }
   }
   __device__ void group_sphere(long long tile, int, double radius, double s[4]) const {
@@ -124,17 +106,15 @@ struct BrickTarget {
 };
 
 
-// One CTA per tile of brick points, one point per thread. Per chunk of
-// staged particles every thread stages one particle and tests it against the
-// tile's bounding sphere (grown by the reach); the survivors are compacted
-// into a shared index list that every point walks. Bin rows are culled
-// against the tile box with the sphere of the shape radius.
-template <class Target, int WEIGHT, bool COUNT = false>
+// Trilinear deposition: one CTA per tile of brick points, one point per
+// thread. Per chunk of staged particles every thread stages one particle and
+// tests it against the tile's bounding sphere (grown by the reach); the
+// survivors are compacted into a shared index list that every point walks.
+template <class Target>
 __global__ void __launch_bounds__(BLOCK, PRT_GRID_MIN_BLOCKS)
-    deposit_grid_kernel(Target T, BinGrid G, DepParticles P, ShapeParams S,
+    deposit_trilinear_kernel(Target T, BinGrid G, DepParticles P, ShapeParams S,
                   double *__restrict__ rho, double *__restrict__ j, long long j_stride,
-                  const prt_brick *__restrict__ tri_bricks,
-                  unsigned long long *__restrict__ pair_counter) {
+                  const prt_brick *__restrict__ tri_bricks) {
   static_assert(BLOCK == CHUNK, "one staged particle per thread");
   constexpr int WARPS = BLOCK / 32;
   __shared__ double sp[PAYLOAD][CHUNK];
@@ -156,18 +136,15 @@ __global__ void __launch_bounds__(BLOCK, PRT_GRID_MIN_BLOCKS)
   const int grp = live ? T.group_of(t) : 0;
   if (t < ng) T.group_sphere(tile, t, S.radius, sph[t]);
 
-  // trilinear: the point's brick and index for the clamped hat weights
+  // the point's brick and index for the clamped hat weights
   int tb = 0, tidx[3] = {0, 0, 0};
   double th[3] = {1, 1, 1};
-  if constexpr (WEIGHT == W_TRILINEAR) {
-    if (live) {
-      T.valid(tile, t, tb, tidx);
-      for (int d = 0; d < 3; ++d) th[d] = tri_bricks[tb].stepwidths[d];
-    }
+  if (live) {
+    T.valid(tile, t, tb, tidx);
+    for (int d = 0; d < 3; ++d) th[d] = tri_bricks[tb].stepwidths[d];
   }
 
   double a_rho = 0, a_jx = 0, a_jy = 0, a_jz = 0;
-  unsigned long long npairs = 0;
 
   double lo[3], hi[3];
   T.box(tile, lo, hi);
@@ -184,42 +161,17 @@ __global__ void __launch_bounds__(BLOCK, PRT_GRID_MIN_BLOCKS)
       u1[d] = min(u1[d], G.dims[d] - 1);
     }
   }
-  // sphere culling of bin rows (not for the per-axis trilinear reach)
-  constexpr bool SPHERE = WEIGHT != W_TRILINEAR;
-  const double reach = S.reach[0] * (1 + 1e-6);
-  const double reach2 = reach * reach;
   __syncthreads();
 
   for (int bz = u0[2]; bz <= u1[2]; ++bz) {
     int wz = bz, qz = 0;
     if (G.periodic[2]) { qz = floor_div(bz, G.dims[2]); wz = bz - qz * G.dims[2]; }
     const double sz = qz * G.period[2];
-    double dz2 = 0;
-    if (SPHERE) {
-      const double blo = G.origin[2] + bz * G.w[2], bhi = blo + G.w[2];
-      const double e = fmax(0.0, fmax(blo - hi[2], lo[2] - bhi)) - G.slack[2];
-      dz2 = e > 0 ? e * e : 0.0;
-      if (dz2 > reach2) continue;
-    }
     for (int by = u0[1]; by <= u1[1]; ++by) {
       int wy = by, qy = 0;
       if (G.periodic[1]) { qy = floor_div(by, G.dims[1]); wy = by - qy * G.dims[1]; }
       const double sy = qy * G.period[1];
-      int bx0 = u0[0], bx1 = u1[0];
-      if (SPHERE) {
-        const double blo = G.origin[1] + by * G.w[1], bhi = blo + G.w[1];
-        const double e = fmax(0.0, fmax(blo - hi[1], lo[1] - bhi)) - G.slack[1];
-        const double dyz2 = dz2 + (e > 0 ? e * e : 0.0);
-        if (dyz2 > reach2) continue;
-        const double rem = sqrt(reach2 - dyz2);
-        int c0 = bin_floor(G, 0, lo[0] - rem), c1 = bin_floor(G, 0, hi[0] + rem);
-        if (G.periodic[0]) {
-          c0 -= 1;
-          c1 += 1;
-        }
-        bx0 = max(bx0, c0);
-        bx1 = min(bx1, c1);
-      }
+      const int bx0 = u0[0], bx1 = u1[0];
       // the x-row splits into segments of constant shift
       int bx = bx0;
       while (bx <= bx1) {
@@ -285,28 +237,18 @@ __global__ void __launch_bounds__(BLOCK, PRT_GRID_MIN_BLOCKS)
               const double dx = x0 - sp[0][k];
               const double dy = x1 - sp[1][k];
               const double dz = x2 - sp[2][k];
-              double s;
-              if constexpr (WEIGHT == W_TRILINEAR) {
-                // clamped hat weight per axis (edge points absorb the outside)
-                double wgt = 1.0;
-                const double dd[3] = {dx, dy, dz};
-                const prt_brick &B = tri_bricks[tb];
+              // clamped hat weight per axis (edge points absorb the outside)
+              double s = 1.0;
+              const double dd[3] = {dx, dy, dz};
+              const prt_brick &B = tri_bricks[tb];
 #pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                  const double u = -dd[d] / th[d];  // (x_p - pt) / h
-                  // edge points also take the weight of the missing neighbour
-                  const bool edge = (tidx[d] == 0 && u < 0) || (tidx[d] == B.dims[d] - 1 && u > 0);
-                  wgt *= edge ? 1.0 : fmax(0.0, 1.0 - fabs(u));
-                }
-                if (wgt == 0) continue;
-                s = wgt;
-              } else {
-                const double r2 = dx * dx + dy * dy + dz * dz;
-                if (r2 > S.radius2) continue;
-                if (COUNT) ++npairs;
-                const double rt = S.radius - r2 * S.inv_radius;
-                s = WEIGHT == W_SHAPE2 ? rt * rt : pow(rt, S.alpha);
+              for (int d = 0; d < 3; ++d) {
+                const double u = -dd[d] / th[d];  // (x_p - pt) / h
+                // edge points also take the weight of the missing neighbour
+                const bool edge = (tidx[d] == 0 && u < 0) || (tidx[d] == B.dims[d] - 1 && u > 0);
+                s *= edge ? 1.0 : fmax(0.0, 1.0 - fabs(u));
               }
+              if (s == 0) continue;
               a_rho = fma(sp[3][k], s, a_rho);
               a_jx = fma(sp[4][k], s, a_jx);
               a_jy = fma(sp[5][k], s, a_jy);
@@ -316,11 +258,6 @@ __global__ void __launch_bounds__(BLOCK, PRT_GRID_MIN_BLOCKS)
         }
       }
     }
-  }
-  if (COUNT) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) npairs += __shfl_down_sync(0xffffffffu, npairs, o);
-    if (lane == 0 && npairs) atomicAdd(pair_counter, npairs);
   }
   if (live) {
     if (rho) rho[oidx] = a_rho;
@@ -343,9 +280,8 @@ struct prt_grid {
   int np;
   std::vector<prt_brick> host_bricks;
   prt_brick *bricks = nullptr;
-  JiggleDev *jiggle = nullptr;
   long long *tile_starts = nullptr;
-  long long tiles = 0;
+  long long tiles_count = 0;  // of 8 x 4 x 4 points (trilinear)
   long long grid_nodes = 0;
   long long eog_count = 0;
   uint32_t *eog_elements = nullptr;
@@ -365,6 +301,9 @@ struct prt_grid {
   mutable unsigned long long uid = 0;
   mutable std::vector<double> pt_host;
   mutable double *pt_dev = nullptr;
+  // the points cut into tiles, for the FP64 deposition (made on its first call)
+  mutable TileSet tiles;
+  mutable std::mutex tiles_mutex;
 };
 
 extern "C" int prt_grid_create(const prt_mesh *mesh, const prt_grid_desc *d, prt_grid **out) {
@@ -389,7 +328,7 @@ extern "C" int prt_grid_create(const prt_mesh *mesh, const prt_grid_desc *d, prt
     ts[b + 1] = ts[b] + t;
     gn = std::max(gn, B.start_index + (long long)B.dims[0] * B.dims[1] * B.dims[2]);
   }
-  g->tiles = ts.back();
+  g->tiles_count = ts.back();
   g->grid_nodes = gn;
   auto up = [&](auto **dst, const auto *src, size_t cnt) -> int {
     using T = std::remove_pointer_t<std::remove_reference_t<decltype(*dst)>>;
@@ -404,24 +343,18 @@ extern "C" int prt_grid_create(const prt_mesh *mesh, const prt_grid_desc *d, prt
   if (!rc) rc = up(&g->tile_starts, ts.data(), ts.size());
   if (!rc && d->point_origins) {
     g->host_origins.assign(d->point_origins, d->point_origins + 9 * d->brick_count);
-    std::vector<JiggleDev> jg(d->brick_count);
     for (int b = 0; b < d->brick_count && !rc; ++b) {
       const prt_brick &B = d->bricks[b];
       for (int a = 0; a < 3; ++a) {
         const double centre = B.origin[a] + B.stepwidths[a] / 2;
-        double pad = 0;
-        for (int i = 0; i < 3; ++i) {
-          const double o = d->point_origins[9 * b + 3 * i + a];
-          jg[b].origins[i][a] = o;
-          pad = std::max(pad, std::fabs(o - centre));
-        }
         // points stay within their cells (the reference's index ranges
         // assume it); the margin covers the rounding of idx * h
-        if (!(pad <= 0.5 * B.stepwidths[a] * (1 + 1e-12))) rc = PRT_ERR_INVALID_ARGUMENT;
-        jg[b].pad[a] = pad * (1 + 1e-9) + 1e-12 * B.stepwidths[a];
+        for (int i = 0; i < 3; ++i)
+          if (!(std::fabs(d->point_origins[9 * b + 3 * i + a] - centre) <=
+                0.5 * B.stepwidths[a] * (1 + 1e-12)))
+            rc = PRT_ERR_INVALID_ARGUMENT;
       }
     }
-    if (!rc) rc = up(&g->jiggle, jg.data(), jg.size());
   }
   g->eog_count = d->eog_count;
   if (d->eog_count > 0) {
@@ -460,11 +393,12 @@ extern "C" int prt_grid_create(const prt_mesh *mesh, const prt_grid_desc *d, prt
 
 extern "C" int prt_grid_destroy(prt_grid *g) {
   if (!g) return PRT_OK;
-  void *ptrs[] = {g->bricks,      g->tile_starts, g->jiggle,      g->eog_elements,
+  void *ptrs[] = {g->bricks,      g->tile_starts, g->eog_elements,
                   g->eog_starts,  g->eog_nodes,   g->eog_weights, g->eog_mstarts,
                   g->eog_matrices, g->avg_starts, g->avg_nodes,   g->pt_dev};
   for (void *p : ptrs)
     if (p) cudaFree(p);
+  prt_free_tiles(&g->tiles);
   delete g;
   return PRT_OK;
 }
@@ -488,6 +422,46 @@ __global__ void brick_tag_kernel(const prt_brick *__restrict__ bricks, int nb, l
   tag[i] = t;
 }
 
+// The position of point (i, j, k) of brick b: the regular cell centre, or the
+// jiggled point of jiggly_brick::point (grid.hpp:386-396).
+static void brick_point(const prt_grid *g, int b, const int idx[3], double p[3]) {
+  const prt_brick &B = g->host_bricks[b];
+  for (int a = 0; a < 3; ++a)
+    p[a] = g->host_origins.empty()
+               ? B.origin[a] + B.stepwidths[a] / 2 + idx[a] * B.stepwidths[a]
+               : g->host_origins[9 * b + 3 * ((idx[0] + idx[1] + idx[2]) % 3) + a] +
+                     idx[a] * B.stepwidths[a];
+}
+
+// The bricks' points and their grid-node numbers, cut into tiles once.
+static int grid_tiles(const prt_grid *g) {
+  std::lock_guard<std::mutex> lock(g->tiles_mutex);
+  if (g->tiles.tiles) return PRT_OK;
+  std::vector<double> P;
+  std::vector<uint32_t> ids;
+  for (int b = 0; b < g->brick_count; ++b) {
+    const prt_brick &B = g->host_bricks[b];
+    long long at = B.start_index;
+    int idx[3];
+    for (idx[2] = 0; idx[2] < B.dims[2]; ++idx[2])
+      for (idx[1] = 0; idx[1] < B.dims[1]; ++idx[1])
+        for (idx[0] = 0; idx[0] < B.dims[0]; ++idx[0], ++at) {
+          double p[3];
+          brick_point(g, b, idx, p);
+          P.insert(P.end(), p, p + 3);
+          ids.push_back((uint32_t)at);
+        }
+  }
+  TileSet T;
+  const int rc = prt_build_tiles(P.data(), (long long)ids.size(), ids.data(), &T);
+  if (rc) {
+    prt_free_tiles(&T);
+    return rc;
+  }
+  g->tiles = T;
+  return PRT_OK;
+}
+
 extern "C" int prt_deposit_grid(const prt_grid *g, prt_workspace *ws, int32_t weights,
                                 prt_shape_function shape, int64_t n, const double *x,
                                 const double *q, const double *v, const uint32_t *el,
@@ -495,7 +469,7 @@ extern "C" int prt_deposit_grid(const prt_grid *g, prt_workspace *ws, int32_t we
   if (!g || !ws || n < 0 || n >= (1ll << 31)) return PRT_ERR_INVALID_ARGUMENT;
   if (weights != PRT_GRID_SHAPE && weights != PRT_GRID_TRILINEAR) return PRT_ERR_INVALID_ARGUMENT;
   if (weights == PRT_GRID_SHAPE && !(shape.radius > 0)) return PRT_ERR_INVALID_ARGUMENT;
-  if (weights == PRT_GRID_TRILINEAR && g->jiggle) return PRT_ERR_INVALID_ARGUMENT;
+  if (weights == PRT_GRID_TRILINEAR && !g->host_origins.empty()) return PRT_ERR_INVALID_ARGUMENT;
   if (n > 0 && (!x || !q || (grid_j && !v))) return PRT_ERR_INVALID_ARGUMENT;
   cudaStream_t s = (cudaStream_t)stream;
   const long long G_n = g->grid_nodes;
@@ -565,32 +539,35 @@ extern "C" int prt_deposit_grid(const prt_grid *g, prt_workspace *ws, int32_t we
     return rc;
   DepParticles P;
   if ((rc = stage_particles(ws, G, n, x, q, v, el, nullptr, normalizer, tag, P, s))) return rc;
+  if (weights == PRT_GRID_SHAPE) {
+    if ((rc = grid_tiles(g))) return rc;
+    // numbers that no brick uses stay zero
+    if (g->tiles.count != G_n) {
+      if (grid_rho) PRT_CHECK_CUDA(cudaMemsetAsync(grid_rho, 0, G_n * sizeof(double), s));
+      if (grid_j) PRT_CHECK_CUDA(cudaMemsetAsync(grid_j, 0, 3 * G_n * sizeof(double), s));
+    }
+    double *out[4] = {grid_rho, nullptr, nullptr, nullptr};
+    for (int d = 0; d < 3; ++d)
+      if (grid_j) out[1 + d] = grid_j + d * G_n;
+    ScopedTimer timer(ws, PRT_TIME_DEPOSIT_GATHER, s);
+    return launch_deposit_tiles(ws, g->tiles, nullptr, G, P, S, out, nullptr, s);
+  }
   BrickTarget T;
   T.bricks = g->bricks;
   T.tile_starts = g->tile_starts;
-  T.jiggle = g->jiggle;
   T.brick_count = g->brick_count;
-  T.check_tag = weights == PRT_GRID_TRILINEAR;
+  T.check_tag = 1;
   if (grid_rho) PRT_CHECK_CUDA(cudaMemsetAsync(grid_rho, 0, G_n * sizeof(double), s));
   if (grid_j) PRT_CHECK_CUDA(cudaMemsetAsync(grid_j, 0, 3 * G_n * sizeof(double), s));
   ScopedTimer timer(ws, PRT_TIME_DEPOSIT_GATHER, s);
-  if (weights == PRT_GRID_TRILINEAR)
-    deposit_grid_kernel<BrickTarget, W_TRILINEAR><<<(unsigned)g->tiles, BLOCK, 0, s>>>(
-        T, G, P, S, grid_rho, grid_j, G_n, g->bricks, nullptr);
-  else if (shape.alpha == 2)
-    deposit_grid_kernel<BrickTarget, W_SHAPE2><<<(unsigned)g->tiles, BLOCK, 0, s>>>(
-        T, G, P, S, grid_rho, grid_j, G_n, g->bricks, nullptr);
-  else
-    deposit_grid_kernel<BrickTarget, W_SHAPE_POW><<<(unsigned)g->tiles, BLOCK, 0, s>>>(
-        T, G, P, S, grid_rho, grid_j, G_n, g->bricks, nullptr);
+  deposit_trilinear_kernel<BrickTarget><<<(unsigned)g->tiles_count, BLOCK, 0, s>>>(
+      T, G, P, S, grid_rho, grid_j, G_n, g->bricks);
   PRT_CHECK_CUDA(cudaGetLastError());
   return PRT_OK;
 }
 
-// The grid's points in grid-node order (host and device), made once: the
-// positions of BrickTarget::point (regular cell centres, or the jiggled
-// points of jiggly_brick::point, grid.hpp:386-396). The bricks must number
-// their points contiguously (brick b starts where brick b-1 ends).
+// The grid's points in grid-node order (host and device), made once. The
+// bricks must number their points contiguously (brick b starts where brick b-1 ends).
 int grid_points(const prt_grid *g) {
   if (g->pt_dev) return PRT_OK;
   long long next = 0;
@@ -606,13 +583,9 @@ int grid_points(const prt_grid *g) {
       for (int jy = 0; jy < B.dims[1]; ++jy)
         for (int i = 0; i < B.dims[0]; ++i) {
           const int idx[3] = {i, jy, k};
-          double *p = &P[3 * (size_t)(B.start_index + i +
-                                      (long long)B.dims[0] * (jy + (long long)B.dims[1] * k))];
-          for (int a = 0; a < 3; ++a)
-            p[a] = g->host_origins.empty()
-                       ? B.origin[a] + B.stepwidths[a] / 2 + idx[a] * B.stepwidths[a]
-                       : g->host_origins[9 * b + 3 * ((i + jy + k) % 3) + a] +
-                             idx[a] * B.stepwidths[a];
+          brick_point(g, b, idx,
+                      &P[3 * (size_t)(B.start_index + i +
+                                      (long long)B.dims[0] * (jy + (long long)B.dims[1] * k))]);
         }
   }
   double *d = nullptr;
@@ -662,20 +635,22 @@ extern "C" int prt_deposit_grid_mixed(const prt_grid *g, prt_workspace *ws,
   return prt_deposit_points_tc(T, ws, shape, n, x, q, v, el, grid_rho, grid_j, s);
 }
 
-// Remap (dep_grid.hpp:270-358): one warp per element-on-grid; lanes own the
-// element's nodes, the weighted grid values of NC components are staged in
-// shared memory, and each matrix entry is read once for all components. A
-// block of grid values that is zero in every component is skipped before the
-// matrix is read (fma(M, 0, acc) = acc: the sums are unchanged).
+// Remap (dep_grid.hpp:270-358): one warp per element-on-grid. The weighted
+// grid values of NC components are staged in shared memory; the lanes own the
+// element's nodes, 32 / np groups of lanes taking different points (np <= 16;
+// two nodes per lane for np > 32), and each matrix entry is read once for all
+// components, four points ahead. A block of grid values that is zero in every
+// component is skipped before the matrix is read (fma(M, 0, acc) = acc: the
+// sums are unchanged). Bound by the matrices' bytes; one point at a time the
+// loads' latency took 289 us for 98,304 elements of order 3.
 template <int NC>
-__global__ void remap_kernel(long long eog_count, int np, const uint32_t *__restrict__ els,
-                             const uint64_t *__restrict__ starts,
-                             const uint32_t *__restrict__ gnodes,
-                             const double *__restrict__ weights,
-                             const uint64_t *__restrict__ mstarts,
-                             const double *__restrict__ mats, const double *__restrict__ from,
-                             long long from_stride, double *__restrict__ to,
-                             long long to_stride, long long offset, long long inc) {
+__global__ void __launch_bounds__(128)
+    remap_kernel(long long eog_count, int np, const uint32_t *__restrict__ els,
+                 const uint64_t *__restrict__ starts, const uint32_t *__restrict__ gnodes,
+                 const double *__restrict__ weights, const uint64_t *__restrict__ mstarts,
+                 const double *__restrict__ mats, const double *__restrict__ from,
+                 long long from_stride, double *__restrict__ to, long long to_stride,
+                 long long offset, long long inc) {
   extern __shared__ double gv_all[];
   const int warps = blockDim.x >> 5;
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -685,6 +660,9 @@ __global__ void remap_kernel(long long eog_count, int np, const uint32_t *__rest
   const int cnt = (int)(starts[e + 1] - s);
   // stage at most 256 points per pass
   double *gv = gv_all + (size_t)wid * 256 * NC;
+  const int groups = np <= 32 ? 32 / np : 1;
+  const int grp = np <= 32 ? lane / np : 0;   // == groups: an idle lane
+  const int row = np <= 32 ? lane % np : lane;
   double acc[NC][2];
 #pragma unroll
   for (int c = 0; c < NC; ++c) acc[c][0] = acc[c][1] = 0;
@@ -706,24 +684,35 @@ __global__ void remap_kernel(long long eog_count, int np, const uint32_t *__rest
     __syncwarp();
     if (__any_sync(0xffffffffu, any)) {
       any_total = true;
-      for (int k = 0; k < m; ++k) {
-        double g[NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) g[c] = gv[c * 256 + k];
+      for (int r = 0; r < 2; ++r) {
+        const int i = row + 32 * r;
+        if (i >= np || grp >= groups) break;
+        const double *Mi = M + i + (size_t)np * base;
+        for (int k = grp; k < m; k += 4 * groups) {
+          double mv[4];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          const int i = lane + 32 * r;
-          if (i < np) {
-            const double Mv = M[i + (size_t)np * (base + k)];
+          for (int u = 0; u < 4; ++u)
+            mv[u] = k + u * groups < m ? __ldg(Mi + (size_t)np * (k + u * groups)) : 0.0;
 #pragma unroll
-            for (int c = 0; c < NC; ++c) acc[c][r] = fma(Mv, g[c], acc[c][r]);
-          }
+          for (int u = 0; u < 4; ++u)
+            if (k + u * groups < m)
+#pragma unroll
+              for (int c = 0; c < NC; ++c)
+                acc[c][r] = fma(mv[u], gv[c * 256 + k + u * groups], acc[c][r]);
         }
       }
     }
     __syncwarp();
   }
   if (!any_total) return;
+  // the groups' sums, in their order
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    double t = acc[c][0];
+    for (int g = 1; g < groups; ++g) t += __shfl_sync(0xffffffffu, acc[c][0], (lane + g * np) & 31);
+    acc[c][0] = t;
+  }
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     double *y = to + c * to_stride + (long long)els[e] * np * inc + offset;

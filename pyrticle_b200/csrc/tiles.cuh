@@ -64,11 +64,11 @@ inline TilesDev tiles_dev(const TileSet &T) { return {T.tiles, T.count, T.rows, 
 // The sums of a plain deposition onto a tile set's targets, FP64: out[d] (or
 // NULL) receives, per target, rho (d = 0) and the three j. `run_starts` (or
 // NULL) gives the nodes per target for the counters (or NULL): pairs within
-// the radius, (particle, node) pairs, evaluated pairs. `order` (or NULL): the
-// launch order of the tiles.
-int launch_deposit_tiles(const TileSet &T, const uint32_t *run_starts, const BinGrid &G,
-                         const DepParticles &P, const ShapeParams &S, double *const out[4],
-                         unsigned long long *counters, const uint32_t *order, cudaStream_t s);
+// the radius, (particle, node) pairs, evaluated pairs. With a workspace the
+// blocks are launched heaviest first.
+int launch_deposit_tiles(prt_workspace *ws, const TileSet &T, const uint32_t *run_starts,
+                         const BinGrid &G, const DepParticles &P, const ShapeParams &S,
+                         double *const out[4], unsigned long long *counters, cudaStream_t s);
 
 // The weight (t)^alpha for t > 0, else 0.
 template <bool ALPHA2>
