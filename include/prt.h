@@ -547,6 +547,16 @@ int prt_average_forces(const prt_mesh *mesh, prt_workspace *ws, prt_shape_functi
                        const uint32_t *elements, const double *const fields[6],
                        double *forces, double *vis, double *scales, void *stream);
 
+/* The same for a store whose neighbours lie together (`ordered` != 0: sorted
+ * by prt_sort_by_element, or otherwise compact in runs of 32): it is taken in
+ * its own order. With 0, as prt_average_forces does, the particles are put in
+ * the order of spatial bins first. */
+int prt_average_forces_ordered(const prt_mesh *mesh, prt_workspace *ws, prt_shape_function shape,
+                       const double *integral_weights, int64_t n, const double *positions,
+                       const double *charges, const double *velocities,
+                       const uint32_t *elements, const double *const fields[6],
+                       double *forces, double *vis, double *scales, int32_t ordered, void *stream);
+
 /* One low-storage RK stage from given forces (a pusher whose forces come
  * from a separate pass): k = a k + dt (v(p), F), (x, p) += b k, relocation,
  * as prt_lsrk_stage after its force. */

@@ -183,6 +183,8 @@ SIGNATURES = {
                                          _vp, _vp, _vp, _vp, _vp, _vp]),
     "prt_average_forces": (_i32, [_vp, _vp, ShapeFunctionDesc, _dp, _i64, _vp, _vp, _vp, _vp,
                                   C.POINTER(_vp), _vp, _vp, _vp, _vp]),
+    "prt_average_forces_ordered": (_i32, [_vp, _vp, ShapeFunctionDesc, _dp, _i64, _vp, _vp, _vp,
+                                          _vp, C.POINTER(_vp), _vp, _vp, _vp, _i32, _vp]),
     "prt_lsrk_update": (_i32, [_vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _d, _d, _d,
                                _d, _vp]),
     "prt_kinetic_energies": (_i32, [_i64, _vp, _vp, _vp, _d, _vp, _vp]),

@@ -9,7 +9,7 @@
 //
 // Gather and scatter swap roles: the forward deposition gathers particles
 // onto node positions, its adjoint gathers node adjoints onto particles
-// (one lane per particle, position groups staged per warp); the forward
+// (particles in registers, positions staged per block, tiles.cuh); the forward
 // interpolation gathers nodal fields onto particles, its adjoint scatters particle
 // adjoints onto the nodes (warp-segmented sums, then FP64 atomics, only when
 // nodal field gradients are requested). Gradients along a few basis fields
@@ -27,8 +27,8 @@
 
 #include <cmath>
 
-#include "gather.cuh"
 #include "push.cuh"
+#include "tiles.cuh"
 
 namespace {
 
@@ -333,16 +333,17 @@ __global__ void velocities_adjoint_kernel(long long n, const double *__restrict_
   lp[2 * n + i] += cs * (w2 - p2 * pw);
 }
 
-// Adjoint of the expansion from positions to nodes: every position sums the
-// node adjoints of its nodes (ascending node order): G[0] from dL/drho,
-// G[1..3] from dL/dj.
-__global__ void contract_kernel(long long npos, long long nn,
+// Adjoint of the expansion from positions to nodes, per tile row: every
+// position sums the node adjoints of its nodes (ascending node order). Records
+// (x, y, z, G0 from dL/drho, G1..G3 from dL/dj).
+__global__ void contract_kernel(prt_dep::TilesDev T, long long nn,
                                 const uint32_t *__restrict__ run_starts,
                                 const uint32_t *__restrict__ run_nodes,
                                 const double *__restrict__ grho, const double *__restrict__ gj,
-                                double *__restrict__ G) {
-  const long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (u >= npos) return;
+                                double2 *__restrict__ records) {
+  const long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (r >= T.count) return;
+  const uint32_t u = T.rows[r];
   double s[4] = {0, 0, 0, 0};
   for (uint32_t k = run_starts[u]; k < run_starts[u + 1]; ++k) {
     const uint32_t node = run_nodes[k];
@@ -353,70 +354,86 @@ __global__ void contract_kernel(long long npos, long long nn,
       s[3] += gj[2 * nn + node];
     }
   }
-#pragma unroll
-  for (int d = 0; d < 4; ++d) G[d * npos + u] = s[d];
+  records[4 * r] = make_double2(T.pos[3 * r], T.pos[3 * r + 1]);
+  records[4 * r + 1] = make_double2(T.pos[3 * r + 2], s[0]);
+  records[4 * r + 2] = make_double2(s[1], s[2]);
+  records[4 * r + 3] = make_double2(s[3], 0);
 }
-
-constexpr int DEP_ADJ_BLOCK = 128;
 
 // Adjoint of the plain shape deposition. With weight w = q N and
 // S = (a - r^2/a)^alpha:
 //   dL/dx_p = w sum_u (G0_u + G_u . v_p) dS/dx_p,
 //   dL/dv_p = w sum_u G_u S,   dS/dx_p = alpha (a - r^2/a)^(alpha-1) (2/a) (x_u - x_p),
-// gathered per particle (lane) over the positions within the radius
-// (warp_gather_positions, gather.cuh).
-template <bool ALPHA2>
-__global__ void __launch_bounds__(DEP_ADJ_BLOCK, 4)
-    deposit_adjoint_kernel(DevMesh M, CentreBinsDev CB, const double *__restrict__ pos,
-                           long long npos, prt_dep::ShapeParams S, double normalizer,
-                           const double *__restrict__ G, long long n,
+// with the particles as targets, in bin order, and the positions as sources
+// (tiles.cuh): 18 FP64 operations per evaluated pair.
+constexpr int DEP_ADJ_PER = 4;
+template <bool ALPHA2, bool SHARE>
+__global__ void __launch_bounds__(32 * prt_dep::BW, 3)
+    deposit_adjoint_kernel(DevMesh M, prt_dep::TilesDev T, prt_dep::TileBinsDev B,
+                           const double2 *__restrict__ records, prt_dep::ShapeWeight S,
+                           double normalizer, long long n, const uint32_t *__restrict__ perm,
                            const double *__restrict__ x, const double *__restrict__ q,
                            const double *__restrict__ v, const uint32_t *__restrict__ el,
                            double *__restrict__ lx, double *__restrict__ lv) {
-  __shared__ GatherStage<4> stage[DEP_ADJ_BLOCK / 32];
-  const int warp = threadIdx.x >> 5;
-  const long long i = blockIdx.x * (long long)DEP_ADJ_BLOCK + threadIdx.x;
-  const bool live = i < n && (!el || el[i] != PRT_INVALID);
-  double p[3] = {0, 0, 0}, vv[3] = {0, 0, 0};
-  if (live) {
+  using namespace prt_dep;
+  constexpr int PER = DEP_ADJ_PER, LANES = 32 / PER;
+  __shared__ BlockStage<4> stage;
+  __shared__ TileRows rows;
+  __shared__ double boxes[BW][6];
+  BlockBox X;
+  ParticleTargets<PER> D;
+  stage_begin(stage);
+  if (!load_particles<PER, SHARE>(D, X, boxes, n, perm, x, el, S)) return;  // whole block
+  double vv[3][PER], acc[6][PER];
+#pragma unroll
+  for (int h = 0; h < PER; ++h) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) vv[d][h] = v && D.live[h] ? v[d * n + D.id[h]] : 0;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) acc[k][h] = 0;
+  }
+  const double mha = -0.5 * S.radius;  // x_u - x_p = w + V (-a/2), V = 2 (x_p - c) / a
+  evaluate_positions<PER, 4, SHARE>(
+      stage, rows, T, B, records, M, X, S.radius, S.inv_radius,
+      [&](double w0, double w1, double w2, double e, const double *g) {
+#pragma unroll
+        for (int h = 0; h < PER; ++h) {
+          const double tr =
+              fma(D.V[0][h], w0, fma(D.V[1][h], w1, fma(D.V[2][h], w2, D.B[h] + e)));
+          // pm = t^(alpha - 1), sv = t^alpha for t > 0
+          double pm, sv;
+          if (ALPHA2) {
+            pm = tr > 0 ? tr : 0.0;
+            sv = pm * pm;
+          } else {
+            pm = tr > 0 ? pow(tr, S.alpha - 1.0) : 0.0;
+            sv = pm * tr;
+          }
+          const double hd =
+              pm * fma(g[2], vv[1][h], fma(g[1], vv[0][h], fma(g[3], vv[2][h], g[0])));
+          acc[0][h] = fma(hd, fma(D.V[0][h], mha, w0), acc[0][h]);
+          acc[1][h] = fma(hd, fma(D.V[1][h], mha, w1), acc[1][h]);
+          acc[2][h] = fma(hd, fma(D.V[2][h], mha, w2), acc[2][h]);
+          acc[3][h] = fma(g[1], sv, acc[3][h]);
+          acc[4][h] = fma(g[2], sv, acc[4][h]);
+          acc[5][h] = fma(g[3], sv, acc[5][h]);
+        }
+      });
+  reduce_groups<PER, 6>(acc);
+  if (SHARE) {
+    share_sums<6, PER>(stage, acc);
+    if (threadIdx.x >= 32) return;
+  }
+  const int grp = (threadIdx.x & 31) / LANES;
+#pragma unroll
+  for (int h = 0; h < PER; ++h) {
+    if (h != grp || !D.live[h]) continue;
+    const long long i = D.id[h];
+    const double w = q[i] * normalizer, wx = w * S.alpha * (2.0 * S.inv_radius);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      p[d] = x[d * n + i];
-      if (v) vv[d] = v[d * n + i];
-    }
-  }
-  double ax0 = 0, ax1 = 0, ax2 = 0, as1 = 0, as2 = 0, as3 = 0;
-  warp_gather_positions<4>(
-      M, CB, pos, npos, G, S.radius, live, p, stage[warp],
-      [&](double f0, double f1, double f2, double r2, const double *g) {
-        const double rt = fmax(fma(-r2, S.inv_radius, S.radius), 0.0);
-        double sv, ds;
-        if (ALPHA2) {
-          sv = rt * rt;
-          ds = rt * (4.0 * S.inv_radius);
-        } else {
-          const double pm = rt > 0 ? pow(rt, S.alpha - 1.0) : 0.0;
-          sv = pm * rt;
-          ds = S.alpha * pm * (2.0 * S.inv_radius);
-        }
-        const double h = fma(g[2], vv[1], fma(g[1], vv[0], fma(g[3], vv[2], g[0])));
-        const double hd = h * ds;
-        ax0 = fma(hd, f0, ax0);
-        ax1 = fma(hd, f1, ax1);
-        ax2 = fma(hd, f2, ax2);
-        as1 = fma(g[1], sv, as1);
-        as2 = fma(g[2], sv, as2);
-        as3 = fma(g[3], sv, as3);
-      });
-  if (live) {
-    const double w = q[i] * normalizer;
-    lx[i] += w * ax0;
-    lx[n + i] += w * ax1;
-    lx[2 * n + i] += w * ax2;
-    if (lv) {
-      lv[i] += w * as1;
-      lv[n + i] += w * as2;
-      lv[2 * n + i] += w * as3;
+      lx[d * n + i] += wx * acc[d][0];
+      if (lv) lv[d * n + i] += w * acc[3 + d][0];
     }
   }
 }
@@ -597,27 +614,31 @@ extern "C" int prt_deposit_shape_adjoint(const prt_mesh *mesh, prt_workspace *ws
   cudaStream_t s = (cudaStream_t)stream;
   ScopedTimer timer(ws, PRT_TIME_DEPOSIT_ADJOINT, s);
   int rc;
-  double *G = (double *)ws_buffer(ws, PRT_WS_ADJ_POSITIONS, sizeof(double) * 4 * PS.count, &rc);
-  if (!G) return rc;
+  double2 *records =
+      (double2 *)ws_buffer(ws, PRT_WS_ADJ_POSITIONS, 4 * sizeof(double2) * PS.count, &rc);
+  if (!records) return rc;
+  const prt_dep::TilesDev T = prt_dep::tiles_dev(PS.tiles);
   contract_kernel<<<prt_grid_blocks(PS.count, 256), 256, 0, s>>>(
-      PS.count, nn, PS.run_starts, PS.run_nodes, grad_rho, grad_j, G);
+      T, nn, PS.run_starts, PS.run_nodes, grad_rho, grad_j, records);
   PRT_CHECK_CUDA(cudaGetLastError());
-  prt_dep::ShapeParams S;
-  S.radius = shape.radius;
-  S.radius2 = shape.radius * shape.radius;
-  S.inv_radius = 1.0 / shape.radius;
-  S.alpha = shape.alpha;
-  for (int d = 0; d < 3; ++d) S.reach[d] = shape.radius;
-  const CentreBinsDev CB = centre_bins_dev(PS);
+  prt_dep::BinGrid G;
+  const uint32_t *perm, *starts;
+  if (!prt_dep::choose_bins(mesh, mesh->box_lo, mesh->box_hi,
+                            shape.radius * prt_dep::BIN_FRACTION, 0.0, G, &rc))
+    return rc;
+  if ((rc = prt_dep::bin_particles(ws, G, n, x, el, &perm, &starts, s))) return rc;
   const double *vv = grad_j ? v : nullptr;
   double *lvv = grad_j ? lam_v : nullptr;
-  const unsigned blocks = (unsigned)((n + DEP_ADJ_BLOCK - 1) / DEP_ADJ_BLOCK);
-  if (shape.alpha == 2)
-    deposit_adjoint_kernel<true><<<blocks, DEP_ADJ_BLOCK, 0, s>>>(
-        mesh->dev, CB, PS.pos, PS.count, S, shape.normalizer, G, n, x, q, vv, el, lam_x, lvv);
-  else
-    deposit_adjoint_kernel<false><<<blocks, DEP_ADJ_BLOCK, 0, s>>>(
-        mesh->dev, CB, PS.pos, PS.count, S, shape.normalizer, G, n, x, q, vv, el, lam_x, lvv);
+  const bool share = n < prt_dep::SHARE_PARTICLES;
+  const long long per = share ? 32 : prt_dep::CHUNK_N;
+  auto kern = shape.alpha == 2
+                  ? (share ? deposit_adjoint_kernel<true, true> : deposit_adjoint_kernel<true, false>)
+                  : (share ? deposit_adjoint_kernel<false, true>
+                           : deposit_adjoint_kernel<false, false>);
+  kern<<<(unsigned)((n + per - 1) / per), 32 * prt_dep::BW, 0, s>>>(
+      mesh->dev, T, prt_dep::tile_bins_dev(PS.tiles), records,
+      prt_dep::ShapeWeight{shape.radius, 1.0 / shape.radius, shape.alpha}, shape.normalizer, n,
+      perm, x, q, vv, el, lam_x, lvv);
   PRT_CHECK_CUDA(cudaGetLastError());
   return PRT_OK;
 }

@@ -9,79 +9,113 @@
 // (the charge cancels). The same sums regroup by node position:
 //   <F> = sum_u S(x_u - x_p) WF_u / sum_u S(x_u - x_p) W_u,
 // W_u = sum over the nodes at u of |J| w, WF_u = sum |J| w F. A per-position
-// pass builds W, WE, WB and the weighted squares (for the verbose standard
-// deviations); a particle-centric gather (gather.cuh, lane = particle) forms
-// the averages. No atomics; deterministic.
+// pass builds records of W, WE, WB (and, for the verbose standard deviations,
+// the weighted squares); the particles gather them as targets of the FP64 pair
+// sums (tiles.cuh). No atomics; deterministic.
 
 #include <cmath>
 
-#include "gather.cuh"
 #include "push.cuh"
+#include "tiles.cuh"
 
 namespace {
 
-constexpr int AVG_BLOCK = 128;
-constexpr int AVG_NV = 9;  // W, WE[3], WB[3], W|E|^2, W|B|^2
+using namespace prt_dep;
 
-__global__ void average_prepare_kernel(long long npos, int np,
-                                       const uint32_t *__restrict__ run_starts,
+// values per position: W, WE[3], WB[3] and, with squares, W|E|^2, W|B|^2
+template <bool SQUARES>
+constexpr int AVG_NV = SQUARES ? 9 : 7;
+
+// Per tile row the record (x, y, z, values).
+template <bool SQUARES>
+__global__ void average_records_kernel(TilesDev T, int np, const uint32_t *__restrict__ run_starts,
                                        const uint32_t *__restrict__ run_nodes,
                                        const double *__restrict__ iw,
                                        const double *__restrict__ jac, Fields6 F,
-                                       double *__restrict__ G) {
-  const long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (u >= npos) return;
-  double s[AVG_NV];
+                                       double2 *__restrict__ records) {
+  constexpr int NV = AVG_NV<SQUARES>, RAW = BlockStage<NV>::RAW;
+  const long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (r >= T.count) return;
+  const uint32_t u = T.rows[r];
+  double s[2 * RAW];
 #pragma unroll
-  for (int k = 0; k < AVG_NV; ++k) s[k] = 0;
+  for (int k = 0; k < 2 * RAW; ++k) s[k] = k < 3 ? T.pos[3 * r + k] : 0;
   for (uint32_t k = run_starts[u]; k < run_starts[u + 1]; ++k) {
     const uint32_t node = run_nodes[k];
     const double w = iw[node % np] * jac[node / np];
     double f[6];
 #pragma unroll
     for (int c = 0; c < 6; ++c) f[c] = F.f[c] ? F.f[c][node] : 0.0;
-    s[0] += w;
+    s[3] += w;
 #pragma unroll
-    for (int c = 0; c < 6; ++c) s[1 + c] += w * f[c];
-    s[7] += w * (f[0] * f[0] + f[1] * f[1] + f[2] * f[2]);
-    s[8] += w * (f[3] * f[3] + f[4] * f[4] + f[5] * f[5]);
+    for (int c = 0; c < 6; ++c) s[4 + c] += w * f[c];
+    if (SQUARES) {
+      s[10] += w * (f[0] * f[0] + f[1] * f[1] + f[2] * f[2]);
+      s[11] += w * (f[3] * f[3] + f[4] * f[4] + f[5] * f[5]);
+    }
   }
 #pragma unroll
-  for (int k = 0; k < AVG_NV; ++k) G[k * npos + u] = s[k];
+  for (int k = 0; k < RAW; ++k) records[RAW * r + k] = make_double2(s[2 * k], s[2 * k + 1]);
 }
 
+template <bool SQUARES>
+struct AverageShared {
+  BlockStage<AVG_NV<SQUARES>> stage;
+  TileRows rows;
+  double boxes[BW][6];
+};
+
 // vis rows [14][n]: pt_e (3), pt_b (3), pt_e_stddev, pt_b_stddev, el_force
-// (3), mag_force (3) (push_average.hpp:388-421)
-template <bool ALPHA2>
-__global__ void __launch_bounds__(AVG_BLOCK, 4)
-    average_forces_kernel(DevMesh M, CentreBinsDev CB, const double *__restrict__ pos,
-                          long long npos, prt_dep::ShapeParams S, double normalizer,
-                          const double *__restrict__ G, long long n,
+// (3), mag_force (3) (push_average.hpp:388-421), written where SQUARES
+constexpr int AVG_PER = 4;
+template <bool ALPHA2, bool SQUARES, bool SHARE>
+__global__ void __launch_bounds__(32 * BW, 3)
+    average_forces_kernel(DevMesh M, TilesDev T, TileBinsDev B,
+                          const double2 *__restrict__ records, ShapeWeight S, double normalizer,
+                          long long n, const uint32_t *__restrict__ perm,
                           const double *__restrict__ x, const double *__restrict__ q,
                           const double *__restrict__ v, const uint32_t *__restrict__ el,
                           double *__restrict__ forces, double *__restrict__ vis,
                           double *__restrict__ scales, DevStatus *st) {
-  __shared__ GatherStage<AVG_NV> stage[AVG_BLOCK / 32];
-  const int warp = threadIdx.x >> 5;
-  const long long i = blockIdx.x * (long long)AVG_BLOCK + threadIdx.x;
-  const bool live = i < n && (!el || el[i] != PRT_INVALID);
-  double p[3] = {0, 0, 0};
-  if (live) {
+  constexpr int PER = AVG_PER, LANES = 32 / PER, NV = AVG_NV<SQUARES>;
+  extern __shared__ __align__(16) unsigned char avg_smem[];
+  AverageShared<SQUARES> &A = *reinterpret_cast<AverageShared<SQUARES> *>(avg_smem);
+  BlockBox X;
+  ParticleTargets<PER> D;
+  stage_begin(A.stage);
+  if (!load_particles<PER, SHARE>(D, X, A.boxes, n, perm, x, el, S)) return;  // whole block
+  double sum[NV][PER];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) p[d] = x[d * n + i];
-  }
-  double acc[AVG_NV];
+  for (int k = 0; k < NV; ++k)
 #pragma unroll
-  for (int k = 0; k < AVG_NV; ++k) acc[k] = 0;
-  warp_gather_positions<AVG_NV>(
-      M, CB, pos, npos, G, S.radius, live, p, stage[warp],
-      [&](double, double, double, double r2, const double *g) {
-        const double rt = fmax(fma(-r2, S.inv_radius, S.radius), 0.0);
-        const double sw = normalizer * (ALPHA2 ? rt * rt : (rt > 0 ? pow(rt, S.alpha) : 0.0));
+    for (int h = 0; h < PER; ++h) sum[k][h] = 0;
+  evaluate_positions<PER, NV, SHARE>(
+      A.stage, A.rows, T, B, records, M, X, S.radius, S.inv_radius,
+      [&](double w0, double w1, double w2, double e, const double *g) {
 #pragma unroll
-        for (int k = 0; k < AVG_NV; ++k) acc[k] = fma(sw, g[k], acc[k]);
+        for (int h = 0; h < PER; ++h) {
+          const double tr =
+              fma(D.V[0][h], w0, fma(D.V[1][h], w1, fma(D.V[2][h], w2, D.B[h] + e)));
+          const double sw = shape_power<ALPHA2>(tr, S.alpha);
+#pragma unroll
+          for (int k = 0; k < NV; ++k) sum[k][h] = fma(sw, g[k], sum[k][h]);
+        }
       });
-  if (!live) return;
+  reduce_groups<PER, NV>(sum);
+  if (SHARE) {
+    share_sums<NV, PER>(A.stage, sum);
+    if (threadIdx.x >= 32) return;
+  }
+  // this lane's particle
+  const int grp = (threadIdx.x & 31) / LANES;
+  long long i = -1;
+#pragma unroll
+  for (int h = 0; h < PER; ++h)
+    if (h == grp && D.live[h]) i = D.id[h];
+  if (i < 0) return;
+  double acc[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) acc[k] = normalizer * sum[k][0];
   const double charge = q[i];
   double f[3] = {0, 0, 0}, ef[6] = {0, 0, 0, 0, 0, 0}, sde = 0, sdb = 0;
   const double den = charge * acc[0];  // the reconstructed charge
@@ -103,15 +137,17 @@ __global__ void __launch_bounds__(AVG_BLOCK, 4)
     mag_f[2] = vv[0] * qb[1] - vv[1] * qb[0];
 #pragma unroll
     for (int d = 0; d < 3; ++d) f[d] = el_f[d] + mag_f[d];
-    const double ve = acc[7] / acc[0] - (ef[0] * ef[0] + ef[1] * ef[1] + ef[2] * ef[2]);
-    const double vb = acc[8] / acc[0] - (ef[3] * ef[3] + ef[4] * ef[4] + ef[5] * ef[5]);
-    sde = ve < 0 ? 0.0 : sqrt(ve);
-    sdb = vb < 0 ? 0.0 : sqrt(vb);
+    if (SQUARES) {
+      const double ve = acc[NV - 2] / acc[0] - (ef[0] * ef[0] + ef[1] * ef[1] + ef[2] * ef[2]);
+      const double vb = acc[NV - 1] / acc[0] - (ef[3] * ef[3] + ef[4] * ef[4] + ef[5] * ef[5]);
+      sde = ve < 0 ? 0.0 : sqrt(ve);
+      sdb = vb < 0 ? 0.0 : sqrt(vb);
+    }
   }
 #pragma unroll
   for (int d = 0; d < 3; ++d) forces[d * n + i] = f[d];
   if (scales) scales[i] = den == 0 ? 0.0 : charge / den;
-  if (vis) {
+  if (SQUARES) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       vis[d * n + i] = ef[d];
@@ -164,49 +200,87 @@ __global__ void __launch_bounds__(256)
 
 }  // namespace
 
+namespace {
+
+template <bool SQUARES>
+int average_forces(const prt_mesh *mesh, prt_workspace *ws, const prt_shape_function &shape,
+                   const double *integral_weights, long long n, const double *positions,
+                   const double *charges, const double *velocities, const uint32_t *elements,
+                   const Fields6 &F, const uint32_t *perm, double *forces, double *vis,
+                   double *scales, cudaStream_t s) {
+  constexpr int NV = AVG_NV<SQUARES>;
+  const PositionSet &PS = mesh->positions;
+  const int np = mesh->dev.Np;
+  int rc;
+  const size_t rec = BlockStage<NV>::RAW * (size_t)PS.count;
+  double2 *records =
+      (double2 *)ws_buffer(ws, PRT_WS_AVERAGE, sizeof(double2) * rec + sizeof(double) * np, &rc);
+  if (!records) return rc;
+  double *iwd = (double *)(records + rec);
+  PRT_CHECK_CUDA(
+      cudaMemcpyAsync(iwd, integral_weights, sizeof(double) * np, cudaMemcpyHostToDevice, s));
+  const TilesDev T = tiles_dev(PS.tiles);
+  average_records_kernel<SQUARES><<<prt_grid_blocks(PS.count, 128), 128, 0, s>>>(
+      T, np, PS.run_starts, PS.run_nodes, iwd, mesh->dev.jacobians, F, records);
+  PRT_CHECK_CUDA(cudaGetLastError());
+  const bool share = n < SHARE_PARTICLES;
+  const long long per = share ? 32 : CHUNK_N;
+  auto kern = shape.alpha == 2 ? (share ? average_forces_kernel<true, SQUARES, true>
+                                        : average_forces_kernel<true, SQUARES, false>)
+                               : (share ? average_forces_kernel<false, SQUARES, true>
+                                        : average_forces_kernel<false, SQUARES, false>);
+  constexpr int smem = (int)sizeof(AverageShared<SQUARES>);
+  PRT_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  kern<<<(unsigned)((n + per - 1) / per), 32 * BW, smem, s>>>(
+      mesh->dev, T, tile_bins_dev(PS.tiles), records,
+      ShapeWeight{shape.radius, 1.0 / shape.radius, shape.alpha}, shape.normalizer, n, perm,
+      positions, charges, velocities, elements, forces, vis, scales, ws->status);
+  PRT_CHECK_CUDA(cudaGetLastError());
+  return PRT_OK;
+}
+
+}  // namespace
+
+extern "C" int prt_average_forces_ordered(const prt_mesh *mesh, prt_workspace *ws,
+                                          prt_shape_function shape,
+                                          const double *integral_weights, int64_t n,
+                                          const double *positions, const double *charges,
+                                          const double *velocities, const uint32_t *elements,
+                                          const double *const fields[6], double *forces,
+                                          double *vis, double *scales, int32_t ordered,
+                                          void *stream) {
+  if (!mesh || !ws || n < 0 || !(shape.radius > 0) || !integral_weights || !fields)
+    return PRT_ERR_INVALID_ARGUMENT;
+  if (n == 0) return PRT_OK;
+  if (!positions || !charges || !velocities || !forces || n >= (1ll << 31))
+    return PRT_ERR_INVALID_ARGUMENT;
+  cudaStream_t s = (cudaStream_t)stream;
+  int rc;
+  // a warp's 32 particles have to lie together: in a store without a spatial
+  // order the bins' order is taken
+  const uint32_t *perm = nullptr, *starts;
+  if (!ordered) {
+    BinGrid G;
+    if (!choose_bins(mesh, mesh->box_lo, mesh->box_hi, shape.radius * BIN_FRACTION, 0.0, G, &rc))
+      return rc;
+    if ((rc = bin_particles(ws, G, n, positions, elements, &perm, &starts, s))) return rc;
+  }
+  Fields6 F;
+  for (int k = 0; k < 6; ++k) F.f[k] = fields[k];
+  return vis ? average_forces<true>(mesh, ws, shape, integral_weights, n, positions, charges,
+                                    velocities, elements, F, perm, forces, vis, scales, s)
+             : average_forces<false>(mesh, ws, shape, integral_weights, n, positions, charges,
+                                     velocities, elements, F, perm, forces, vis, scales, s);
+}
+
 extern "C" int prt_average_forces(const prt_mesh *mesh, prt_workspace *ws,
                                   prt_shape_function shape, const double *integral_weights,
                                   int64_t n, const double *positions, const double *charges,
                                   const double *velocities, const uint32_t *elements,
                                   const double *const fields[6], double *forces, double *vis,
                                   double *scales, void *stream) {
-  if (!mesh || !ws || n < 0 || !(shape.radius > 0) || !integral_weights || !fields)
-    return PRT_ERR_INVALID_ARGUMENT;
-  if (n == 0) return PRT_OK;
-  if (!positions || !charges || !velocities || !forces) return PRT_ERR_INVALID_ARGUMENT;
-  const PositionSet &PS = mesh->positions;
-  const int np = mesh->dev.Np;
-  cudaStream_t s = (cudaStream_t)stream;
-  int rc;
-  double *buf = (double *)ws_buffer(ws, PRT_WS_AVERAGE,
-                                    sizeof(double) * ((size_t)AVG_NV * PS.count + np), &rc);
-  if (!buf) return rc;
-  double *G = buf, *iwd = buf + (size_t)AVG_NV * PS.count;
-  PRT_CHECK_CUDA(
-      cudaMemcpyAsync(iwd, integral_weights, sizeof(double) * np, cudaMemcpyHostToDevice, s));
-  Fields6 F;
-  for (int k = 0; k < 6; ++k) F.f[k] = fields[k];
-  average_prepare_kernel<<<prt_grid_blocks(PS.count, 256), 256, 0, s>>>(
-      PS.count, np, PS.run_starts, PS.run_nodes, iwd, mesh->dev.jacobians, F, G);
-  PRT_CHECK_CUDA(cudaGetLastError());
-  prt_dep::ShapeParams S;
-  S.radius = shape.radius;
-  S.radius2 = shape.radius * shape.radius;
-  S.inv_radius = 1.0 / shape.radius;
-  S.alpha = shape.alpha;
-  for (int d = 0; d < 3; ++d) S.reach[d] = shape.radius;
-  const CentreBinsDev CB = centre_bins_dev(PS);
-  const unsigned blocks = (unsigned)((n + AVG_BLOCK - 1) / AVG_BLOCK);
-  if (shape.alpha == 2)
-    average_forces_kernel<true><<<blocks, AVG_BLOCK, 0, s>>>(
-        mesh->dev, CB, PS.pos, PS.count, S, shape.normalizer, G, n, positions, charges,
-        velocities, elements, forces, vis, scales, ws->status);
-  else
-    average_forces_kernel<false><<<blocks, AVG_BLOCK, 0, s>>>(
-        mesh->dev, CB, PS.pos, PS.count, S, shape.normalizer, G, n, positions, charges,
-        velocities, elements, forces, vis, scales, ws->status);
-  PRT_CHECK_CUDA(cudaGetLastError());
-  return PRT_OK;
+  return prt_average_forces_ordered(mesh, ws, shape, integral_weights, n, positions, charges,
+                                    velocities, elements, fields, forces, vis, scales, 0, stream);
 }
 
 extern "C" int prt_lsrk_update(const prt_mesh *mesh, prt_workspace *ws, int64_t n,

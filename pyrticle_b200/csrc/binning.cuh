@@ -67,6 +67,17 @@ __device__ __forceinline__ int floor_div(int a, int b) {
 int choose_bins(const prt_mesh *m, const double lo[3], const double hi[3], double bin_width,
                 double radius, BinGrid &G, int *rc);
 
+// Bins and sorts the live particles: the store index per particle in bin order
+// (removed ones last) and the bins' starts (workspace scratch).
+int bin_particles(prt_workspace *ws, const BinGrid &G, long long n, const double *x,
+                  const uint32_t *el, const uint32_t **perm, const uint32_t **starts,
+                  cudaStream_t s);
+
+// Packs the particles in that order into P (workspace scratch); see below.
+int pack_particles(prt_workspace *ws, long long n, const uint32_t *perm, const uint32_t *starts,
+                   const double *x, const double *q, const double *v, const double *scale,
+                   double normalizer, const uint32_t *tag, DepParticles &P, cudaStream_t s);
+
 // Bins, sorts and packs the live particles into P (workspace scratch).
 // `scale` (or NULL: q) times `normalizer` is the payload weight; `tag` (or
 // NULL) fills the last payload slot.

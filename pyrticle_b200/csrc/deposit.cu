@@ -46,7 +46,6 @@
 
 #include "binning.cuh"
 #include "bisect.cuh"
-#include "gather.cuh"
 #include "tiles.cuh"
 
 namespace prt_dep {
@@ -139,10 +138,9 @@ int choose_bins(const prt_mesh *m, const double box_lo[3], const double box_hi[3
   return 1;
 }
 
-int stage_particles(prt_workspace *ws, const BinGrid &G, long long n, const double *x,
-                    const double *q, const double *v, const uint32_t *el,
-                    const double *scale, double normalizer, const uint32_t *tag,
-                    DepParticles &P, cudaStream_t s) {
+int bin_particles(prt_workspace *ws, const BinGrid &G, long long n, const double *x,
+                  const uint32_t *el, const uint32_t **perm, const uint32_t **bin_starts,
+                  cudaStream_t s) {
   int rc;
   uint32_t *keys = (uint32_t *)ws_buffer(ws, PRT_WS_DEP_KEYS, 8 * (size_t)n, &rc);
   if (!keys) return rc;
@@ -166,16 +164,35 @@ int stage_particles(prt_workspace *ws, const BinGrid &G, long long n, const doub
   bin_starts_kernel<<<prt_grid_blocks(G.nbins + 1, 256), 256, 0, s>>>(G.nbins, n, keys_out,
                                                                       starts);
   PRT_CHECK_CUDA(cudaGetLastError());
+  *perm = vals_out;
+  *bin_starts = starts;
+  return PRT_OK;
+}
+
+int pack_particles(prt_workspace *ws, long long n, const uint32_t *perm, const uint32_t *starts,
+                   const double *x, const double *q, const double *v, const double *scale,
+                   double normalizer, const uint32_t *tag, DepParticles &P, cudaStream_t s) {
+  int rc;
   double *payload =
       (double *)ws_buffer(ws, PRT_WS_DEP_PARTICLES, sizeof(double) * PAYLOAD * (size_t)n, &rc);
   if (!payload) return rc;
   // rows past starts[nbins] (removed particles) are packed but never read
-  payload_kernel<<<prt_grid_blocks(n, 256), 256, 0, s>>>(n, vals_out, x, q, v, scale,
-                                                         normalizer, tag, payload);
+  payload_kernel<<<prt_grid_blocks(n, 256), 256, 0, s>>>(n, perm, x, q, v, scale, normalizer, tag,
+                                                         payload);
   PRT_CHECK_CUDA(cudaGetLastError());
   P.payload = payload;
   P.starts = starts;
   return PRT_OK;
+}
+
+int stage_particles(prt_workspace *ws, const BinGrid &G, long long n, const double *x,
+                    const double *q, const double *v, const uint32_t *el,
+                    const double *scale, double normalizer, const uint32_t *tag,
+                    DepParticles &P, cudaStream_t s) {
+  const uint32_t *perm, *starts;
+  int rc;
+  if ((rc = bin_particles(ws, G, n, x, el, &perm, &starts, s))) return rc;
+  return pack_particles(ws, n, perm, starts, x, q, v, scale, normalizer, tag, P, s);
 }
 
 }  // namespace prt_dep
@@ -446,8 +463,9 @@ struct DepositTargets {
 };
 
 constexpr int BLOCK_PER = 4;  // targets per lane
-// Four tiles per block.
-template <bool ALPHA2, bool COUNT>
+// Four tiles per block; SHARE: one, its particles shared by the four warps,
+// for jobs with too few tiles to give every SM a block of four.
+template <bool ALPHA2, bool COUNT, bool SHARE>
 __global__ void __launch_bounds__(32 * BW, 3)
     deposit_blocks_kernel(TilesDev T, const uint32_t *__restrict__ run_starts, BinGrid G,
                           DepParticles P, ShapeWeight S, TileSums O,
@@ -458,7 +476,7 @@ __global__ void __launch_bounds__(32 * BW, 3)
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int tg = lane % LANES, grp = lane / LANES;
   const long long blk = order ? (long long)order[blockIdx.x] : (long long)blockIdx.x;
-  const long long t = BW * blk + wid;
+  const long long t0 = SHARE ? blk : BW * blk, t = SHARE ? blk : t0 + wid;
   const bool have = t < T.tiles;
   const long long p0 = t * TILE;
   const int npt = have ? (int)min((long long)TILE, T.count - p0) : 0;
@@ -466,7 +484,7 @@ __global__ void __launch_bounds__(32 * BW, 3)
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     double lo = INFINITY, hi = -INFINITY;
-    for (long long k = BW * blk; k < min(T.tiles, BW * blk + BW); ++k) {
+    for (long long k = t0; k < min(T.tiles, t0 + (SHARE ? 1 : BW)); ++k) {
       lo = fmin(lo, T.boxes[6 * k + d] - T.boxes[6 * k + 3 + d]);
       hi = fmax(hi, T.boxes[6 * k + d] + T.boxes[6 * k + 3 + d]);
     }
@@ -479,114 +497,19 @@ __global__ void __launch_bounds__(32 * BW, 3)
   DepositTargets<PER, ALPHA2, COUNT> D;
   D.load(T, p0, npt, tg, X.c, S);
   const uint32_t evaluated =
-      evaluate_particles<PER, 4>(stage, G, P, X, S.radius, S.inv_radius, D);
+      evaluate_particles<PER, 4, SHARE>(stage, G, P, X, S.radius, S.inv_radius, D);
   if (COUNT) D.count(T, run_starts, p0, npt, tg, evaluated, counters);
   reduce_groups<PER, 4>(D.sum);
+  if (SHARE) {
+    share_sums<4, PER>(stage, D.sum);
+    if (threadIdx.x >= 32) return;
+  }
   const int row = PER * tg + grp;
   if (row < npt) {
     const long long u = T.rows[p0 + row];
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       if (O.out[k]) O.out[k][u] = D.sum[k][0];
-  }
-}
-
-// A tile per block, its four warps sharing the tile's particles (each streams
-// every fourth batch, adds up at the end): for jobs with too few tiles to fill
-// the SMs, where a block of four tiles would run one after the other on an
-// otherwise idle SM.
-constexpr int TILE_WARPS = 4;
-template <bool ALPHA2, bool COUNT>
-__global__ void __launch_bounds__(32 * TILE_WARPS, 3)
-    deposit_split_kernel(TilesDev T, const uint32_t *__restrict__ run_starts, BinGrid G,
-                         DepParticles P, ShapeWeight S, TileSums O,
-                         unsigned long long *__restrict__ counters) {
-  constexpr int PER = 4, LANES = 32 / PER, RING = 64;
-  // ring entries: (wx, wy), (wz, -|w|^2/a), (q N, q N vx), (q N vy, q N vz)
-  __shared__ double2 ring[TILE_WARPS][4][RING];
-  __shared__ Segments segments[TILE_WARPS];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int tg = lane % LANES, grp = lane / LANES;
-  const long long t = blockIdx.x;
-  const long long p0 = t * TILE;
-  const int npt = (int)min((long long)TILE, T.count - p0);
-  double c[3], hfd[3];
-  float hf[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    c[d] = T.boxes[6 * t + d];
-    hfd[d] = T.boxes[6 * t + 3 + d] + 1e-5 * S.radius;
-    hf[d] = (float)hfd[d];
-  }
-  DepositTargets<PER, ALPHA2, COUNT> D;
-  D.load(T, p0, npt, tg, c, S);
-  double2(*R)[RING] = ring[wid];
-  int head = 0, count = 0;
-  unsigned long long evaluated = 0;
-  // the 32 entries from head: PER at a time, one per group of lanes
-  auto drain = [&]() {
-#pragma unroll 1
-    for (int i = 0; i < 32; i += PER) {
-      const int e = head + i + grp;
-      const double2 w01 = R[0][e], w2e = R[1][e], qx = R[2][e], yz = R[3][e];
-      const double v[4] = {qx.x, qx.y, yz.x, yz.y};
-      D(w01.x, w01.y, w2e.x, w2e.y, v);
-    }
-    head ^= 32;
-    count -= 32;
-  };
-  const float rc4 = near_limit(S.radius);
-  const double2 *__restrict__ pay = reinterpret_cast<const double2 *>(P.payload);
-  stream_particles(G, P, c, hfd, S.radius, segments[wid], wid, TILE_WARPS,
-                   [&](bool valid, uint32_t k, double w0, double w1, double w2, double q) {
-                     const bool in = valid && near_box(w0, w1, w2, hf, rc4);
-                     const unsigned bal = __ballot_sync(0xffffffffu, in);
-                     if (in) {
-                       const double2 jv = pay[4 * (size_t)k + 2], jt = pay[4 * (size_t)k + 3];
-                       const int slot =
-                           (head + count + __popc(bal & ((1u << lane) - 1u))) & (RING - 1);
-                       R[0][slot] = make_double2(w0, w1);
-                       R[1][slot] =
-                           make_double2(w2, -(w0 * w0 + w1 * w1 + w2 * w2) * S.inv_radius);
-                       R[2][slot] = make_double2(q, jv.x);
-                       R[3][slot] = make_double2(jv.y, jt.x);
-                     }
-                     count += __popc(bal);
-                     if (COUNT) evaluated += __popc(bal);
-                     __syncwarp();
-                     if (count >= 32) {
-                       drain();
-                       __syncwarp();
-                     }
-                   });
-  if (count > 0) {
-    // the rest, filled up with entries beyond every radius
-    if (lane >= count) {
-      const int e = head + lane;
-      R[0][e] = R[2][e] = R[3][e] = make_double2(0, 0);
-      R[1][e] = make_double2(0, -1e300);
-    }
-    __syncwarp();
-    drain();
-  }
-  if (COUNT) D.count(T, run_starts, p0, npt, tg, evaluated, counters);
-  reduce_groups<PER, 4>(D.sum);
-  const int row = PER * tg + grp;
-  __syncwarp();
-  // (the ring is done with: four sums per row)
-  double *part = reinterpret_cast<double *>(&ring[wid][0][0]);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) part[32 * k + row] = D.sum[k][0];
-  __syncthreads();
-  if (wid != 0 || lane >= npt) return;
-  const long long u = T.rows[p0 + lane];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    double v = 0;
-#pragma unroll
-    for (int w = 0; w < TILE_WARPS; ++w)
-      v += reinterpret_cast<const double *>(&ring[w][0][0])[32 * k + lane];
-    if (O.out[k]) O.out[k][u] = v;
   }
 }
 
@@ -767,60 +690,96 @@ __global__ void position_weights_kernel(long long npos, const uint32_t *__restri
   W[u] = s;
 }
 
+// The same per tile row, as the normalising pass's sources: (x, y, z, W).
+__global__ void weight_records_kernel(TilesDev T, const uint32_t *__restrict__ run_starts,
+                                      const uint32_t *__restrict__ run_nodes, int np,
+                                      const double *__restrict__ iw,
+                                      const double *__restrict__ jac,
+                                      double2 *__restrict__ records) {
+  const long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (r >= T.count) return;
+  const uint32_t u = T.rows[r];
+  double s = 0;
+  for (uint32_t k = run_starts[u]; k < run_starts[u + 1]; ++k) {
+    const uint32_t node = run_nodes[k];
+    s += iw[node % np] * jac[node / np];
+  }
+  records[2 * r] = make_double2(T.pos[3 * r], T.pos[3 * r + 1]);
+  records[2 * r + 1] = make_double2(T.pos[3 * r + 2], s);
+}
+
 // Normalising pre-pass (dep_normshape.hpp:125-199): per particle the
 // integral of its deposited shape, sum_u W_u N S(x_u - x_p), over the
 // positions within the radius; scale = q / integral, or 0 with a warning for
-// a zero integral (the reference skips such a particle). A warp takes 32
-// consecutive particles (element-sorted particles are close together), one
-// per lane, and walks the position groups near them with the positions and
-// W staged in shared memory (gather.cuh); each particle's sum runs in a fixed
-// order. hits_out: the positions within the radius (-1 for a dead particle).
-constexpr int NORM_WARPS = 4;
-template <bool ALPHA2>
-__global__ void __launch_bounds__(32 * NORM_WARPS)
-    normalize_kernel(DevMesh M, CentreBinsDev CB, const double *__restrict__ pos,
-                     long long npos, const double *__restrict__ W, ShapeParams S,
-                     double normalizer, long long n, const double *__restrict__ x,
+// a zero integral (the reference skips such a particle). Targets are 32
+// particles per warp in bin order (close together whatever the store's order),
+// sources the positions of the tiles near them (tiles.cuh): six FP64
+// operations per evaluated pair. hits_out: the positions within the radius
+// (-1 for a dead particle).
+constexpr int NORM_PER = 4;  // (8: 10% slower at 1M particles, spills)
+template <bool ALPHA2, bool SHARE>
+__global__ void __launch_bounds__(32 * BW, 3)
+    normalize_kernel(DevMesh M, TilesDev T, TileBinsDev B, const double2 *__restrict__ records,
+                     ShapeWeight S, double normalizer, long long n,
+                     const uint32_t *__restrict__ perm, const double *__restrict__ x,
                      const double *__restrict__ q, const uint32_t *__restrict__ el,
                      double *__restrict__ scale_out, double *__restrict__ hits_out,
                      DevStatus *st) {
-  __shared__ GatherStage<1> stage[NORM_WARPS];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const long long w0 = (blockIdx.x * (long long)NORM_WARPS + wid) * 32;
-  if (w0 >= n) return;  // whole warp
-  const long long i = w0 + lane;
-  const bool valid = i < n;
-  const bool live = valid && !(el && el[i] == PRT_INVALID);
-  double p[3] = {0, 0, 0};
-  if (live) {
-    p[0] = x[i];
-    p[1] = x[n + i];
-    p[2] = x[2 * n + i];
+  constexpr int PER = NORM_PER, LANES = 32 / PER;
+  __shared__ BlockStage<1> stage;
+  __shared__ TileRows rows;
+  __shared__ double boxes[BW][6];
+  const int lane = threadIdx.x & 31;
+  BlockBox X;
+  ParticleTargets<PER> D;
+  stage_begin(stage);
+  const bool any = load_particles<PER, SHARE>(D, X, boxes, n, perm, x, el, S);
+  double sum[2][PER];  // the integral, and the hits (exact)
+  unsigned hits[PER];
+#pragma unroll
+  for (int h = 0; h < PER; ++h) {
+    sum[0][h] = 0;
+    hits[h] = 0;
   }
-  double integral = 0, hits = 0;
-  warp_gather_positions<1>(M, CB, pos, npos, W, S.radius, live, p, stage[wid],
-                           [&](double, double, double, double r2, const double *vals) {
-                             const bool in = r2 <= S.radius2;
-                             const double rt = S.radius - r2 * S.inv_radius;
-                             const double sv =
-                                 in ? normalizer * (ALPHA2 ? rt * rt : pow(rt, S.alpha))
-                                    : 0.0;
-                             integral = fma(sv, vals[0], integral);
-                             hits += in ? 1.0 : 0.0;
-                           });
-  if (!valid) return;
-  if (!live) {
-    scale_out[i] = 0;
-    hits_out[i] = -1;
-    return;
+  if (any)
+    evaluate_positions<PER, 1, SHARE>(
+        stage, rows, T, B, records, M, X, S.radius, S.inv_radius,
+        [&](double w0, double w1, double w2, double e, const double *v) {
+#pragma unroll
+          for (int h = 0; h < PER; ++h) {
+            const double tr =
+                fma(D.V[0][h], w0, fma(D.V[1][h], w1, fma(D.V[2][h], w2, D.B[h] + e)));
+            sum[0][h] = fma(shape_power<ALPHA2>(tr, S.alpha), v[0], sum[0][h]);
+            hits[h] += __double2hiint(tr) >= 0;
+          }
+        });
+#pragma unroll
+  for (int h = 0; h < PER; ++h) sum[1][h] = (double)hits[h];
+  // lane (tg, grp): particle PER tg + grp of the warp's
+  reduce_groups<PER, 2>(sum);
+  if (SHARE) {
+    share_sums<2, PER>(stage, sum);
+    if (threadIdx.x >= 32) return;
   }
-  if (integral == 0) {
-    scale_out[i] = 0;
-    record_warning(st, PRT_WARN_ZERO_MASS, i);
-  } else {
-    scale_out[i] = q[i] / integral;
+  const int grp = lane / LANES;
+#pragma unroll
+  for (int h = 0; h < PER; ++h) {
+    if (h != grp || D.id[h] < 0) continue;
+    const long long i = D.id[h];
+    if (!D.live[h]) {
+      scale_out[i] = 0;
+      hits_out[i] = -1;
+      continue;
+    }
+    const double integral = normalizer * sum[0][0];
+    if (integral == 0) {
+      scale_out[i] = 0;
+      record_warning(st, PRT_WARN_ZERO_MASS, i);
+    } else {
+      scale_out[i] = q[i] / integral;
+    }
+    hits_out[i] = sum[1][0];
   }
-  hits_out[i] = hits;
 }
 
 // Count / sum / sum of squares / min / max of the applied scales (non-zero
@@ -898,7 +857,8 @@ int upload_vec(const std::vector<T> &v, const T **dst) {
 
 // ------------------------------------------------------------------- tiles
 
-int prt_build_tiles(const double *points, long long count, const uint32_t *ids, TileSet *out) {
+int prt_build_tiles(const double *points, long long count, const uint32_t *ids, bool bins,
+                    TileSet *out) {
   const int TILE_ = prt_dep::TILE;
   std::vector<uint32_t> rows((size_t)count);
   std::iota(rows.begin(), rows.end(), 0u);
@@ -931,11 +891,55 @@ int prt_build_tiles(const double *points, long long count, const uint32_t *ids, 
   int rc;
   if ((rc = upload_vec(rows, &out->rows))) return rc;
   if ((rc = upload_vec(pos, &out->pos))) return rc;
-  return upload_vec(boxes, &out->boxes);
+  if ((rc = upload_vec(boxes, &out->boxes))) return rc;
+  if (!bins) return PRT_OK;
+  // bins about as wide as the tiles' mean extent
+  auto &TB = out->bins;
+  long long nb = 1;
+  for (int a = 0; a < 3; ++a) {
+    double lo = INFINITY, hi = -INFINITY, sum = 0;
+    TB.max_half[a] = 0;
+    for (long long t = 0; t < nt; ++t) {
+      const double c = boxes[6 * (size_t)t + a], h = boxes[6 * (size_t)t + 3 + a];
+      lo = std::min(lo, c);
+      hi = std::max(hi, c);
+      sum += 2 * h;
+      TB.max_half[a] = std::max(TB.max_half[a], h);
+    }
+    const double ext = hi - lo, w = std::max(sum / std::max<long long>(1, nt), 1e-300);
+    TB.dims[a] = ext > 0 ? (int)std::max(1.0, std::min(512.0, std::floor(ext / w))) : 1;
+    TB.origin[a] = lo;
+    TB.inv_w[a] = ext;
+  }
+  for (;;) {  // (thin or few tiles: no more than some bins per tile)
+    nb = (long long)TB.dims[0] * TB.dims[1] * TB.dims[2];
+    if (nb <= 4 * nt + 64) break;
+    int a = 0;
+    for (int b = 1; b < 3; ++b)
+      if (TB.dims[b] > TB.dims[a]) a = b;
+    TB.dims[a] = (TB.dims[a] + 1) / 2;
+  }
+  for (int a = 0; a < 3; ++a) TB.inv_w[a] = TB.inv_w[a] > 0 ? TB.dims[a] / TB.inv_w[a] : 0.0;
+  std::vector<uint32_t> bin((size_t)nt), starts((size_t)nb + 1, 0), order((size_t)nt);
+  for (long long t = 0; t < nt; ++t) {
+    long long b = 0, mul = 1;
+    for (int a = 0; a < 3; ++a) {
+      const double u = std::floor((boxes[6 * (size_t)t + a] - TB.origin[a]) * TB.inv_w[a]);
+      b += mul * (long long)std::max(0.0, std::min(u, TB.dims[a] - 1.0));
+      mul *= TB.dims[a];
+    }
+    bin[t] = (uint32_t)b;
+    ++starts[b + 1];
+  }
+  for (long long b = 0; b < nb; ++b) starts[b + 1] += starts[b];
+  std::vector<uint32_t> fill(starts.begin(), starts.end() - 1);
+  for (long long t = 0; t < nt; ++t) order[fill[bin[t]]++] = (uint32_t)t;
+  if ((rc = upload_vec(starts, &TB.starts))) return rc;
+  return upload_vec(order, &TB.tiles);
 }
 
 void prt_free_tiles(TileSet *T) {
-  const void *ptrs[] = {T->rows, T->pos, T->boxes};
+  const void *ptrs[] = {T->rows, T->pos, T->boxes, T->bins.starts, T->bins.tiles};
   for (const void *p : ptrs)
     if (p) cudaFree((void *)p);
   *T = TileSet();
@@ -947,15 +951,15 @@ static void launch_tiles(bool split, const TileSet &T, const uint32_t *run_start
                          const TileSums &O, unsigned long long *counters, const uint32_t *order,
                          cudaStream_t s) {
   if (split)
-    deposit_split_kernel<ALPHA2, COUNT><<<(unsigned)T.tiles, 32 * TILE_WARPS, 0, s>>>(
-        tiles_dev(T), run_starts, G, P, W, O, counters);
+    deposit_blocks_kernel<ALPHA2, COUNT, true><<<(unsigned)T.tiles, 32 * BW, 0, s>>>(
+        tiles_dev(T), run_starts, G, P, W, O, counters, nullptr);
   else
-    deposit_blocks_kernel<ALPHA2, COUNT><<<(unsigned)((T.tiles + BW - 1) / BW), 32 * BW, 0, s>>>(
+    deposit_blocks_kernel<ALPHA2, COUNT, false><<<(unsigned)((T.tiles + BW - 1) / BW), 32 * BW, 0, s>>>(
         tiles_dev(T), run_starts, G, P, W, O, counters, order);
 }
 
 // tiles whose blocks of four give every SM a block: below it a tile takes a
-// block of its own (10,000 particles on 577 tiles: 81 us for the deposition
+// block of its own (10,000 particles on 577 tiles: 77 us for the deposition
 // against 160 with two positions per lane)
 constexpr long long SPLIT_TILES = 4 * 148;
 
@@ -1087,112 +1091,51 @@ int prt_mesh_build_positions(prt_mesh *m, const prt_mesh_desc *d) {
   if ((rc = upload_vec(node_to_pos, &P.node_to_pos))) return rc;
   if ((rc = upload_vec(run_starts, &P.run_starts))) return rc;
   if ((rc = upload_vec(order, &P.run_nodes))) return rc;
-  if ((rc = prt_build_tiles(pos.data(), npos, nullptr, &P.tiles))) return rc;
+  if ((rc = prt_build_tiles(pos.data(), npos, nullptr, true, &P.tiles))) return rc;
 
-  // warp groups: runs of at most 32 positions, cut wherever the Morton cell
-  // of about PRT_GROUP_TARGET positions changes, so that no group straddles
-  // two cells (compact groups, tight spheres)
+  // wide warp groups (mixed_simt): runs of at most 64 positions, cut wherever
+  // the Morton cell of about twice PRT_GROUP_TARGET positions changes, so that
+  // no group straddles two cells (compact groups, tight spheres)
   {
     double vol = 1;
     for (int a = 0; a < 3; ++a) vol *= std::max(m->box_hi[a] - m->box_lo[a], 1e-300);
     const double side = std::cbrt(PRT_GROUP_TARGET * vol / std::max<long long>(1, npos));
     int level = (int)std::lround(std::log2(ext / side));
     level = std::min(std::max(level, 0), 21);
-    const int shift = 3 * (21 - level);
-    // runs of <= maxlen positions cut at Morton cells (key >> cell_shift),
-    // with their bounding spheres
-    auto build_groups = [&](int cell_shift, long long maxlen, std::vector<uint32_t> &gs,
-                            std::vector<double> &sph) {
-      gs.clear();
-      gs.reserve(npos / 16 + 2);
-      uint64_t prev_cell = ~0ull;
-      for (long long u = 0; u < npos; ++u) {
-        const uint64_t cell = key[order[run_starts[u]]] >> cell_shift;
-        if (u == 0 || cell != prev_cell || u - gs.back() >= maxlen) gs.push_back((uint32_t)u);
-        prev_cell = cell;
-      }
-      gs.push_back((uint32_t)npos);
-      const long long ng = (long long)gs.size() - 1;
-      sph.assign(4 * (size_t)std::max<long long>(1, ng), 0.0);
-      for (long long g = 0; g < ng; ++g) {
-        double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-        for (uint32_t p = gs[g]; p < gs[g + 1]; ++p)
-          for (int a = 0; a < 3; ++a) {
-            lo[a] = std::min(lo[a], pos[3 * p + a]);
-            hi[a] = std::max(hi[a], pos[3 * p + a]);
-          }
-        double c[3], r2 = 0;
-        for (int a = 0; a < 3; ++a) c[a] = 0.5 * (lo[a] + hi[a]);
-        for (uint32_t p = gs[g]; p < gs[g + 1]; ++p) {
-          double s = 0;
-          for (int a = 0; a < 3; ++a) s += (pos[3 * p + a] - c[a]) * (pos[3 * p + a] - c[a]);
-          r2 = std::max(r2, s);
+    const int cell_shift = std::min(3 * (21 - level) + PRT_WIDE_CELL_BITS, 63);
+    const long long maxlen = 2 * PRT_WARP_NODES;
+    std::vector<uint32_t> gs;
+    std::vector<double> sph;
+    gs.reserve(npos / 16 + 2);
+    uint64_t prev_cell = ~0ull;
+    for (long long u = 0; u < npos; ++u) {
+      const uint64_t cell = key[order[run_starts[u]]] >> cell_shift;
+      if (u == 0 || cell != prev_cell || u - gs.back() >= maxlen) gs.push_back((uint32_t)u);
+      prev_cell = cell;
+    }
+    gs.push_back((uint32_t)npos);
+    const long long ng = (long long)gs.size() - 1;
+    sph.assign(4 * (size_t)std::max<long long>(1, ng), 0.0);
+    for (long long g = 0; g < ng; ++g) {
+      double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+      for (uint32_t p = gs[g]; p < gs[g + 1]; ++p)
+        for (int a = 0; a < 3; ++a) {
+          lo[a] = std::min(lo[a], pos[3 * p + a]);
+          hi[a] = std::max(hi[a], pos[3 * p + a]);
         }
-        for (int a = 0; a < 3; ++a) sph[4 * g + a] = c[a];
-        sph[4 * g + 3] = std::sqrt(r2) * (1 + 1e-9) + 1e-300;
+      double c[3], r2 = 0;
+      for (int a = 0; a < 3; ++a) c[a] = 0.5 * (lo[a] + hi[a]);
+      for (uint32_t p = gs[g]; p < gs[g + 1]; ++p) {
+        double s = 0;
+        for (int a = 0; a < 3; ++a) s += (pos[3 * p + a] - c[a]) * (pos[3 * p + a] - c[a]);
+        r2 = std::max(r2, s);
       }
-    };
-    std::vector<uint32_t> gstart;
-    std::vector<double> spheres;
-    build_groups(shift, PRT_WARP_NODES, gstart, spheres);
-    const long long groups = (long long)gstart.size() - 1;
-    {
-      std::vector<uint32_t> wstart;
-      std::vector<double> wsph;
-      build_groups(std::min(shift + PRT_WIDE_CELL_BITS, 63), 2 * PRT_WARP_NODES, wstart, wsph);
-      P.wide_groups = (long long)wstart.size() - 1;
-      if ((rc = upload_vec(wstart, &P.wide_starts))) return rc;
-      if ((rc = upload_vec(wsph, &P.wide_spheres))) return rc;
+      for (int a = 0; a < 3; ++a) sph[4 * g + a] = c[a];
+      sph[4 * g + 3] = std::sqrt(r2) * (1 + 1e-9) + 1e-300;
     }
-    P.groups = groups;
-    if ((rc = upload_vec(gstart, &P.group_starts))) return rc;
-    if ((rc = upload_vec(spheres, &P.group_spheres))) return rc;
-
-
-
-    // centre bins: width about the mean group radius
-    auto &CB = P.centre_bins;
-    double rsum = 0, rmax = 0;
-    for (long long g = 0; g < groups; ++g) {
-      rsum += spheres[4 * g + 3];
-      rmax = std::max(rmax, spheres[4 * g + 3]);
-    }
-    const double wbin = std::max(rsum / std::max<long long>(1, groups), 1e-300);
-    long long ncb = 1;
-    for (int a = 0; a < 3; ++a) {
-      const double e = m->box_hi[a] - m->box_lo[a];
-      const int dims = e > 0 ? (int)std::max(1.0, std::min(1024.0, std::floor(e / wbin))) : 1;
-      CB.dims[a] = dims;
-      CB.origin[a] = m->box_lo[a];
-      CB.inv_w[a] = e > 0 ? dims / e : 0.0;
-      ncb *= dims;
-    }
-    CB.max_radius = rmax;
-    std::vector<uint32_t> gbin(std::max<long long>(1, groups));
-    std::vector<uint32_t> cstarts(ncb + 1, 0);
-    for (long long g = 0; g < groups; ++g) {
-      long long b = 0, mul = 1;
-      for (int a = 0; a < 3; ++a) {
-        const double u = std::floor((spheres[4 * g + a] - CB.origin[a]) * CB.inv_w[a]);
-        b += mul * (long long)std::max(0.0, std::min(u, CB.dims[a] - 1.0));
-        mul *= CB.dims[a];
-      }
-      gbin[g] = (uint32_t)b;
-      ++cstarts[b + 1];
-    }
-    for (long long b = 0; b < ncb; ++b) cstarts[b + 1] += cstarts[b];
-    std::vector<uint32_t> fill(cstarts.begin(), cstarts.end() - 1);
-    std::vector<double> csph(4 * (size_t)std::max<long long>(1, groups));
-    std::vector<uint32_t> crange(2 * (size_t)std::max<long long>(1, groups));
-    for (long long g = 0; g < groups; ++g) {
-      const uint32_t k = fill[gbin[g]]++;
-      for (int a = 0; a < 4; ++a) csph[4 * k + a] = spheres[4 * g + a];
-      crange[2 * k] = gstart[g];
-      crange[2 * k + 1] = gstart[g + 1] - gstart[g];
-    }
-    if ((rc = upload_vec(cstarts, &CB.starts))) return rc;
-    if ((rc = upload_vec(csph, &CB.spheres))) return rc;
-    if ((rc = upload_vec(crange, &CB.ranges))) return rc;
+    P.wide_groups = ng;
+    if ((rc = upload_vec(gs, &P.wide_starts))) return rc;
+    if ((rc = upload_vec(sph, &P.wide_spheres))) return rc;
   }
 
   return PRT_OK;
@@ -1293,38 +1236,42 @@ extern "C" int prt_deposit_shape(const prt_mesh *mesh, prt_workspace *ws, int32_
     return rc;
   const bool a2 = shape.alpha == 2;
 
+  const uint32_t *perm = nullptr, *starts = nullptr;
+  {
+    ScopedTimer timer(ws, PRT_TIME_DEPOSIT_STAGE, s);
+    if ((rc = bin_particles(ws, G, n, x, el, &perm, &starts, s))) return rc;
+  }
   const double *scale = nullptr;
   if (mode == PRT_DEPOSIT_NORMALIZED) {
     double *sc = (double *)ws_buffer(ws, PRT_WS_DEP_SCALE, 2 * sizeof(double) * (size_t)n, &rc);
     if (!sc) return rc;
-    double *aux = (double *)ws_buffer(
-        ws, PRT_WS_DEP_STATS,
-        sizeof(double) * (64 + mesh->dev.Np + PS.count + 10 * STATS_BLOCKS), &rc);
+    // statistics, integration weights, block partials; then the records
+    const size_t head = ((64 + mesh->dev.Np + 10 * STATS_BLOCKS) + 1) / 2 * 2;
+    double *aux = (double *)ws_buffer(ws, PRT_WS_DEP_STATS,
+                                      sizeof(double) * (head + 4 * (size_t)PS.count), &rc);
     if (!aux) return rc;
-    double *iwd = aux + 16, *W = aux + 64 + mesh->dev.Np;
+    double *iwd = aux + 16, *partials = aux + 64 + mesh->dev.Np;
+    double2 *records = (double2 *)(aux + head);
     PRT_CHECK_CUDA(cudaMemcpyAsync(iwd, iw, sizeof(double) * mesh->dev.Np,
                                    cudaMemcpyHostToDevice, s));
-    position_weights_kernel<<<prt_grid_blocks(PS.count, 256), 256, 0, s>>>(
-        PS.count, PS.run_starts, PS.run_nodes, mesh->dev.Np, iwd, mesh->dev.jacobians, W);
+    const TilesDev T = tiles_dev(PS.tiles);
+    weight_records_kernel<<<prt_grid_blocks(PS.count, 256), 256, 0, s>>>(
+        T, PS.run_starts, PS.run_nodes, mesh->dev.Np, iwd, mesh->dev.jacobians, records);
     PRT_CHECK_CUDA(cudaGetLastError());
-    const CentreBinsDev CB = centre_bins_dev(PS);
-    const unsigned nblk = (unsigned)((n + 32 * NORM_WARPS - 1) / (32 * NORM_WARPS));
     {
       ScopedTimer norm_timer(ws, PRT_TIME_DEPOSIT_NORMALIZE, s);
-      if (a2)
-        normalize_kernel<true><<<nblk, 32 * NORM_WARPS, 0, s>>>(
-            mesh->dev, CB, PS.pos, PS.count, W, S, shape.normalizer, n, x, q, el, sc, sc + n,
-            ws->status);
-      else
-        normalize_kernel<false><<<nblk, 32 * NORM_WARPS, 0, s>>>(
-            mesh->dev, CB, PS.pos, PS.count, W, S, shape.normalizer, n, x, q, el, sc, sc + n,
-            ws->status);
+      const bool share = n < SHARE_PARTICLES;
+      const unsigned nblk = (unsigned)((n + (share ? 32 : CHUNK_N) - 1) / (share ? 32 : CHUNK_N));
+      auto kern = a2 ? (share ? normalize_kernel<true, true> : normalize_kernel<true, false>)
+                     : (share ? normalize_kernel<false, true> : normalize_kernel<false, false>);
+      kern<<<nblk, 32 * BW, 0, s>>>(mesh->dev, T, tile_bins_dev(PS.tiles), records,
+                                    ShapeWeight{S.radius, S.inv_radius, S.alpha},
+                                    shape.normalizer, n, perm, x, q, el, sc, sc + n, ws->status);
       PRT_CHECK_CUDA(cudaGetLastError());
     }
     if (stats) {
       const long long need = (n + 255) / 256;
       const int sb = (int)(need < STATS_BLOCKS ? need : STATS_BLOCKS);
-      double *partials = W + PS.count;
       stats_kernel<<<sb, 256, 0, s>>>(n, sc, sc + n, partials);
       PRT_CHECK_CUDA(cudaGetLastError());
       stats_final_kernel<<<1, 320, 0, s>>>(sb, partials, aux);
@@ -1349,7 +1296,7 @@ extern "C" int prt_deposit_shape(const prt_mesh *mesh, prt_workspace *ws, int32_
   DepParticles P;
   {
     ScopedTimer timer(ws, PRT_TIME_DEPOSIT_STAGE, s);
-    if ((rc = stage_particles(ws, G, n, x, q, v, el, scale, shape.normalizer, nullptr, P, s)))
+    if ((rc = pack_particles(ws, n, perm, starts, x, q, v, scale, shape.normalizer, nullptr, P, s)))
       return rc;
   }
   unsigned long long *counter = nullptr;
@@ -1362,19 +1309,13 @@ extern "C" int prt_deposit_shape(const prt_mesh *mesh, prt_workspace *ws, int32_
   if (!vals) return rc;
   {
     ScopedTimer timer(ws, PRT_TIME_DEPOSIT_GATHER, s);
-    auto groups_for = [&](int ppl, long long &ng, const uint32_t *&gs, const double *&gsp) {
-      ng = ppl == 2 ? PS.wide_groups : PS.groups;
-      gs = ppl == 2 ? PS.wide_starts : PS.group_starts;
-      gsp = ppl == 2 ? PS.wide_spheres : PS.group_spheres;
-      return (unsigned)((ng + WARPS - 1) / WARPS);
-    };
-    long long ng;
-    const uint32_t *gs;
-    const double *gsp;
     const uint32_t *order = nullptr;
     if (precision != PRT_PRECISION_FP64) {
       constexpr int W = PRT_MIXED_PPL;
-      const unsigned nb = groups_for(W, ng, gs, gsp);
+      const long long ng = PS.wide_groups;
+      const uint32_t *gs = PS.wide_starts;
+      const double *gsp = PS.wide_spheres;
+      const unsigned nb = (unsigned)((ng + WARPS - 1) / WARPS);
       if ((rc = heavy_first(ws, ng, gsp, false, G, P, S.radius, &order, s))) return rc;
       if (a2)
         deposit_groups_mixed_kernel<true, W><<<nb, BLOCK, 0, s>>>(PS.pos, ng, gs, gsp, G, P, S,

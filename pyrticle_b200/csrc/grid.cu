@@ -453,7 +453,7 @@ static int grid_tiles(const prt_grid *g) {
         }
   }
   TileSet T;
-  const int rc = prt_build_tiles(P.data(), (long long)ids.size(), ids.data(), &T);
+  const int rc = prt_build_tiles(P.data(), (long long)ids.size(), ids.data(), false, &T);
   if (rc) {
     prt_free_tiles(&T);
     return rc;

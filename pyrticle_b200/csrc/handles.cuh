@@ -39,10 +39,19 @@ struct TileSet {
   const uint32_t *rows = nullptr;  // [count] the target of each row
   const double *pos = nullptr;     // [count][3], row order
   const double *boxes = nullptr;   // [tiles][6]: centre, half extents
+  // the tiles by the uniform bin of their centre (bins about a tile wide),
+  // where asked for: the searches for the tiles near some particles
+  struct {
+    double origin[3], inv_w[3], max_half[3];
+    int dims[3];
+    const uint32_t *starts = nullptr;  // [nbins + 1]
+    const uint32_t *tiles = nullptr;   // [tiles], bin order
+  } bins;
 };
 // Cuts the host points [count][3] into tiles and uploads them; point i is
 // target ids[i] (NULL: i). Freed with prt_free_tiles.
-int prt_build_tiles(const double *points, long long count, const uint32_t *ids, TileSet *out);
+int prt_build_tiles(const double *points, long long count, const uint32_t *ids, bool bins,
+                    TileSet *out);
 void prt_free_tiles(TileSet *tiles);
 
 // Distinct node positions (coincident DG nodes merged), in Morton order:
@@ -53,30 +62,14 @@ struct PositionSet {
   const uint32_t *node_to_pos = nullptr;  // [Nn]
   const uint32_t *run_starts = nullptr;   // [count + 1] into run_nodes
   const uint32_t *run_nodes = nullptr;    // [Nn] node ids grouped by position, ascending
-  // warp groups: runs of <= 32 consecutive positions that never straddle a
-  // Morton cell of about 24 positions, with their bounding spheres
-  long long groups = 0;
-  const uint32_t *group_starts = nullptr; // [groups + 1]
-  const double *group_spheres = nullptr;  // [groups][4]: centre xyz, radius
-  // the FP64 deposition's tiles
+  // the FP64 sums' tiles, with bins
   TileSet tiles;
-  // wide warp groups for the deposition (two positions per lane): runs of
+  // wide warp groups for the mixed_simt deposition (two positions per lane): runs of
   // <= 64 positions that never straddle a Morton cell of about twice the
   // group target
   long long wide_groups = 0;
   const uint32_t *wide_starts = nullptr;  // [wide_groups + 1]
   const double *wide_spheres = nullptr;   // [wide_groups][4]
-  // the groups binned by the bin of their sphere centre (each group in
-  // exactly one bin; uniform bins of about a group radius), in bin order:
-  // spheres and position ranges, with CSR bin starts
-  struct {
-    double origin[3], inv_w[3];
-    int dims[3];
-    double max_radius = 0;
-    const uint32_t *starts = nullptr;   // [nbins + 1]
-    const double *spheres = nullptr;    // [groups][4], bin order
-    const uint32_t *ranges = nullptr;   // [groups][2]: first position, count
-  } centre_bins;
 };
 
 struct prt_mesh {
@@ -146,7 +139,7 @@ int launch_stage_mixed(const prt_pusher *P, prt_workspace *ws, long long n, doub
                        cudaStream_t s);
 
 constexpr int PRT_WARP_NODES = 32;
-// target positions per Morton cell when cutting warp groups
+// target positions per Morton cell before the wide groups' factor
 constexpr double PRT_GROUP_TARGET = 24.0;
 // Morton bits dropped from the group cells for the wide groups (1: cells of
 // two sibling cells, about twice the positions)

@@ -100,174 +100,8 @@ __device__ __forceinline__ void reduce_groups(double (&v)[N][PER]) {
   }
 }
 
-// Candidate segments of one warp: runs of consecutive particles in bin order.
-// At most SEGS per turn of 32 bin rows: a row falls into at most four pieces
-// along a periodic x (a tile no wider than the period, a radius below half).
-struct Segments {
-  static constexpr int PIECES = 4, SEGS = 32 * PIECES;
-  uint32_t cum[SEGS + 1];  // candidates before the segment
-  uint32_t start[SEGS];    // its first bin-order particle
-  double shift[SEGS][3];   // from a particle's position to the tile's frame
-};
-
-// Walks the particles of the bin rows within `radius` of the box c +- hf, 32
-// at a time: visit(valid, k, w0, w1, w2, q) on all lanes, with w relative to c
-// (periodic image included). Warps part of `parts` takes every parts-th batch.
-// The rows are laid out 32 at a time, one per lane, and their particles
-// numbered through, so that short rows fill the lanes together; the next
-// batch's particles are loaded before the present one is visited (`q` is the
-// payload's charge).
-template <class Visit>
-__device__ __forceinline__ void stream_particles(const BinGrid &G, const DepParticles &P,
-                                                 const double c[3], const double hf[3],
-                                                 double radius, Segments &S, int part,
-                                                 int parts, Visit &&visit) {
-  const int lane = threadIdx.x & 31;
-  const double rr = radius * (1 + 1e-5), rr2 = rr * rr;
-  int ulo[3], uhi[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    ulo[d] = bin_floor(G, d, c[d] - hf[d] - rr);
-    uhi[d] = bin_floor(G, d, c[d] + hf[d] + rr);
-    if (G.periodic[d]) {
-      ulo[d] -= 1;
-      uhi[d] += 1;
-    } else {
-      ulo[d] = max(ulo[d], 0);
-      uhi[d] = min(uhi[d], G.dims[d] - 1);
-    }
-  }
-  const double2 *__restrict__ pay = reinterpret_cast<const double2 *>(P.payload);
-  auto slab_gap = [&](int d, double blo) {
-    const double e =
-        fmax(0.0, fmax(blo - (c[d] + hf[d]), (c[d] - hf[d]) - (blo + G.w[d]))) - G.slack[d];
-    return e > 0 ? e * e : 0.0;
-  };
-  const int ny = max(0, uhi[1] - ulo[1] + 1), nz = max(0, uhi[2] - ulo[2] + 1);
-  const long long nrows = (long long)ny * nz;
-  for (long long r0 = 0; r0 < nrows; r0 += 32) {
-    const long long r = r0 + lane;
-    uint32_t s_start[Segments::PIECES], s_len[Segments::PIECES];
-    int s_q[Segments::PIECES];
-    int cnt = 0;
-    uint32_t mine = 0;
-    int qz = 0, qy = 0;
-    if (r < nrows) {
-      const int bz = ulo[2] + (int)(r / ny), by = ulo[1] + (int)(r % ny);
-      int wz = bz, wy = by;
-      if (G.periodic[2]) {
-        qz = floor_div(bz, G.dims[2]);
-        wz = bz - qz * G.dims[2];
-      }
-      if (G.periodic[1]) {
-        qy = floor_div(by, G.dims[1]);
-        wy = by - qy * G.dims[1];
-      }
-      const double dyz2 =
-          slab_gap(2, G.origin[2] + bz * G.w[2]) + slab_gap(1, G.origin[1] + by * G.w[1]);
-      if (dyz2 <= rr2) {
-        const double rem = sqrt(rr2 - dyz2);
-        int bx0 = bin_floor(G, 0, c[0] - hf[0] - rem);
-        int bx1 = bin_floor(G, 0, c[0] + hf[0] + rem);
-        if (G.periodic[0]) {
-          bx0 -= 1;
-          bx1 += 1;
-        }
-        bx0 = max(bx0, ulo[0]);
-        bx1 = min(bx1, uhi[0]);
-        const long long row = (long long)G.dims[0] * (wy + (long long)G.dims[1] * wz);
-        int bx = bx0;
-#pragma unroll
-        for (int i = 0; i < Segments::PIECES; ++i) {
-          if (bx <= bx1) {
-            int wx = bx, q = 0, end = bx1;
-            if (G.periodic[0]) {
-              q = floor_div(bx, G.dims[0]);
-              wx = bx - q * G.dims[0];
-              end = min(bx1, (q + 1) * G.dims[0] - 1);
-            }
-            s_start[i] = P.starts[row + wx];
-            s_len[i] = P.starts[row + wx + (end - bx) + 1] - s_start[i];
-            s_q[i] = q;
-            mine += s_len[i];
-            cnt = i + 1;
-            bx = end + 1;
-          }
-        }
-      }
-    }
-    // place the segments: exclusive scans of their number and candidates
-    int ns = cnt;
-    uint32_t nc = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int a = __shfl_up_sync(0xffffffffu, ns, o);
-      const uint32_t b = __shfl_up_sync(0xffffffffu, nc, o);
-      if (lane >= o) {
-        ns += a;
-        nc += b;
-      }
-    }
-    const int segs = __shfl_sync(0xffffffffu, ns, 31);
-    const uint32_t total = __shfl_sync(0xffffffffu, nc, 31);
-    if (total == 0) continue;
-    __syncwarp();
-    {
-      int at = ns - cnt;
-      uint32_t before = nc - mine;
-#pragma unroll
-      for (int i = 0; i < Segments::PIECES; ++i)
-        if (i < cnt) {
-          S.cum[at] = before;
-          S.start[at] = s_start[i];
-          S.shift[at][0] = s_q[i] * G.period[0] - c[0];
-          S.shift[at][1] = qy * G.period[1] - c[1];
-          S.shift[at][2] = qz * G.period[2] - c[2];
-          before += s_len[i];
-          ++at;
-        }
-      if (lane == 31) S.cum[segs] = total;
-    }
-    __syncwarp();
-    int sg = 0;
-    uint32_t k = 0;
-    double2 xy = make_double2(0, 0), zq = make_double2(0, 0);
-    int seg = 0;
-    auto load = [&](uint32_t f) {
-      if (f < total) {
-        while (f >= S.cum[sg + 1]) ++sg;
-        seg = sg;
-        k = S.start[sg] + (f - S.cum[sg]);
-        xy = pay[4 * (size_t)k];
-        zq = pay[4 * (size_t)k + 1];
-      }
-    };
-    uint32_t b = 32u * part;
-    load(b + lane);
-    for (; b < total; b += 32u * parts) {
-      const bool valid = b + lane < total;
-      const uint32_t k0 = k;
-      const double w0 = xy.x + S.shift[seg][0], w1 = xy.y + S.shift[seg][1],
-                   w2 = zq.x + S.shift[seg][2], q = zq.y;
-      load(b + 32u * parts + lane);
-      visit(valid, k0, w0, w1, w2, q);
-    }
-    __syncwarp();
-  }
-}
-
-// Whether a source at w (relative to the centre of a box with half extents hf,
-// grown by 1e-5 radii) may lie within the radius of the box; rc4 = 4 radius^2,
-// grown likewise. Per axis 2 max(|w| - hf, 0) = d + |d|. It only chooses what
-// is evaluated: FP32 on the FP64 offsets, with the margin above its rounding.
-__device__ __forceinline__ bool near_box(double w0, double w1, double w2, const float hf[3],
-                                         float rc4) {
-  const float d0 = fabsf((float)w0) - hf[0], d1 = fabsf((float)w1) - hf[1],
-              d2 = fabsf((float)w2) - hf[2];
-  const float e0 = d0 + fabsf(d0), e1 = d1 + fabsf(d1), e2 = d2 + fabsf(d2);
-  return e0 * e0 + e1 * e1 + e2 * e2 <= rc4;
-}
-
+// 4 radius^2 for the choice of entries near a box, with a margin above FP32
+// rounding (the choice only decides what is evaluated).
 __device__ __forceinline__ float near_limit(double radius) {
   const float r = (float)(radius * (1 + 1e-5));
   return 4.0f * r * r;
@@ -337,10 +171,11 @@ __device__ __forceinline__ void stage_begin(BlockStage<NV> &S) {
 // Evaluates the `total` sources of the present segments (S.cum, S.start,
 // S.shift; written before a barrier) against the block's tiles:
 // op(w0, w1, w2, e, v) on every lane with its group's entry. mid, hf: this
-// warp's tile box in the block's frame, grown as near_box wants it; a warp
+// warp's tile box in the block's frame, grown by the FP32 margin; a warp
 // without a tile passes hf < 0 with a magnitude that keeps everything out.
+// SHARE: the warps have the same tile and take 32 of a chunk's entries each.
 // Returns the entries evaluated (per warp). Ends with a barrier.
-template <int PER, int NV, class Op>
+template <int PER, int NV, bool SHARE, class Op>
 __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV> &S,
                                                       const double2 *__restrict__ records,
                                                       uint32_t total, const float mid[3],
@@ -411,6 +246,7 @@ __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV> &S,
     int n = 0;
 #pragma unroll
     for (int q = 0; q < BW; ++q) {
+      if (SHARE && q != wid) continue;
       const float4 w = S.w[st][32 * q + lane];
       const float d0 = fabsf(w.x - mid[0]) - hf[0], d1 = fabsf(w.y - mid[1]) - hf[1],
                   d2 = fabsf(w.z - mid[2]) - hf[2];
@@ -455,7 +291,7 @@ struct BlockBox {
 
 // All particles of the bin rows near the block's box, evaluated against its
 // tiles (evaluate_segments).
-template <int PER, int NV, class Op>
+template <int PER, int NV, bool SHARE, class Op>
 __device__ __forceinline__ uint32_t evaluate_particles(BlockStage<NV> &S, const BinGrid &G,
                                                        const DepParticles &P, const BlockBox &X,
                                                        double radius, double inv_radius,
@@ -542,10 +378,230 @@ __device__ __forceinline__ uint32_t evaluate_particles(BlockStage<NV> &S, const 
     for (int d = 0; d < 3; ++d) S.shift[tid][d] = sh[d];
     if (tid == 0) S.cum[CHUNK_N] = total;
     __syncthreads();
-    evaluated += evaluate_segments<PER, NV>(S, reinterpret_cast<const double2 *>(P.payload), total,
-                                            X.mid, X.hf, rc4, inv_radius, op);
+    evaluated += evaluate_segments<PER, NV, SHARE>(
+        S, reinterpret_cast<const double2 *>(P.payload), total, X.mid, X.hf, rc4, inv_radius, op);
   }
   return evaluated;
 }
+
+// ------------------------------------------- particles as the targets
+
+struct TileBinsDev {
+  double origin[3], inv_w[3], max_half[3];
+  int dims[3];
+  const uint32_t *__restrict__ starts, *__restrict__ tiles;
+};
+
+inline TileBinsDev tile_bins_dev(const TileSet &T) {
+  TileBinsDev B;
+  for (int d = 0; d < 3; ++d) {
+    B.origin[d] = T.bins.origin[d];
+    B.inv_w[d] = T.bins.inv_w[d];
+    B.max_half[d] = T.bins.max_half[d];
+    B.dims[d] = T.bins.dims[d];
+  }
+  B.starts = T.bins.starts;
+  B.tiles = T.bins.tiles;
+  return B;
+}
+
+// The rows of tile bins of one turn of the search.
+struct TileRows {
+  uint32_t cum[CHUNK_N + 1], first[CHUNK_N];
+};
+
+// All positions of the tiles near the block's box (periodic images included),
+// evaluated against its targets: `records` in the tiles' row order.
+template <int PER, int NV, bool SHARE, class Op>
+__device__ __forceinline__ void evaluate_positions(BlockStage<NV> &S, TileRows &Q,
+                                                   const TilesDev &T, const TileBinsDev &B,
+                                                   const double2 *__restrict__ records,
+                                                   const DevMesh &M, const BlockBox &X,
+                                                   double radius, double inv_radius, Op &&op) {
+  const int tid = threadIdx.x;
+  const double rr = radius * (1 + 1e-5), rr2 = rr * rr;
+  const float rc4 = near_limit(radius);
+  int lo_img[3], hi_img[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    lo_img[d] = hi_img[d] = 0;
+    if (M.pmin[d] != M.pmax[d]) {
+      if (X.c[d] - X.h[d] - rr < M.pmin[d]) hi_img[d] = 1;
+      if (X.c[d] + X.h[d] + rr > M.pmax[d]) lo_img[d] = -1;
+    }
+  }
+  for (int iz = lo_img[2]; iz <= hi_img[2]; ++iz)
+    for (int iy = lo_img[1]; iy <= hi_img[1]; ++iy)
+      for (int ix = lo_img[0]; ix <= hi_img[0]; ++ix) {
+        // the box moved by whole periods
+        const double c[3] = {X.c[0] + ix * (M.pmax[0] - M.pmin[0]),
+                             X.c[1] + iy * (M.pmax[1] - M.pmin[1]),
+                             X.c[2] + iz * (M.pmax[2] - M.pmin[2])};
+        int b0[3], b1[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const double reach = X.h[d] + rr + B.max_half[d];
+          const double l = floor((c[d] - reach - B.origin[d]) * B.inv_w[d]);
+          const double h = floor((c[d] + reach - B.origin[d]) * B.inv_w[d]);
+          b0[d] = (int)fmax(0.0, fmin(l, B.dims[d] - 1.0));
+          b1[d] = (int)fmax(0.0, fmin(h, B.dims[d] - 1.0));
+        }
+        const int ny = b1[1] - b0[1] + 1;
+        const int nrows = ny * (b1[2] - b0[2] + 1);
+        for (int r0 = 0; r0 < nrows; r0 += CHUNK_N) {
+          const int r = r0 + tid;
+          uint32_t first = 0, len = 0;
+          if (r < nrows) {
+            const long long row =
+                (long long)B.dims[0] * (b0[1] + r % ny + (long long)B.dims[1] * (b0[2] + r / ny));
+            first = B.starts[row + b0[0]];
+            len = B.starts[row + b1[0] + 1] - first;
+          }
+          uint32_t tiles;
+          const uint32_t before = block_scan(S, len, tiles);
+          if (tiles == 0) continue;
+          Q.cum[tid] = before;
+          Q.first[tid] = first;
+          if (tid == 0) Q.cum[CHUNK_N] = tiles;
+          __syncthreads();
+          for (uint32_t t0 = 0; t0 < tiles; t0 += CHUNK_N) {
+            const uint32_t j = t0 + tid;
+            uint32_t tile = 0, n = 0;
+            if (j < tiles) {
+              int at = 0;
+#pragma unroll
+              for (int step = CHUNK_N / 2; step > 0; step >>= 1)
+                if (Q.cum[at + step] <= j) at += step;
+              tile = B.tiles[Q.first[at] + (j - Q.cum[at])];
+              double d2 = 0;
+#pragma unroll
+              for (int d = 0; d < 3; ++d) {
+                const double e = fmax(0.0, fabs(T.boxes[6 * (size_t)tile + d] - c[d]) -
+                                               T.boxes[6 * (size_t)tile + 3 + d] - X.h[d]);
+                d2 = fma(e, e, d2);
+              }
+              if (d2 <= rr2) n = (uint32_t)min((long long)TILE, T.count - (long long)TILE * tile);
+            }
+            uint32_t total;
+            const uint32_t at = block_scan(S, n, total);
+            if (total == 0) continue;
+            S.cum[tid] = at;
+            S.start[tid] = TILE * tile;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) S.shift[tid][d] = -c[d];
+            if (tid == 0) S.cum[CHUNK_N] = total;
+            __syncthreads();
+            evaluate_segments<PER, NV, SHARE>(S, records, total, X.mid, X.hf, rc4, inv_radius, op);
+          }
+          __syncthreads();
+        }
+      }
+}
+
+// The particles of a warp's lanes as targets: lane (tg, .) holds PER of the 32
+// from k0 (bin order with `perm`, else store order), and the block's and the
+// warp's boxes around the live ones. SHARE: all warps have the same 32.
+// Returns whether the block has a live particle at all.
+template <int PER>
+struct ParticleTargets {
+  long long id[PER];  // store index, -1 for none
+  bool live[PER];
+  double V[3][PER], B[PER];
+};
+
+template <int PER, bool SHARE>
+__device__ __forceinline__ bool load_particles(ParticleTargets<PER> &D, BlockBox &X,
+                                               double (*boxes)[6], long long n,
+                                               const uint32_t *__restrict__ perm,
+                                               const double *__restrict__ x,
+                                               const uint32_t *__restrict__ el,
+                                               const ShapeWeight &S) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int tg = lane % (32 / PER);
+  const long long k0 = 32 * (SHARE ? (long long)blockIdx.x : BW * (long long)blockIdx.x + wid);
+  double p[3][PER], lo[3] = {INFINITY, INFINITY, INFINITY},
+                    hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int h = 0; h < PER; ++h) {
+    const long long k = k0 + PER * tg + h;
+    D.id[h] = k < n ? (perm ? (long long)perm[k] : k) : -1;
+    D.live[h] = D.id[h] >= 0 && !(el && el[D.id[h]] == PRT_INVALID);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      p[d][h] = D.live[h] ? x[d * n + D.id[h]] : 0;
+      if (D.live[h]) {
+        lo[d] = fmin(lo[d], p[d][h]);
+        hi[d] = fmax(hi[d], p[d][h]);
+      }
+    }
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+#pragma unroll
+    for (int o = 16 / PER; o > 0; o >>= 1) {
+      lo[d] = fmin(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
+      hi[d] = fmax(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+    }
+  if (lane == 0) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      boxes[wid][d] = lo[d];
+      boxes[wid][3 + d] = hi[d];
+    }
+  }
+  __syncthreads();
+  bool any = false;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    double bl = INFINITY, bh = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < BW; ++w) {
+      bl = fmin(bl, boxes[w][d]);
+      bh = fmax(bh, boxes[w][3 + d]);
+    }
+    any = bl <= bh;
+    X.c[d] = any ? 0.5 * (bl + bh) : 0;
+    X.h[d] = any ? 0.5 * (bh - bl) + 1e-5 * S.radius : 0;
+    const bool have = lo[d] <= hi[d];
+    X.mid[d] = have ? (float)(0.5 * (lo[d] + hi[d]) - X.c[d]) : 0;
+    X.hf[d] = have ? (float)(0.5 * (hi[d] - lo[d]) + 1e-5 * S.radius) : -1e30f;
+  }
+#pragma unroll
+  for (int h = 0; h < PER; ++h) {
+    double u2 = 0;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double u = p[d][h] - X.c[d];
+      u2 = fma(u, u, u2);
+      D.V[d][h] = 2 * u * S.inv_radius;
+    }
+    // absent and removed particles: never within the radius
+    D.B[h] = D.live[h] ? S.radius - u2 * S.inv_radius : -1e300;
+    if (!D.live[h]) D.V[0][h] = D.V[1][h] = D.V[2][h] = 0;
+  }
+  return any;
+}
+
+// Adds up the sums of the warps that shared a tile (after evaluate_...):
+// v[k][0] of every lane; the first warp's lanes get the totals.
+template <int N, int PER, class Stage>
+__device__ __forceinline__ void share_sums(Stage &S, double (&v)[N][PER]) {
+  double *part = reinterpret_cast<double *>(&S.e[0][0][0]);
+  const int tid = threadIdx.x;
+  static_assert(sizeof(S.e) >= N * CHUNK_N * sizeof(double), "partial sums fit the staging");
+#pragma unroll
+  for (int k = 0; k < N; ++k) part[k * CHUNK_N + tid] = v[k][0];
+  __syncthreads();
+  if (tid < 32) {
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+#pragma unroll
+      for (int w = 1; w < BW; ++w) v[k][0] += part[k * CHUNK_N + 32 * w + tid];
+  }
+}
+
+// particles below which a block takes 32 (its warps share them) instead of 128:
+// with 128 the blocks would leave SMs empty
+constexpr long long SHARE_PARTICLES = 148 * CHUNK_N;
 
 }  // namespace prt_dep

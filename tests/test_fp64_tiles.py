@@ -113,3 +113,81 @@ def test_normalized(cubes, order, n, periodic, radius):
     assert stats.node_pair_count == float(within.sum())
     # per particle the positions within the radius: the same pairs in both passes
     assert stats.pair_count == stats.el_sum <= stats.node_pair_count <= within.shape[0] * n
+
+
+@pytest.mark.parametrize("n", [1, 130, 19001])
+@pytest.mark.parametrize("periodic,radius,alpha", [(False, 0.004, 2), (True, 0.003, 2),
+                                                   (False, 0.004, 3)])
+@pytest.mark.parametrize("ordered", [False, True])
+def test_average_forces(n, periodic, radius, alpha, ordered):
+    m, s = setup(ShapeFunctionDepositor(), (5, 5, 5), 2, n, periodic, radius, alpha)
+    s.el[::9] = -1  # removed particles: forces stay as they were
+    if ordered:
+        m.sort_by_element(s)
+    S, _ = shape(m, s, radius, alpha, periodic)
+    mesh = m.discretization.mesh
+    iw = np.ascontiguousarray(
+        m.discretization.element_groups[0].local_discretization.mass_matrix().sum(axis=1))
+    w = torch.as_tensor(np.outer(mesh.jacobians, iw).ravel(), device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(n)
+    F = torch.randn((6, len(w)), generator=g, dtype=F64, device="cuda")
+    v = m.velocities_device(s)
+    out = torch.full((3, n), 7.0, dtype=F64, device="cuda")
+    vis = torch.full((14, n), 7.0, dtype=F64, device="cuda")
+    ptrs = (C.c_void_p * 6)(*[F[k].data_ptr() for k in range(6)])
+    live = s.el != -1
+    den = (w @ S)[live]
+    avg = torch.stack([(w * F[k]) @ S for k in range(6)])[:, live] / den
+    want = s.q[live] * (avg[:3] + torch.linalg.cross(v[:, live].T, avg[3:].T).T)
+    for k in range(2):
+        _lib.check(m.lib.prt_average_forces_ordered(
+            m.mesh_data.handle, m.workspace, m.depositor._shape_desc(), _lib.ptr(iw), n,
+            s.x.data_ptr(), s.q.data_ptr(), v.data_ptr(), s.el.data_ptr(), ptrs, out.data_ptr(),
+            vis.data_ptr() if k else None, None, int(ordered), C.c_void_p(0)))
+        if int(live.sum()):
+            # (order 2 has negative weights: the denominators cancel up to ~100x)
+            assert rel(out[:, live], want) <= 100 * TOL
+        assert bool((out[:, ~live] == 7.0).all())
+    if int(live.sum()):
+        assert rel(vis[:6, live], avg) <= 100 * TOL
+        sq = torch.stack([(w * (F[3 * k:3 * k + 3] ** 2).sum(0)) @ S for k in range(2)])[:, live]
+        var = sq / den - torch.stack([(avg[:3] ** 2).sum(0), (avg[3:] ** 2).sum(0)])
+        big = var > 1e-3 * sq.abs() / den.abs()
+        assert torch.allclose(vis[6:8, live][big] ** 2, var[big], rtol=1e-8, atol=0)
+
+
+@pytest.mark.parametrize("n", [1, 130, 19001])
+@pytest.mark.parametrize("periodic,radius,alpha", [(False, 0.004, 2), (True, 0.003, 2),
+                                                   (False, 0.004, 3)])
+def test_deposit_adjoint(n, periodic, radius, alpha):
+    m, s = setup(ShapeFunctionDepositor(), (5, 5, 5), 2, n, periodic, radius, alpha)
+    nn = len(m.discretization)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    grho = torch.randn(nn, generator=g, dtype=F64, device="cuda")
+    gj = torch.randn((3, nn), generator=g, dtype=F64, device="cuda") / U.VACUUM_LIGHT_SPEED()
+    v = m.velocities_device(s)
+    lx = torch.zeros_like(s.x)
+    lv = torch.zeros_like(s.x)
+    _lib.check(m.lib.prt_deposit_shape_adjoint(
+        m.mesh_data.handle, m.workspace, m.depositor._shape_desc(), n, s.x.data_ptr(),
+        s.q.data_ptr(), v.data_ptr(), s.el.data_ptr(), grho.data_ptr(), gj.data_ptr(),
+        lx.data_ptr(), lv.data_ptr(), C.c_void_p(0)))
+    nodes = torch.as_tensor(np.ascontiguousarray(m.discretization.nodes), device="cuda")
+    norm = m.depositor.shape_function.normalizer
+    h = grho[:, None] + gj.T @ v  # [nodes, particles]
+    wx = torch.zeros_like(lx)
+    r2 = torch.zeros((nn, n), dtype=F64, device="cuda")
+    diffs = []
+    for d, ext in enumerate((0.01, 0.012, 0.014)):
+        diff = nodes[:, d, None] - s.x[d][None]
+        if periodic:
+            diff = diff - ext * torch.round(diff / ext)
+        diffs.append(diff)
+        r2 += diff * diff
+    t = torch.clamp(radius - r2 / radius, min=0)
+    ds = s.q * norm * alpha * t ** (alpha - 1) * (2 / radius) * h
+    for d in range(3):
+        wx[d] = (ds * diffs[d]).sum(0)
+    wv = s.q * norm * torch.stack([gj[d] @ t ** alpha for d in range(3)])
+    assert rel(lx, wx) <= TOL
+    assert rel(lv, wv) <= TOL
