@@ -448,13 +448,15 @@ def adjoint_bench(torch, scale, hbm_gbs, reps=3, checkpoint_every=10):
         adj_ms, adj_n = timing_read(m, _lib.TIME_STAGE_ADJOINT)
         dep_ms, dep_n = timing_read(m, _lib.TIME_DEPOSIT_ADJOINT)
         n = len(w.positions)
-        # per adjoint stage: read x, p (48 B), element (4), q, m (16), four
-        # adjoints (96); write four adjoints (96)
-        adj_gbs = 260.0 * n / (adj_ms / max(adj_n, 1) * 1e-3) / 1e9
+        # per launch (a segment): the stages' x, p (48 B) and element (4), then
+        # q, m (16) and four adjoints read and written (192)
+        stages = 5 * checkpoint_every
+        adj_gbs = (52.0 * stages + 208.0) * n / (adj_ms / max(adj_n, 1) * 1e-3) / 1e9
         out[form] = {"forward_ms": f / reps, "backward_ms": b / reps,
                      "ratio_backward_over_forward": b / f, "loss": L,
                      "grad_p0": gp, "grad_theta": gth,
-                     "stage_adjoint_kernel_ms": adj_ms / max(adj_n, 1),
+                     "steps_adjoint_kernel_ms": adj_ms / max(adj_n, 1),
+                     "stage_adjoint_kernel_ms": adj_ms / max(adj_n, 1) / stages,
                      "stage_adjoint_gbs": adj_gbs, "stage_adjoint_frac_hbm": adj_gbs / hbm_gbs,
                      "deposit_adjoint_ms": dep_ms / max(dep_n, 1),
                      "backward_phases_ms": dict(trajs[form].phase_ms)}

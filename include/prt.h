@@ -223,7 +223,8 @@ int prt_field_coefficients(const prt_pusher *pusher, const double *const fields[
  * and `fields` may be NULL; without, from the nodal `fields` in FP64.
  * A first stage with rk_a[0] = 0 does not read kx and kp; they are written at
  * the end. tape_x, tape_p [stages + 1][3][n] and tape_el [stages + 1][n] (all
- * or none NULL) receive the state after stage t in slot t + 1. */
+ * or none NULL) receive the state after stage t in slot t + 1. Where positions,
+ * momenta and elements are the tape's slot 0 they are left as they are. */
 int prt_lsrk_steps(const prt_pusher *pusher, prt_workspace *ws, int64_t n,
                    double *positions, double *momenta, const double *charges,
                    const double *masses, uint32_t *elements, double *kx,
@@ -511,6 +512,23 @@ int prt_lsrk_stage_adjoint(const prt_pusher *pusher, prt_workspace *ws, int64_t 
                            double *const grad_fields[6],
                            int32_t nbasis, const double *const *basis,
                            double *grad_theta, void *stream);
+
+/* prt_lsrk_stage_adjoint for the stages `stages` - 1 .. 0 of a tape that
+ * prt_lsrk_steps wrote (slot t holds the input of stage t), in one launch;
+ * without nodal field gradients. `coefficients` are the FP64 ones of
+ * prt_field_coefficients; components whose bit (1 << k) in `field_mask` is
+ * clear are taken as zero. The basis fields come as for
+ * prt_lsrk_stage_adjoint. */
+int prt_lsrk_steps_adjoint(const prt_pusher *pusher, prt_workspace *ws, int64_t n,
+                           const double *tape_x, const double *tape_p,
+                           const uint32_t *tape_el, const double *charges,
+                           const double *masses, double *lam_x, double *lam_p,
+                           double *lam_kx, double *lam_kp, const double *coefficients,
+                           uint32_t field_mask, const double *rk_a, const double *rk_b,
+                           int32_t rk_count, int32_t stages, double dt, double vacuum_c,
+                           int32_t nbasis, const double *const *basis, double *grad_theta,
+                           void *stream);
+
 
 /* Adjoint of prt_get_velocities: lam_p += (dv/dp)^T lam_v. */
 int prt_velocities_adjoint(int64_t n, const double *momenta, const double *masses,

@@ -177,6 +177,9 @@ SIGNATURES = {
     "prt_lsrk_stage_adjoint": (_i32, [_vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                                       _vp, _vp, C.POINTER(_vp), _d, _d, _d, _d,
                                       C.POINTER(_vp), _i32, C.POINTER(_vp), _vp, _vp]),
+    "prt_lsrk_steps_adjoint": (_i32, [_vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
+                                      _vp, _vp, C.c_uint32, _dp, _dp, _i32, _i32, _d, _d, _i32,
+                                      C.POINTER(_vp), _vp, _vp]),
     "prt_velocities_adjoint": (_i32, [_i64, _vp, _vp, _d, _vp, _vp, _vp]),
     "prt_fields_to_monomial": (_i32, [_vp, _i32, C.POINTER(_vp), C.POINTER(_vp), _vp]),
     "prt_deposit_shape_adjoint": (_i32, [_vp, _vp, ShapeFunctionDesc, _i64, _vp, _vp, _vp,

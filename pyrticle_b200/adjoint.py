@@ -11,19 +11,20 @@ Fields: ``F = fields + sum_k theta[k] * basis[k]`` ([6, Nn] each: ex, ey,
 ez, bx, by, bz at the nodes). The forward keeps a checkpoint of the particle
 state (x, p, element, order) every ``checkpoint_every`` steps; the backward
 walks the segments in reverse, recomputes each from its checkpoint while
-recording every stage's input state (``prt_lsrk_stage_record``: bitwise the
-forward's arithmetic), then runs the stage adjoints in reverse
-(``prt_lsrk_stage_adjoint``). The last segment is recorded by the forward
-itself, so the backward starts with its stage adjoints. The deposition adjoint
+recording every stage's input state (one ``prt_lsrk_steps`` launch with a tape:
+bitwise the forward's arithmetic), then runs the stage adjoints in reverse (one
+``prt_lsrk_steps_adjoint`` launch, or with nodal field gradients a
+``prt_lsrk_stage_adjoint`` per stage). The last segment is recorded by the
+forward itself, so the backward starts with its stage adjoints. The deposition adjoint
 (``prt_deposit_shape_adjoint``) and the velocity adjoint start the chain.
 Every derivative is computed by libprt's CUDA kernels; torch tensors are the
 device buffers and the autograd boundary.
 
 Particles are sorted by element at each checkpoint (the element-sorted order
 keeps the field gathers coherent); adjoints are carried across segments by
-the particle order stored with each checkpoint. The launches of a segment
-(recomputation and stage adjoints) are captured once into a CUDA graph and
-replayed for the other segments of the same length.
+the particle order stored with each checkpoint. With nodal field gradients the
+launches of a segment (recomputation and stage adjoints) are captured once into
+a CUDA graph and replayed for the other segments of the same length.
 """
 
 from __future__ import annotations
@@ -33,7 +34,7 @@ import ctypes as C
 import torch
 
 from . import _lib
-from .cloud import LSRK4_A, LSRK4_B, stream_handle
+from .cloud import _RK_A, _RK_B, LSRK4_A, LSRK4_B, stream_handle
 from .deposition.shape import PRECISIONS
 
 F64 = torch.float64
@@ -55,9 +56,15 @@ def _arg_key(a):
     return a
 
 
+def _nonzero(f):
+    """Per component of [..., 6, Nn] fields, whether it is not identically
+    zero (one device pass and one host read for all of them)."""
+    return (f != 0).any(dim=-1).tolist()
+
+
 def _field_components(f):
     """Six component tensors of a [6, Nn] field, None where identically zero."""
-    return [f[k] if bool(torch.any(f[k] != 0)) else None for k in range(6)]
+    return [f[k] if use else None for k, use in enumerate(_nonzero(f))]
 
 
 def monomial_coefficients(method, comps):
@@ -101,11 +108,11 @@ class DifferentiableTrajectory:
         self.precision = PRECISIONS[precision]
         self.c = method.units.VACUUM_LIGHT_SPEED()
         self.nn = len(method.discretization)
-        # replay each segment's recomputation and adjoint launches from a
-        # CUDA graph captured on the first full segment; the graphs are kept
-        # across backward calls, keyed by every launch argument they hold
-        # (the caching allocator hands a repeated call the same buffers, so
-        # the capture happens once)
+        # with nodal field gradients (a launch per stage adjoint): replay each
+        # segment's launches from a CUDA graph captured on the first full
+        # segment; the graphs are kept across backward calls, keyed by every
+        # launch argument they hold (the caching allocator hands a repeated
+        # call the same buffers, so the capture happens once)
         self.use_graphs = True
         self._graphs = {}
         # when True, backward_run records CUDA events between its phases
@@ -130,12 +137,21 @@ class DifferentiableTrajectory:
             F += torch.einsum("k,kcn->cn", theta.detach().to(F.device), self.basis)
         return F.contiguous()
 
-    def _stage(self, F, x, p, q, m, el, kx, kp, a, b):
-        _lib.check(self.lib.prt_lsrk_stage(
-            self.method.pusher.handle, self.method.workspace, x.shape[1], x.data_ptr(),
-            p.data_ptr(), q.data_ptr(), m.data_ptr(), el.data_ptr(), kx.data_ptr(),
-            kp.data_ptr(), F, a, b, self.dt, self.c, 0, C.c_void_p(stream_handle())),
-            "prt_lsrk_stage")
+    def _coefficients(self, Fp, n):
+        """The fields as per-element monomial coefficients for the trajectory's
+        steps, or None where the nodal form is the cheaper one."""
+        if n and self.method._use_coefficients(n, self.steps):
+            return self.method.pusher.field_coefficients(Fp)
+        return None
+
+    def _steps_args(self, Fp, coef, x, p, q, m, el, kx, kp, stages, tape=None):
+        """Arguments of prt_lsrk_steps (without the stream); ``tape``: the
+        (tx, tp, te) whose slot 0 the store is."""
+        return (self.method.pusher.handle, self.method.workspace, x.shape[-1], x.data_ptr(),
+                p.data_ptr(), q.data_ptr(), m.data_ptr(), el.data_ptr(), kx.data_ptr(),
+                kp.data_ptr(), None if coef is None else coef.data_ptr(), Fp, 0, _RK_A, _RK_B, 5,
+                stages, self.dt, self.c,
+                *((None,) * 3 if tape is None else [t.data_ptr() for t in tape]))
 
     def _sort(self, el, x, p, q, m, kx, kp, order):
         _lib.check(self.lib.prt_sort_by_element(
@@ -164,41 +180,35 @@ class DifferentiableTrajectory:
         order = torch.arange(n, dtype=torch.int64, device=dev)
         kx = torch.zeros_like(x)
         kp = torch.zeros_like(p)
+        coef = self._coefficients(Fp, n)
         checkpoints = []
-        # the last segment runs recorded (prt_lsrk_stage_record, bitwise the
-        # in-place stage): its tape spares the backward that recomputation
+        # the last segment runs recorded (the same stages, with a tape): that
+        # spares the backward its recomputation
         last = ((self.steps - 1) // self.K) * self.K if self.steps else 0
         Tmax = 5 * min(self.K, self.steps) if self.steps else 0
         tape = None
-        t = 0
         cs = C.c_void_p(stream_handle())
-        for step in range(self.steps):
-            if step % self.K == 0:
-                self._sort(el, x, p, q, m, kx, kp, order)
-                checkpoints.append((x.clone(), p.clone(), el.clone(), order.clone()))
-                if step == last:
-                    tape = (torch.empty((Tmax + 1, 3, n), dtype=F64, device=dev),
-                            torch.empty((Tmax + 1, 3, n), dtype=F64, device=dev),
-                            torch.empty((Tmax + 1, n), dtype=torch.int32, device=dev))
-                    tape[0][0].copy_(x)
-                    tape[1][0].copy_(p)
-                    tape[2][0].copy_(el)
-            if tape is None:
-                for a, b in zip(LSRK4_A, LSRK4_B):
-                    self._stage(Fp, x, p, q, m, el, kx, kp, a, b)
+        for step in range(0, self.steps, self.K):
+            self._sort(el, x, p, q, m, kx, kp, order)
+            checkpoints.append((x.clone(), p.clone(), el.clone(), order.clone()))
+            stages = 5 * min(self.K, self.steps - step)
+            if step != last:
+                _lib.check(self.lib.prt_lsrk_steps(
+                    *self._steps_args(Fp, coef, x, p, q, m, el, kx, kp, stages), cs),
+                    "prt_lsrk_steps")
                 continue
-            tx, tp, te = tape
-            for a, b in zip(LSRK4_A, LSRK4_B):
-                _lib.check(self.lib.prt_lsrk_stage_record(
-                    meth.pusher.handle, meth.workspace, n, tx[t].data_ptr(), tp[t].data_ptr(),
-                    te[t].data_ptr(), tx[t + 1].data_ptr(), tp[t + 1].data_ptr(),
-                    te[t + 1].data_ptr(), q.data_ptr(), m.data_ptr(), kx.data_ptr(),
-                    kp.data_ptr(), Fp, a, b, self.dt, self.c, cs), "prt_lsrk_stage_record")
-                t += 1
-        if tape is not None:
-            x = tape[0][t].clone()
-            p = tape[1][t].clone()
-            el = tape[2][t].clone()
+            tape = (torch.empty((Tmax + 1, 3, n), dtype=F64, device=dev),
+                    torch.empty((Tmax + 1, 3, n), dtype=F64, device=dev),
+                    torch.empty((Tmax + 1, n), dtype=torch.int32, device=dev))
+            tape[0][0].copy_(x)
+            tape[1][0].copy_(p)
+            tape[2][0].copy_(el)
+            _lib.check(self.lib.prt_lsrk_steps(
+                *self._steps_args(Fp, coef, tape[0][0], tape[1][0], q, m, tape[2][0], kx, kp,
+                                  stages, tape), cs), "prt_lsrk_steps")
+            x = tape[0][stages].clone()
+            p = tape[1][stages].clone()
+            el = tape[2][stages].clone()
         if not checkpoints:  # zero steps: the initial state is the final one
             self._sort(el, x, p, q, m, kx, kp, order)
             checkpoints.append((x.clone(), p.clone(), el.clone(), order.clone()))
@@ -247,16 +257,23 @@ class DifferentiableTrajectory:
         self._mark(marks, "deposit_adjoint")
         lam_kx = torch.zeros_like(x)
         lam_kp = torch.zeros_like(p)
-        comps = _field_components(F)
-        Fp = _ptrs(comps)
-        fcoef = monomial_coefficients(meth, comps)  # kept alive: Cp points into it
-        Cp = _ptrs(fcoef)
+        used = _nonzero(F)
+        Fp = _ptrs([F[k] if use else None for k, use in enumerate(used)])
+        mask = sum(1 << k for k, use in enumerate(used) if use)
+        coef = self._coefficients(Fp, n)  # the form the forward took
+        if want_fields:
+            # a launch per stage, coefficients per component
+            fcoef = monomial_coefficients(meth, [F[k] if use else None
+                                                 for k, use in enumerate(used)])
+            Cp = _ptrs(fcoef)
+        else:
+            adj_coef = meth.pusher.field_coefficients(Fp) if coef is None else coef
         nb = self.basis.shape[0] if (self.basis is not None and want_theta) else 0
         grad_theta = torch.zeros((max(nb, 1),), dtype=F64, device=dev)
         if nb:
-            bcomps = []
-            for k in range(nb):
-                bcomps += _field_components(self.basis[k])
+            bcomps = [self.basis[k, d] if use else None
+                      for k, row in enumerate(_nonzero(self.basis[:nb]))
+                      for d, use in enumerate(row)]
             bcoef = monomial_coefficients(meth, bcomps)  # kept alive: Bp points into it
             Bp = _ptrs(bcoef)
         else:
@@ -280,30 +297,40 @@ class DifferentiableTrajectory:
         ms = torch.empty_like(self.m)
         gth_ptr = grad_theta.data_ptr() if nb else None
         ptr = lambda t: t.data_ptr()  # noqa: E731
-        # launch arguments of every stage of a segment, built once
-        rec_args = [(meth.pusher.handle, meth.workspace, n, ptr(tx[t]), ptr(tp[t]), ptr(te[t]),
-                     ptr(tx[t + 1]), ptr(tp[t + 1]), ptr(te[t + 1]), ptr(qs), ptr(ms), ptr(kx),
-                     ptr(kp), Fp, LSRK4_A[t % 5], LSRK4_B[t % 5], self.dt, self.c)
-                    for t in range(Tmax)]
-        adj_args = [(meth.pusher.handle, meth.workspace, n, ptr(tx[t]), ptr(tp[t]), ptr(te[t]),
-                     ptr(qs), ptr(ms), ptr(lam_x), ptr(lam_p), ptr(lam_kx), ptr(lam_kp), Cp,
-                     LSRK4_A[t % 5], LSRK4_B[t % 5], self.dt, self.c, Gp, nb, Bp, gth_ptr)
-                    for t in range(Tmax)]
+        if want_fields:
+            # launch arguments of every stage adjoint of a segment, built once
+            adj_args = [(meth.pusher.handle, meth.workspace, n, ptr(tx[t]), ptr(tp[t]),
+                         ptr(te[t]), ptr(qs), ptr(ms), ptr(lam_x), ptr(lam_p), ptr(lam_kx),
+                         ptr(lam_kp), Cp, LSRK4_A[t % 5], LSRK4_B[t % 5], self.dt, self.c, Gp,
+                         nb, Bp, gth_ptr) for t in range(Tmax)]
+
+        def adjoint(T):
+            """The T stage adjoints in reverse, on the current stream."""
+            cs = C.c_void_p(stream_handle())
+            if not want_fields:
+                _lib.check(lib.prt_lsrk_steps_adjoint(
+                    meth.pusher.handle, meth.workspace, n, ptr(tx), ptr(tp), ptr(te), ptr(qs),
+                    ptr(ms), ptr(lam_x), ptr(lam_p), ptr(lam_kx), ptr(lam_kp), ptr(adj_coef),
+                    mask, _RK_A, _RK_B, 5, T, self.dt, self.c, nb, Bp, gth_ptr, cs),
+                    "prt_lsrk_steps_adjoint")
+            else:
+                for t in reversed(range(T)):
+                    _lib.check(lib.prt_lsrk_stage_adjoint(*adj_args[t], cs),
+                               "prt_lsrk_stage_adjoint")
+            self._mark(marks, "stage_adjoint")
 
         def segment(T):
             """Recompute T stages from tape slot 0, recording their inputs,
             then run the T stage adjoints in reverse, on the current stream
             (the capture stream while a graph is being captured)."""
-            cs = C.c_void_p(stream_handle())
-            kx.zero_()
-            kp.zero_()
-            for t in range(T):
-                _lib.check(lib.prt_lsrk_stage_record(*rec_args[t], cs), "prt_lsrk_stage_record")
+            _lib.check(lib.prt_lsrk_steps(*seg_args(T), C.c_void_p(stream_handle())),
+                       "prt_lsrk_steps")
             self._mark(marks, "recompute")
-            for t in reversed(range(T)):
-                _lib.check(lib.prt_lsrk_stage_adjoint(*adj_args[t], cs),
-                           "prt_lsrk_stage_adjoint")
-            self._mark(marks, "stage_adjoint")
+            adjoint(T)
+
+        def seg_args(T):
+            return self._steps_args(Fp, coef, tx[0], tp[0], qs, ms, te[0], kx, kp, T,
+                                    (tx, tp, te))
 
         graphs = self._graphs
         self._mark(marks, "setup")
@@ -327,20 +354,16 @@ class DifferentiableTrajectory:
             if fwd_tape is not None and seg == len(cps) - 1:
                 # recorded by the forward: the stage adjoints only
                 self._mark(marks, "carry")
-                cs = C.c_void_p(stream_handle())
-                for t in reversed(range(T)):
-                    _lib.check(lib.prt_lsrk_stage_adjoint(*adj_args[t], cs),
-                               "prt_lsrk_stage_adjoint")
-                self._mark(marks, "stage_adjoint")
+                adjoint(T)
                 continue
             tx[0].copy_(xs)
             tp[0].copy_(ps)
             te[0].copy_(els)
             self._mark(marks, "carry")
-            if not self.use_graphs or self.time_phases or seg == len(cps) - 1:
+            if not (want_fields and self.use_graphs) or self.time_phases or seg == len(cps) - 1:
                 segment(T)  # eager (the first one also sizes libprt's scratch)
                 continue
-            key = (T, tuple(tuple(_arg_key(a) for a in args) for args in rec_args[:T]),
+            key = (T, tuple(_arg_key(a) for a in seg_args(T)),
                    tuple(tuple(_arg_key(a) for a in args) for args in adj_args[:T]))
             g = graphs.get(key)
             if g is None:

@@ -297,6 +297,163 @@ __global__ void __launch_bounds__(ADJ_BLOCK, ORDER >= 4 ? 3 : ADJ_MIN_BLOCKS)
   }
 }
 
+// The adjoints of stages `stages` - 1 .. 0 of a tape, one thread per particle
+// with its adjoints in registers: a stage reads 52 bytes of the tape (loaded a
+// stage ahead) where a launch per stage moved 260, and the basis projections
+// are reduced once. Field coefficients interleaved ([E][6][COEF_ROW]), the
+// components of `mask`. Same arithmetic per stage as lsrk_stage_adjoint_kernel.
+// 300,000 particles, order 3, two basis fields: X us a stage, with a launch per
+// stage 100.
+template <int ORDER>
+__global__ void __launch_bounds__(ADJ_BLOCK, ORDER >= 4 ? 3 : 4)
+    lsrk_steps_adjoint_kernel(DevMesh M, const double2 *__restrict__ coef, uint32_t mask,
+                              const __grid_constant__ FieldBasis FB, long long n,
+                              const double *__restrict__ tx, const double *__restrict__ tp,
+                              const uint32_t *__restrict__ te, const double *__restrict__ q,
+                              const double *__restrict__ mass, double *__restrict__ lx,
+                              double *__restrict__ lp, double *__restrict__ lkx,
+                              double *__restrict__ lkp, const __grid_constant__ RkTable rk,
+                              int stages, double dt, double c,
+                              double *__restrict__ theta_partials) {
+  constexpr int NP = Lagrange<ORDER>::NP, ROW = COEF_ROW<ORDER>;
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  double tb[PRT_MAX_FIELD_BASIS];
+#pragma unroll
+  for (int k = 0; k < PRT_MAX_FIELD_BASIS; ++k) tb[k] = 0;
+  if (i < n) {
+    const double charge = q[i], m = mass[i], mc2 = m * m * c * c;
+    double ax[3], ap[3], akx[3], akp[3], x[3], p[3];
+    uint32_t e;
+    auto load = [&](int t) {
+      const double *sx = tx + (long long)t * 3 * n + i, *sp = tp + (long long)t * 3 * n + i;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        x[d] = __ldg(sx + d * n);
+        p[d] = __ldg(sp + d * n);
+      }
+      e = __ldg(te + (long long)t * n + i);
+    };
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      ax[d] = lx[d * n + i];
+      ap[d] = lp[d * n + i];
+      akx[d] = lkx[d * n + i];
+      akp[d] = lkp[d * n + i];
+    }
+    load(stages - 1);
+    int s = (stages - 1) % rk.n;
+#pragma unroll 1
+    for (int t = stages - 1; t >= 0; --t) {
+      const double a = rk.a[s], b = rk.b[s];
+      s = s == 0 ? rk.n - 1 : s - 1;
+      const uint32_t el = e;
+      double pp[3], r[3] = {0, 0, 0};
+      if (el != PRT_INVALID) reference_coords(M, el, x[0], x[1], x[2], r);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) pp[d] = p[d];
+      if (t > 0) load(t - 1);
+      if (el == PRT_INVALID) continue;  // passed through, as the stage left it untouched
+      double LX[3], LP[3], v[3], gE[3], gB[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        LX[d] = fma(b, ax[d], akx[d]);
+        LP[d] = fma(b, ap[d], akp[d]);
+      }
+      const double is = rsqrt(mc2 + pp[0] * pp[0] + pp[1] * pp[1] + pp[2] * pp[2]);
+      const double cs = c * is;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) v[d] = cs * pp[d];
+      {
+        double w[3];
+        cross3(LP, v, w);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          gE[d] = dt * charge * LP[d];
+          gB[d] = dt * charge * w[d];
+        }
+      }
+      const Powers<ORDER> pw(r);
+      double Bx[3] = {0, 0, 0}, gr[3] = {0, 0, 0};
+      const double2 *C = coef + (size_t)el * (6 * ROW / 2);
+      const size_t nb = (size_t)el * NP;
+      double2 u[6];
+      int idx = 0;
+#pragma unroll
+      for (int cc = 0; cc <= ORDER; ++cc)
+#pragma unroll
+        for (int bb = 0; bb <= ORDER - cc; ++bb)
+#pragma unroll
+          for (int aa = 0; aa <= ORDER - bb - cc; ++aa) {
+            const double mj = pw.p0[aa] * pw.p1[bb] * pw.p2[cc];
+            double h = 0;
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+              if (mask >> k & 1) {
+                if (idx % 2 == 0) u[k] = __ldg(C + k * (ROW / 2) + idx / 2);
+                const double ck = idx % 2 == 0 ? u[k].x : u[k].y;
+                if (k >= 3) Bx[k - 3] = fma(ck, mj, Bx[k - 3]);
+                h = fma(k < 3 ? gE[k] : gB[k - 3], ck, h);
+              }
+            if (aa > 0) gr[0] = fma(h, aa * pw.p0[aa - 1] * pw.p1[bb] * pw.p2[cc], gr[0]);
+            if (bb > 0) gr[1] = fma(h, bb * pw.p0[aa] * pw.p1[bb - 1] * pw.p2[cc], gr[1]);
+            if (cc > 0) gr[2] = fma(h, cc * pw.p0[aa] * pw.p1[bb] * pw.p2[cc - 1], gr[2]);
+#pragma unroll
+            for (int k = 0; k < PRT_MAX_FIELD_BASIS; ++k) {
+              if (k >= FB.count) break;
+              double hb = 0;
+#pragma unroll
+              for (int d = 0; d < 3; ++d) {
+                if (FB.f[k][d]) hb = fma(gE[d], __ldg(FB.f[k][d] + nb + idx), hb);
+                if (FB.f[k][3 + d]) hb = fma(gB[d], __ldg(FB.f[k][3 + d] + nb + idx), hb);
+              }
+              tb[k] = fma(hb, mj, tb[k]);
+            }
+            ++idx;
+          }
+      double w[3];
+      {
+        double z[3];
+        cross3(Bx, LP, z);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) w[d] = dt * (LX[d] + charge * z[d]);
+      }
+      const double pwd = (pp[0] * w[0] + pp[1] * w[1] + pp[2] * w[2]) * (is * is);
+      const double *A = M.inv_maps + 12 * (size_t)el;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        // r = A[0..8] x + A[9..11]: d r_k / d x_d = A[3k + d]
+        ax[d] += gr[0] * __ldg(A + d) + gr[1] * __ldg(A + 3 + d) + gr[2] * __ldg(A + 6 + d);
+        ap[d] += cs * (w[d] - pp[d] * pwd);
+        akx[d] = a * LX[d];
+        akp[d] = a * LP[d];
+      }
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      lx[d * n + i] = ax[d];
+      lp[d * n + i] = ap[d];
+      lkx[d * n + i] = akx[d];
+      lkp[d * n + i] = akp[d];
+    }
+  }
+  if (FB.count > 0) {
+    __shared__ double red[PRT_MAX_FIELD_BASIS][ADJ_BLOCK / 32];
+#pragma unroll
+    for (int k = 0; k < PRT_MAX_FIELD_BASIS; ++k) {
+      double t = tb[k];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < FB.count) {
+      double t = 0;
+      for (int w2 = 0; w2 < ADJ_BLOCK / 32; ++w2) t += red[threadIdx.x][w2];
+      theta_partials[(size_t)blockIdx.x * FB.count + threadIdx.x] = t;
+    }
+  }
+}
+
 // grad_theta[k] += sum over blocks of the partials, in a fixed order.
 __global__ void theta_reduce_kernel(long long blocks, int count,
                                     const double *__restrict__ partials,
@@ -556,6 +713,72 @@ extern "C" int prt_lsrk_stage_adjoint(const prt_pusher *P, prt_workspace *ws, in
     case 2: return dispatch_adjoint<2>(nodal, P, ws, n, x, p, el, q, m, lam_x, lam_p, lam_kx, lam_kp, F, FB, GF, a, b, dt, c, grad_theta, s);
     case 3: return dispatch_adjoint<3>(nodal, P, ws, n, x, p, el, q, m, lam_x, lam_p, lam_kx, lam_kp, F, FB, GF, a, b, dt, c, grad_theta, s);
     case 4: return dispatch_adjoint<4>(nodal, P, ws, n, x, p, el, q, m, lam_x, lam_p, lam_kx, lam_kp, F, FB, GF, a, b, dt, c, grad_theta, s);
+  }
+  return PRT_ERR_INVALID_ARGUMENT;
+}
+
+template <int ORDER>
+static int launch_steps_adjoint(const prt_pusher *P, prt_workspace *ws, const double *coef,
+                                uint32_t mask, const FieldBasis &FB, long long n,
+                                const double *tx, const double *tp, const uint32_t *te,
+                                const double *q, const double *m, double *lx, double *lp,
+                                double *lkx, double *lkp, const RkTable &rk, int stages,
+                                double dt, double c, double *grad_theta, cudaStream_t s) {
+  const long long blocks = prt_grid_blocks(n, ADJ_BLOCK);
+  double *partials = nullptr;
+  int rc = PRT_OK;
+  if (FB.count > 0) {
+    partials = (double *)ws_buffer(ws, PRT_WS_ADJ_PARTIALS,
+                                   sizeof(double) * (size_t)blocks * FB.count, &rc);
+    if (!partials) return rc;
+  }
+  {
+    ScopedTimer timer(ws, PRT_TIME_STAGE_ADJOINT, s);
+    lsrk_steps_adjoint_kernel<ORDER><<<blocks, ADJ_BLOCK, 0, s>>>(
+        P->mesh->dev, (const double2 *)coef, mask, FB, n, tx, tp, te, q, m, lx, lp, lkx, lkp, rk,
+        stages, dt, c, partials);
+    PRT_CHECK_CUDA(cudaGetLastError());
+  }
+  if (FB.count > 0) {
+    theta_reduce_kernel<<<1, 256, 0, s>>>(blocks, FB.count, partials, grad_theta);
+    PRT_CHECK_CUDA(cudaGetLastError());
+  }
+  return PRT_OK;
+}
+
+extern "C" int prt_lsrk_steps_adjoint(const prt_pusher *P, prt_workspace *ws, int64_t n,
+                                      const double *tx, const double *tp, const uint32_t *te,
+                                      const double *q, const double *m, double *lam_x,
+                                      double *lam_p, double *lam_kx, double *lam_kp,
+                                      const double *coef, uint32_t mask, const double *rk_a,
+                                      const double *rk_b, int32_t rk_count, int32_t stages,
+                                      double dt, double c, int32_t nbasis,
+                                      const double *const *basis, double *grad_theta,
+                                      void *stream) {
+  if (!P || !ws || n < 0 || stages < 0 || !rk_a || !rk_b || rk_count < 1 || rk_count > MAX_RK)
+    return PRT_ERR_INVALID_ARGUMENT;
+  if (nbasis < 0 || nbasis > PRT_MAX_FIELD_BASIS || (nbasis > 0 && (!basis || !grad_theta)))
+    return PRT_ERR_INVALID_ARGUMENT;
+  if (n == 0 || stages == 0) return PRT_OK;
+  if (!tx || !tp || !te || !q || !m || !lam_x || !lam_p || !lam_kx || !lam_kp || !coef ||
+      (uintptr_t)coef % 16)
+    return PRT_ERR_INVALID_ARGUMENT;
+  FieldBasis FB;
+  FB.count = nbasis;
+  for (int k = 0; k < PRT_MAX_FIELD_BASIS; ++k)
+    for (int d = 0; d < 6; ++d) FB.f[k][d] = k < nbasis ? basis[6 * k + d] : nullptr;
+  RkTable rk;
+  rk.n = rk_count;
+  for (int k = 0; k < MAX_RK; ++k) {
+    rk.a[k] = k < rk_count ? rk_a[k] : 0;
+    rk.b[k] = k < rk_count ? rk_b[k] : 0;
+  }
+  cudaStream_t s = (cudaStream_t)stream;
+  switch (P->order) {
+    case 1: return launch_steps_adjoint<1>(P, ws, coef, mask, FB, n, tx, tp, te, q, m, lam_x, lam_p, lam_kx, lam_kp, rk, stages, dt, c, grad_theta, s);
+    case 2: return launch_steps_adjoint<2>(P, ws, coef, mask, FB, n, tx, tp, te, q, m, lam_x, lam_p, lam_kx, lam_kp, rk, stages, dt, c, grad_theta, s);
+    case 3: return launch_steps_adjoint<3>(P, ws, coef, mask, FB, n, tx, tp, te, q, m, lam_x, lam_p, lam_kx, lam_kp, rk, stages, dt, c, grad_theta, s);
+    case 4: return launch_steps_adjoint<4>(P, ws, coef, mask, FB, n, tx, tp, te, q, m, lam_x, lam_p, lam_kx, lam_kp, rk, stages, dt, c, grad_theta, s);
   }
   return PRT_ERR_INVALID_ARGUMENT;
 }

@@ -90,6 +90,33 @@ static Lagrange<ORDER> make_lagrange(const prt_pusher *P) {
   return L;
 }
 
+// The RK coefficients of a run of stages: stage t uses a[t % n], b[t % n].
+constexpr int MAX_RK = 8;
+struct RkTable {
+  double a[MAX_RK], b[MAX_RK];
+  int n;
+};
+
+// Powers of the reference coordinates.
+template <int ORDER>
+struct Powers {
+  double p0[ORDER + 1], p1[ORDER + 1], p2[ORDER + 1];
+  __device__ __forceinline__ explicit Powers(const double r[3]) {
+    p0[0] = p1[0] = p2[0] = 1.0;
+#pragma unroll
+    for (int k = 1; k <= ORDER; ++k) {
+      p0[k] = p0[k - 1] * r[0];
+      p1[k] = p1[k - 1] * r[1];
+      p2[k] = p2[k - 1] * r[2];
+    }
+  }
+};
+
+// Entries per field and element of FP64 monomial coefficients (Np rounded up
+// to even), [E][6][ROW].
+template <int ORDER>
+constexpr int COEF_ROW = (Lagrange<ORDER>::NP + 1) / 2 * 2;
+
 // RK update of one particle: k = a k + dt f, y += b k (rounded as written).
 __device__ __forceinline__ void rk_update(double a, double b, double dt, double f, double &k,
                                           double &y) {

@@ -35,30 +35,11 @@
 namespace {
 
 constexpr int ST_BLOCK = 128;
-constexpr int MAX_RK = 8;
-
-struct RkTable {
-  double a[MAX_RK], b[MAX_RK];
-  int n;
-};
-
+// The state after every stage; in_place: the store is updated too.
 struct Tape {
   double *__restrict__ x, *__restrict__ p;  // [stages + 1][3][n], slots 1.. written
   uint32_t *__restrict__ el;                // [stages + 1][n]
-};
-
-template <int ORDER>
-struct Powers {
-  double p0[ORDER + 1], p1[ORDER + 1], p2[ORDER + 1];
-  __device__ __forceinline__ explicit Powers(const double r[3]) {
-    p0[0] = p1[0] = p2[0] = 1.0;
-#pragma unroll
-    for (int k = 1; k <= ORDER; ++k) {
-      p0[k] = p0[k - 1] * r[0];
-      p1[k] = p1[k - 1] * r[1];
-      p2[k] = p2[k - 1] * r[2];
-    }
-  }
+  bool in_place;
 };
 
 // The monomials of a point in pairs or quadruples, in the canonical order:
@@ -92,7 +73,7 @@ __device__ __forceinline__ void monomial_groups(const double r[3], V &&visit) {
 // of two monomials' coefficients of one field.
 template <int ORDER>
 struct Coefficients64 {
-  static constexpr int ROW = (Lagrange<ORDER>::NP + 1) / 2 * 2;
+  static constexpr int ROW = COEF_ROW<ORDER>;
   const double2 *__restrict__ c;
   __device__ __forceinline__ void fields(const DevMesh &, uint32_t e, const double r[3],
                                          const double *, double ef[6]) const {
@@ -237,12 +218,14 @@ __global__ void __launch_bounds__(ST_BLOCK, MIN_BLOCKS)
   if (mine && stages > 0) {
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      x[d * n + i] = xx[d];
-      p[d * n + i] = pp[d];
       kx[d * n + i] = kxx[d];
       kp[d * n + i] = kpp[d];
+      if (tape.in_place) {
+        x[d * n + i] = xx[d];
+        p[d * n + i] = pp[d];
+      }
     }
-    el[i] = e;
+    if (tape.in_place) el[i] = e;
   }
   flush_counters(st, ctr);
 }
@@ -440,6 +423,9 @@ extern "C" int prt_lsrk_steps(const prt_pusher *P, prt_workspace *ws, int64_t n,
   if (!x || !p || !q || !m || !el || !kx || !kp) return PRT_ERR_INVALID_ARGUMENT;
   if ((tape_x || tape_p || tape_el) && (!tape_x || !tape_p || !tape_el))
     return PRT_ERR_INVALID_ARGUMENT;
+  // a store that is the tape's slot 0 is that in all three arrays
+  if ((x == tape_x) != (p == tape_p) || (x == tape_x) != (el == tape_el))
+    return PRT_ERR_INVALID_ARGUMENT;
   Fields6 F;
   for (int k = 0; k < 6; ++k) F.f[k] = fields ? fields[k] : nullptr;
   StepArgs A;
@@ -462,6 +448,7 @@ extern "C" int prt_lsrk_steps(const prt_pusher *P, prt_workspace *ws, int64_t n,
   A.tape.x = tape_x;
   A.tape.p = tape_p;
   A.tape.el = tape_el;
+  A.tape.in_place = x != tape_x;
   cudaStream_t s = (cudaStream_t)stream;
   switch (P->order) {
     case 1: return steps<1>(P, ws, coef, F, precision, A, s);
