@@ -297,6 +297,13 @@ __global__ void __launch_bounds__(ADJ_BLOCK, ORDER >= 4 ? 3 : ADJ_MIN_BLOCKS)
   }
 }
 
+// The non-zero components of the basis fields.
+struct BasisList {
+  int bases, count;
+  const double *f[6 * PRT_MAX_FIELD_BASIS];
+  int comp[6 * PRT_MAX_FIELD_BASIS], basis[6 * PRT_MAX_FIELD_BASIS];
+};
+
 // The adjoints of stages `stages` - 1 .. 0 of a tape, one thread per particle
 // with its adjoints in registers: a stage reads 52 bytes of the tape (loaded a
 // stage ahead) where a launch per stage moved 260, and the basis projections
@@ -307,7 +314,7 @@ __global__ void __launch_bounds__(ADJ_BLOCK, ORDER >= 4 ? 3 : ADJ_MIN_BLOCKS)
 template <int ORDER>
 __global__ void __launch_bounds__(ADJ_BLOCK, ORDER >= 4 ? 3 : 4)
     lsrk_steps_adjoint_kernel(DevMesh M, const double2 *__restrict__ coef, uint32_t mask,
-                              const __grid_constant__ FieldBasis FB, long long n,
+                              const __grid_constant__ BasisList FB, long long n,
                               const double *__restrict__ tx, const double *__restrict__ tp,
                               const uint32_t *__restrict__ te, const double *__restrict__ q,
                               const double *__restrict__ mass, double *__restrict__ lx,
@@ -397,19 +404,35 @@ __global__ void __launch_bounds__(ADJ_BLOCK, ORDER >= 4 ? 3 : 4)
             if (aa > 0) gr[0] = fma(h, aa * pw.p0[aa - 1] * pw.p1[bb] * pw.p2[cc], gr[0]);
             if (bb > 0) gr[1] = fma(h, bb * pw.p0[aa] * pw.p1[bb - 1] * pw.p2[cc], gr[1]);
             if (cc > 0) gr[2] = fma(h, cc * pw.p0[aa] * pw.p1[bb] * pw.p2[cc - 1], gr[2]);
-#pragma unroll
-            for (int k = 0; k < PRT_MAX_FIELD_BASIS; ++k) {
-              if (k >= FB.count) break;
-              double hb = 0;
-#pragma unroll
-              for (int d = 0; d < 3; ++d) {
-                if (FB.f[k][d]) hb = fma(gE[d], __ldg(FB.f[k][d] + nb + idx), hb);
-                if (FB.f[k][3 + d]) hb = fma(gB[d], __ldg(FB.f[k][3 + d] + nb + idx), hb);
-              }
-              tb[k] = fma(hb, mj, tb[k]);
-            }
             ++idx;
           }
+      // the basis fields' non-zero components, one after the other: the value
+      // at x times its adjoint (unrolled over basis and component too, the
+      // loop above outgrew the instruction cache)
+#pragma unroll 1
+      for (int o = 0; o < FB.count; ++o) {
+        const double *f = FB.f[o] + nb;
+        const int comp = FB.comp[o], base = FB.basis[o];
+        double val = 0;
+        int at = 0;
+#pragma unroll
+        for (int cc = 0; cc <= ORDER; ++cc)
+#pragma unroll
+          for (int bb = 0; bb <= ORDER - cc; ++bb) {
+            const double t2 = pw.p1[bb] * pw.p2[cc];
+#pragma unroll
+            for (int aa = 0; aa <= ORDER - bb - cc; ++aa)
+              val = fma(__ldg(f + at++), pw.p0[aa] * t2, val);
+          }
+        const double g = comp == 0   ? gE[0]
+                         : comp == 1 ? gE[1]
+                         : comp == 2 ? gE[2]
+                         : comp == 3 ? gB[0]
+                         : comp == 4 ? gB[1]
+                                     : gB[2];
+#pragma unroll
+        for (int k = 0; k < PRT_MAX_FIELD_BASIS; ++k) tb[k] = fma(k == base ? g : 0.0, val, tb[k]);
+      }
       double w[3];
       {
         double z[3];
@@ -436,7 +459,7 @@ __global__ void __launch_bounds__(ADJ_BLOCK, ORDER >= 4 ? 3 : 4)
       lkp[d * n + i] = akp[d];
     }
   }
-  if (FB.count > 0) {
+  if (FB.bases > 0) {
     __shared__ double red[PRT_MAX_FIELD_BASIS][ADJ_BLOCK / 32];
 #pragma unroll
     for (int k = 0; k < PRT_MAX_FIELD_BASIS; ++k) {
@@ -446,10 +469,10 @@ __global__ void __launch_bounds__(ADJ_BLOCK, ORDER >= 4 ? 3 : 4)
       if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = t;
     }
     __syncthreads();
-    if (threadIdx.x < FB.count) {
+    if (threadIdx.x < FB.bases) {
       double t = 0;
       for (int w2 = 0; w2 < ADJ_BLOCK / 32; ++w2) t += red[threadIdx.x][w2];
-      theta_partials[(size_t)blockIdx.x * FB.count + threadIdx.x] = t;
+      theta_partials[(size_t)blockIdx.x * FB.bases + threadIdx.x] = t;
     }
   }
 }
@@ -719,7 +742,7 @@ extern "C" int prt_lsrk_stage_adjoint(const prt_pusher *P, prt_workspace *ws, in
 
 template <int ORDER>
 static int launch_steps_adjoint(const prt_pusher *P, prt_workspace *ws, const double *coef,
-                                uint32_t mask, const FieldBasis &FB, long long n,
+                                uint32_t mask, const BasisList &FB, long long n,
                                 const double *tx, const double *tp, const uint32_t *te,
                                 const double *q, const double *m, double *lx, double *lp,
                                 double *lkx, double *lkp, const RkTable &rk, int stages,
@@ -727,9 +750,9 @@ static int launch_steps_adjoint(const prt_pusher *P, prt_workspace *ws, const do
   const long long blocks = prt_grid_blocks(n, ADJ_BLOCK);
   double *partials = nullptr;
   int rc = PRT_OK;
-  if (FB.count > 0) {
+  if (FB.bases > 0) {
     partials = (double *)ws_buffer(ws, PRT_WS_ADJ_PARTIALS,
-                                   sizeof(double) * (size_t)blocks * FB.count, &rc);
+                                   sizeof(double) * (size_t)blocks * FB.bases, &rc);
     if (!partials) return rc;
   }
   {
@@ -739,8 +762,8 @@ static int launch_steps_adjoint(const prt_pusher *P, prt_workspace *ws, const do
         stages, dt, c, partials);
     PRT_CHECK_CUDA(cudaGetLastError());
   }
-  if (FB.count > 0) {
-    theta_reduce_kernel<<<1, 256, 0, s>>>(blocks, FB.count, partials, grad_theta);
+  if (FB.bases > 0) {
+    theta_reduce_kernel<<<1, 256, 0, s>>>(blocks, FB.bases, partials, grad_theta);
     PRT_CHECK_CUDA(cudaGetLastError());
   }
   return PRT_OK;
@@ -763,10 +786,16 @@ extern "C" int prt_lsrk_steps_adjoint(const prt_pusher *P, prt_workspace *ws, in
   if (!tx || !tp || !te || !q || !m || !lam_x || !lam_p || !lam_kx || !lam_kp || !coef ||
       (uintptr_t)coef % 16)
     return PRT_ERR_INVALID_ARGUMENT;
-  FieldBasis FB;
-  FB.count = nbasis;
-  for (int k = 0; k < PRT_MAX_FIELD_BASIS; ++k)
-    for (int d = 0; d < 6; ++d) FB.f[k][d] = k < nbasis ? basis[6 * k + d] : nullptr;
+  BasisList FB;
+  FB.bases = nbasis;
+  FB.count = 0;
+  for (int k = 0; k < nbasis; ++k)
+    for (int d = 0; d < 6; ++d)
+      if (basis[6 * k + d]) {
+        FB.f[FB.count] = basis[6 * k + d];
+        FB.comp[FB.count] = d;
+        FB.basis[FB.count++] = k;
+      }
   RkTable rk;
   rk.n = rk_count;
   for (int k = 0; k < MAX_RK; ++k) {
