@@ -309,7 +309,7 @@ struct BasisList {
 // stage ahead) where a launch per stage moved 260, and the basis projections
 // are reduced once. Field coefficients interleaved ([E][6][COEF_ROW]), the
 // components of `mask`. Same arithmetic per stage as lsrk_stage_adjoint_kernel.
-// 300,000 particles, order 3, two basis fields: X us a stage, with a launch per
+// 300,000 particles, order 3, two basis fields: 24 us a stage, with a launch per
 // stage 100.
 template <int ORDER>
 __global__ void __launch_bounds__(ADJ_BLOCK, ORDER >= 4 ? 3 : 4)

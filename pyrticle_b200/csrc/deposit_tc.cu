@@ -23,12 +23,11 @@
 //     coordinates (v = 2 SIGMA w), the position term SIGMA (1 - |u|^2) and
 //     the particle term -SIGMA |w|^2, each as two terms; the tensor cores
 //     accumulate in FP32 into tensor memory;
-//  3. weight: each thread reads its row (tcgen05.ld), forms
-//     t = s + |s| = 2 max(s, 0) and the integer F = round(t^2) =
-//     round(4 SIGMA^2 max(1 - r^2/a^2, 0)^2) < 2^23 with one FMA
-//     (t t + 2^23 puts the rounded integer in the low mantissa bits), and
-//     writes the word back in place (tcgen05.st): its bytes 0-2 are F's
-//     base-256 digits, byte 3 a constant;
+//  3. weight: each thread reads its row (tcgen05.ld), forms t = max(s, 0)
+//     and the integer F = round(4 t^2) = round(4 SIGMA^2 max(1 - r^2/a^2, 0)^2)
+//     < 2^23 with half a packed FMA (t t + 2^21, whose last place is 1/4, has
+//     F in its low mantissa bits), and writes the word back in place
+//     (tcgen05.st): its bytes 0-2 are F's base-256 digits, byte 3 a constant;
 //  4. sums: tcgen05.mma kind::i8 with A in tensor memory (the weight words
 //     as unsigned 8-bit K elements; int32 accumulation, exact) against digit
 //     rows in shared memory laid out so that three views one row apart
@@ -103,7 +102,7 @@ struct Smem {
   uint8_t apos[2 * TM * 16];     // position operand, K-major: [K chunk][row][16 B]
   uint8_t bcand[2 * RING * 16];  // candidate operands, K-major: [K chunk][slot][16 B]
   // The sums' B operand (MN-major rows of 16 digit bytes, one row per K): a
-  // weight word holds the K elements 4 c .. 4 c + 3 (bytes 0-3 of F + 2^23),
+  // weight word holds the K elements 4 c .. 4 c + 3 (bytes 0-3 of the word),
   // so each candidate (deposition) or position (normalisation) c has four
   // rows, its digits in row 4 c + 3 and zeros in 4 c .. 4 c + 2; three views
   // one row apart (SBO 16 bytes) multiply bytes 2, 1, 0 by the digits
@@ -350,14 +349,21 @@ __device__ __forceinline__ void candidate_operand(float w0, float w1, float w2, 
   k1 = make_uint4((H2G & 0xffffu) | (ONE << 16), ONE | (H2G & 0xffff0000u), L2G >> 16, 0u);
 }
 
-// Bin-row segments of a tile (warp 0): every run of bins along x, in the
-// rows (bz, by) within the radius of the box [c - hf, c + hf], as ranges of
-// bin-order particles with the origin of the run's first bin relative to the
-// tile centre (periodic image included, FP64 rounded once to FP32: within
-// 2.5 radii, so to ~2e-7 radii); the stream of candidates is the
-// concatenation of the segments.
-__device__ void build_segments(Smem &S, const TcArgs &A, const double c[3], const double hf[3],
-                               int lane) {
+// Bin-row segments of a tile (all warps, a row per thread): every run of bins
+// along x, in the rows (bz, by) within the radius of the box [c - hf, c + hf],
+// as ranges of bin-order particles with the origin of the run's first bin
+// relative to the tile centre (periodic image included, FP64 rounded once to
+// FP32: within 2.5 radii, so to ~2e-7 radii); the stream of candidates is the
+// concatenation of the segments, in the order in which the warps add theirs
+// (the sums do not depend on it). S.nseg starts at zero; a tile of more than
+// MAXSEG segments sets S.abort. The rows' starts are loads that depend on one
+// another, and no more than two CTAs share an SM, so the tile waits for them:
+// with one warp taking 32 rows at a time a whole step of 16M particles,
+// normalised, took 78.2 ms, with all eight at once 76.0; 10k particles 523 us
+// and 475.
+__device__ __forceinline__ void build_segments(Smem &S, const TcArgs &A, const double c[3],
+                                               const double hf[3]) {
+  const int lane = threadIdx.x & 31;
   const BinGrid &G = A.G;
   const double rr = A.radius * (1 + 1e-5), rr2 = rr * rr;
   int ulo[3], uhi[3];
@@ -380,10 +386,9 @@ __device__ void build_segments(Smem &S, const TcArgs &A, const double c[3], cons
   };
   const int ny = max(0, uhi[1] - ulo[1] + 1), nz = max(0, uhi[2] - ulo[2] + 1);
   const int nrows = ny * nz;
-  int nseg = 0;
-  bool overflow = false;
-  for (int r0 = 0; r0 < nrows; r0 += 32) {
+  for (int r0 = (int)(threadIdx.x - lane); r0 < nrows; r0 += THREADS) {
     const int r = r0 + lane;
+    bool overflow = false;
     uint32_t s_start[3], s_len[3];
     float s_ox[3], s_bx[3], oy = 0, oz = 0;
     int cnt = 0;
@@ -445,22 +450,18 @@ __device__ void build_segments(Smem &S, const TcArgs &A, const double c[3], cons
       const int c2 = __shfl_up_sync(0xffffffffu, cs, o);
       if (lane >= o) cs += c2;
     }
-    const int sbase = nseg + cs - cnt;
+    int base = 0;
+    if (lane == 31 && cs > 0) base = atomicAdd(&S.nseg, cs);
+    const int sbase = __shfl_sync(0xffffffffu, base, 31) + cs - cnt;
     for (int i = 0; i < cnt; ++i) {
       if (sbase + i < MAXSEG) {
         S.seg_sl[sbase + i] = make_uint2(s_start[i], s_len[i]);
         S.seg_o[sbase + i] = make_float4(s_ox[i], oy, oz, s_bx[i]);
+      } else {
+        overflow = true;
       }
     }
-    nseg += __shfl_sync(0xffffffffu, cs, 31);
-  }
-  overflow = __any_sync(0xffffffffu, overflow) || nseg > MAXSEG;
-  if (lane == 0) {
-    S.nseg = overflow ? 0 : nseg;
-    if (overflow) {
-      S.abort = 1;
-      record_error(A.st, PRT_ERR_CAPACITY, -1);
-    }
+    if (overflow && atomicExch(&S.abort, 1) == 0) record_error(A.st, PRT_ERR_CAPACITY, -1);
   }
 }
 
@@ -508,7 +509,7 @@ __device__ __forceinline__ void cursor_init(const Smem &S, const TcArgs &A, Curs
                                             int lane) {
   C.cseg = warp;
   C.coff = 0;
-  C.nseg = S.nseg;
+  C.nseg = S.abort ? 0 : S.nseg;
   C.rot = 0;
   C.q0.pos = C.q1.pos = C.q2.pos = make_float4(0, 0, 0, 0);
   C.q0.dig = C.q1.dig = C.q2.dig = make_uint4(0, 0, 0, 0);
@@ -594,10 +595,15 @@ __device__ __forceinline__ void pad_chunk(Smem &S, int from, int to, int tid) {
 // The weights of one chunk, in place in tensor memory: thread (warp w, lane
 // l) takes row 32 (w % 4) + l (a position in the deposition pass, a
 // candidate in the normalisation pass) and columns 64 (w / 4) .. + 63, reads
-// the scores s (tcgen05.ld), and writes back the words F + 2^23 with
-// F = round(t^2), t = s + |s| (one FMA: t t + 2^23 puts the rounded integer
-// in the low mantissa bits), so bytes 0-2 are F's base-256 digits and byte 3
-// a constant the sums multiply by zero. Counts the words with F > 0 (hits).
+// the scores s (tcgen05.ld), and writes back the words 2^21 + t^2 with
+// t = max(s, 0): the sum is rounded to quarters, so its low 23 bits are
+// F = round(4 t^2), bytes 0-2 are F's base-256 digits (bit 23, the exponent's
+// lowest, is zero) and byte 3 a constant the sums multiply by zero. The issue
+// slots bound the kernel (a half to six tenths of them in use, the FMA units a
+// third), so a weight takes one maximum on the integer units and half of a
+// two-wide FMA: 16M particles, normalised, 71.1 -> 69.0 ms against two
+// one-wide FP32 operations per weight, the same bits. Counts the words with
+// F > 0 (hits).
 template <bool HITS>
 __device__ __forceinline__ uint32_t weights(uint32_t tmem, int warp, int lane) {
   const uint32_t base = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(64 * (warp >> 2));
@@ -608,12 +614,19 @@ __device__ __forceinline__ uint32_t weights(uint32_t tmem, int warp, int lane) {
     tmem_ld32(base + 32 * half, r);
     tmem_wait_ld();
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float sc = __uint_as_float(r[i]);
-      const float t = sc + fabsf(sc);                        // 2 max(s, 0), exact
-      const float f = fmaf(t, t, 8388608.0f);                // 2^23 + round(t^2)
-      r[i] = __float_as_uint(f);
-      if (HITS) hits += __saturatef(f - 8388608.0f);         // F > 0: 1, else 0
+    for (int i = 0; i < 32; i += 2) {
+      const float t0 = fmaxf(__uint_as_float(r[i]), 0.0f);
+      const float t1 = fmaxf(__uint_as_float(r[i + 1]), 0.0f);
+      asm("{\n\t.reg .b64 t, c;\n\t"
+          "mov.b64 t, {%2, %3};\n\t"
+          "mov.b64 c, {%4, %4};\n\t"
+          "fma.rn.f32x2 t, t, t, c;\n\t"
+          "mov.b64 {%0, %1}, t;\n\t}\n"
+          : "=r"(r[i]), "=r"(r[i + 1])
+          : "f"(t0), "f"(t1), "f"(2097152.0f));
+      if (HITS)  // F > 0: 1, else 0
+        hits += __saturatef(fmaf(__uint_as_float(r[i]), 4.0f, -8388608.0f)) +
+                __saturatef(fmaf(__uint_as_float(r[i + 1]), 4.0f, -8388608.0f));
     }
     tmem_st32(base + 32 * half, r);
   }
@@ -684,6 +697,7 @@ __global__ void __launch_bounds__(THREADS, 2) tc_deposit_kernel(TcArgs A) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&S.bar_a)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     S.tail = 0;
+    S.nseg = 0;
     S.abort = 0;
   }
   {
@@ -701,7 +715,7 @@ __global__ void __launch_bounds__(THREADS, 2) tc_deposit_kernel(TcArgs A) {
     }
   }
   __syncthreads();
-  if (warp == 0) build_segments(S, A, c, hfd, lane);
+  build_segments(S, A, c, hfd);
   fence_async_smem();
   fence_before();
   __syncthreads();
@@ -738,9 +752,13 @@ __global__ void __launch_bounds__(THREADS, 2) tc_deposit_kernel(TcArgs A) {
 
   // readout of a normalisation chunk: per candidate its sum over the tile,
   // P = H 2^40 + L (0 <= L < 2^40), both parts added exactly to the
-  // particle's integral (H modulo 2^64): warps 0-3 add H, warps 4-7 add L
-  // and the hit count (a warp reads the tensor-memory lanes 32 (warp % 4) ..)
+  // particle's integral (H modulo 2^64), and the hit count. Warps 0-3 take the
+  // even chunks, warps 4-7 the odd ones (a warp reads the tensor-memory lanes
+  // 32 (warp % 4) ..): with H on one half of the warps and L on the other both
+  // did all the arithmetic, 9.92 ms for the pass over 4M particles against
+  // 9.66.
   auto norm_readout = [&](int chunk, int nvalid) {
+    if ((warp >> 2) != (chunk & 1)) return;
     uint32_t d2[8], d1[8], d0[8];
     const uint32_t lane_addr = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
     tmem_ld8(lane_addr + COL_ACC, d2);
@@ -766,14 +784,11 @@ __global__ void __launch_bounds__(THREADS, 2) tc_deposit_kernel(TcArgs A) {
       const long long L = l1 & M40;
       const long long H = (plo >> 40) + (phi >> 8) + (l1 >> 40);
       const uint32_t id = S.n.slot_id[(chunk * NC + cr) % RING];
-      if (warp < 4) {
-        if (H != 0) atomicAdd(A.norm_hi + id, (unsigned long long)H);
-      } else {
-        if (L != 0) atomicAdd(A.norm_lo + id, (unsigned long long)L);
-        if (IND) {
-          const uint32_t h = S.n.hits[chunk & 1][0][cr] + S.n.hits[chunk & 1][1][cr];
-          if (h) atomicAdd(A.hits + id, h);
-        }
+      if (H != 0) atomicAdd(A.norm_hi + id, (unsigned long long)H);
+      if (L != 0) atomicAdd(A.norm_lo + id, (unsigned long long)L);
+      if (IND) {
+        const uint32_t h = S.n.hits[chunk & 1][0][cr] + S.n.hits[chunk & 1][1][cr];
+        if (h) atomicAdd(A.hits + id, h);
       }
     }
   };
