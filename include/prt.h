@@ -623,6 +623,13 @@ int prt_sort_by_element(prt_workspace *ws, int64_t n, uint32_t *elements,
                         double *masses, double *kx, double *kp, int64_t *ids,
                         void *stream);
 
+/* The same with every element an element of `mesh` or PRT_INVALID_ELEMENT: the
+ * sort then reads only the key bits that tell these apart. */
+int prt_sort_by_element_of(const prt_mesh *mesh, prt_workspace *ws, int64_t n,
+                           uint32_t *elements, double *positions, double *momenta,
+                           double *charges, double *masses, double *kx, double *kp,
+                           int64_t *ids, void *stream);
+
 /* Library version string. */
 const char *prt_version(void);
 

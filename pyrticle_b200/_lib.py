@@ -172,6 +172,8 @@ SIGNATURES = {
     "prt_remap_grid_to_mesh": (_i32, [_vp, _vp, _vp, _i64, _i64, _vp]),
     "prt_remap_grid_to_mesh_components": (_i32, [_vp, _vp, _vp, _i32, _vp]),
     "prt_sort_by_element": (_i32, [_vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "prt_sort_by_element_of": (_i32, [_vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
+                                      _vp]),
     "prt_lsrk_stage_record": (_i32, [_vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp,
                                      _vp, _vp, _vp, C.POINTER(_vp), _d, _d, _d, _d, _vp]),
     "prt_lsrk_stage_adjoint": (_i32, [_vp, _vp, _i64, _vp, _vp, _vp, _vp, _vp, _vp, _vp,

@@ -154,10 +154,10 @@ class DifferentiableTrajectory:
                 *((None,) * 3 if tape is None else [t.data_ptr() for t in tape]))
 
     def _sort(self, el, x, p, q, m, kx, kp, order):
-        _lib.check(self.lib.prt_sort_by_element(
-            self.method.workspace, x.shape[1], el.data_ptr(), x.data_ptr(), p.data_ptr(),
+        _lib.check(self.lib.prt_sort_by_element_of(
+            self.method.mesh_data.handle, self.method.workspace, x.shape[1], el.data_ptr(), x.data_ptr(), p.data_ptr(),
             q.data_ptr(), m.data_ptr(), kx.data_ptr(), kp.data_ptr(), order.data_ptr(),
-            C.c_void_p(stream_handle())), "prt_sort_by_element")
+            C.c_void_p(stream_handle())), "prt_sort_by_element_of")
 
     def _velocities(self, p, m):
         v = torch.empty_like(p)

@@ -552,12 +552,12 @@ class PicMethod:
         """Sort the store by containing element; `residuals=False` leaves the
         LSRK residuals unpermuted (valid only at a step boundary)."""
         kx, kp = state.residuals()
-        _lib.check(self.lib.prt_sort_by_element(
-            self.workspace, len(state), state.el.data_ptr(), state.x.data_ptr(),
+        _lib.check(self.lib.prt_sort_by_element_of(
+            self.mesh_data.handle, self.workspace, len(state), state.el.data_ptr(), state.x.data_ptr(),
             state.p.data_ptr(), state.q.data_ptr(), state.m.data_ptr(),
             kx.data_ptr() if residuals else None, kp.data_ptr() if residuals else None,
             state.ids.data_ptr(), C.c_void_p(stream_handle())),
-            "prt_sort_by_element")
+            "prt_sort_by_element_of")
         state.element_sorted = True
         state.derived_quantity_cache.clear()
 
