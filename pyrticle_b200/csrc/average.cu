@@ -26,34 +26,43 @@ using namespace prt_dep;
 template <bool SQUARES>
 constexpr int AVG_NV = SQUARES ? 9 : 7;
 
-// Per tile row the record (x, y, z, values).
+// Per tile row the record (x, y, z, values); RUN_LANES lanes share a row.
 template <bool SQUARES>
 __global__ void average_records_kernel(TilesDev T, int np, const uint32_t *__restrict__ run_starts,
                                        const uint32_t *__restrict__ run_nodes,
-                                       const double *__restrict__ iw,
+                                       const __grid_constant__ NodeWeights N,
                                        const double *__restrict__ jac, Fields6 F,
                                        double2 *__restrict__ records) {
   constexpr int NV = AVG_NV<SQUARES>, RAW = BlockStage<NV>::RAW;
-  const long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (r >= T.count) return;
-  const uint32_t u = T.rows[r];
+  __shared__ double shared[PRT_NODE_WEIGHTS];
+  const double *iw = stage_node_weights(N, np, shared);
+  const long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / RUN_LANES;
+  const int part = threadIdx.x % RUN_LANES;
   double s[2 * RAW];
 #pragma unroll
-  for (int k = 0; k < 2 * RAW; ++k) s[k] = k < 3 ? T.pos[3 * r + k] : 0;
-  for (uint32_t k = run_starts[u]; k < run_starts[u + 1]; ++k) {
-    const uint32_t node = run_nodes[k];
-    const double w = iw[node % np] * jac[node / np];
-    double f[6];
+  for (int k = 0; k < 2 * RAW; ++k) s[k] = 0;
+  if (r < T.count) {
+    const uint32_t u = T.rows[r];
+    for (uint32_t k = run_starts[u] + part; k < run_starts[u + 1]; k += RUN_LANES) {
+      const uint32_t node = run_nodes[k];
+      const double w = iw[node % np] * jac[node / np];
+      double f[6];
 #pragma unroll
-    for (int c = 0; c < 6; ++c) f[c] = F.f[c] ? F.f[c][node] : 0.0;
-    s[3] += w;
+      for (int c = 0; c < 6; ++c) f[c] = F.f[c] ? F.f[c][node] : 0.0;
+      s[3] += w;
 #pragma unroll
-    for (int c = 0; c < 6; ++c) s[4 + c] += w * f[c];
-    if (SQUARES) {
-      s[10] += w * (f[0] * f[0] + f[1] * f[1] + f[2] * f[2]);
-      s[11] += w * (f[3] * f[3] + f[4] * f[4] + f[5] * f[5]);
+      for (int c = 0; c < 6; ++c) s[4 + c] += w * f[c];
+      if (SQUARES) {
+        s[10] += w * (f[0] * f[0] + f[1] * f[1] + f[2] * f[2]);
+        s[11] += w * (f[3] * f[3] + f[4] * f[4] + f[5] * f[5]);
+      }
     }
   }
+#pragma unroll
+  for (int k = 3; k < 3 + NV; ++k) s[k] = sum_run(s[k]);
+  if (r >= T.count || part != 0) return;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) s[k] = T.pos[3 * r + k];
 #pragma unroll
   for (int k = 0; k < RAW; ++k) records[RAW * r + k] = make_double2(s[2 * k], s[2 * k + 1]);
 }
@@ -216,12 +225,11 @@ int average_forces(const prt_mesh *mesh, prt_workspace *ws, const prt_shape_func
   double2 *records =
       (double2 *)ws_buffer(ws, PRT_WS_AVERAGE, sizeof(double2) * rec + sizeof(double) * np, &rc);
   if (!records) return rc;
-  double *iwd = (double *)(records + rec);
-  PRT_CHECK_CUDA(
-      cudaMemcpyAsync(iwd, integral_weights, sizeof(double) * np, cudaMemcpyHostToDevice, s));
+  NodeWeights N;
+  if ((rc = prt_node_weights(integral_weights, np, (double *)(records + rec), &N, s))) return rc;
   const TilesDev T = tiles_dev(PS.tiles);
-  average_records_kernel<SQUARES><<<prt_grid_blocks(PS.count, 128), 128, 0, s>>>(
-      T, np, PS.run_starts, PS.run_nodes, iwd, mesh->dev.jacobians, F, records);
+  average_records_kernel<SQUARES><<<prt_grid_blocks(RUN_LANES * PS.count, 128), 128, 0, s>>>(
+      T, np, PS.run_starts, PS.run_nodes, N, mesh->dev.jacobians, F, records);
   PRT_CHECK_CUDA(cudaGetLastError());
   const bool share = n < SHARE_PARTICLES;
   const long long per = share ? 32 : CHUNK_N;

@@ -15,8 +15,8 @@
 //   1. set-up (host, once per mesh): merge coincident nodes into positions,
 //      order them along a Morton curve, cut them by recursive bisection into
 //      tiles of 32 in blocks of four (the FP64 sums' targets, tiles.cuh), and
-//      cut the Morton order into position groups (<= 32, and wide ones <= 64
-//      for mixed_simt) with bounding spheres;
+//      cut the Morton order into groups (<= 64, for mixed_simt) with bounding
+//      spheres;
 //   2. per call: bin the particles (bin width radius/2), radix sort by bin,
 //      pack a 64-byte payload per particle in bin order; estimate each
 //      block's work (the particles of its bin rows) and launch the blocks
@@ -674,36 +674,43 @@ __global__ void expand_kernel(long long nn, long long npos,
 
 // Integration weight of a position: sum over its nodes of w_i |J_e| (the
 // normalising depositor's sum_e |J_e| sum_i w_i S_i, dep_normshape.hpp:155-164,
-// regrouped by position), in ascending node order.
+// regrouped by position); RUN_LANES neighbouring lanes share a position.
+__device__ __forceinline__ double position_weight(const NodeWeights &N, const uint32_t *run_starts,
+                                                  const uint32_t *run_nodes, int np,
+                                                  const double *jac, uint32_t u, bool in) {
+  __shared__ double shared[PRT_NODE_WEIGHTS];
+  const double *iw = stage_node_weights(N, np, shared);
+  double s = 0;
+  if (in)
+    for (uint32_t k = run_starts[u] + threadIdx.x % RUN_LANES; k < run_starts[u + 1];
+         k += RUN_LANES) {
+      const uint32_t node = run_nodes[k];
+      s += iw[node % np] * jac[node / np];
+    }
+  return sum_run(s);
+}
+
 __global__ void position_weights_kernel(long long npos, const uint32_t *__restrict__ run_starts,
                                         const uint32_t *__restrict__ run_nodes, int np,
-                                        const double *__restrict__ iw,
+                                        const __grid_constant__ NodeWeights N,
                                         const double *__restrict__ jac,
                                         double *__restrict__ W) {
-  long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (u >= npos) return;
-  double s = 0;
-  for (uint32_t k = run_starts[u]; k < run_starts[u + 1]; ++k) {
-    const uint32_t node = run_nodes[k];
-    s += iw[node % np] * jac[node / np];
-  }
-  W[u] = s;
+  const long long u = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / RUN_LANES;
+  const double s = position_weight(N, run_starts, run_nodes, np, jac, (uint32_t)u, u < npos);
+  if (u < npos && threadIdx.x % RUN_LANES == 0) W[u] = s;
 }
 
 // The same per tile row, as the normalising pass's sources: (x, y, z, W).
 __global__ void weight_records_kernel(TilesDev T, const uint32_t *__restrict__ run_starts,
                                       const uint32_t *__restrict__ run_nodes, int np,
-                                      const double *__restrict__ iw,
+                                      const __grid_constant__ NodeWeights N,
                                       const double *__restrict__ jac,
                                       double2 *__restrict__ records) {
-  const long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (r >= T.count) return;
-  const uint32_t u = T.rows[r];
-  double s = 0;
-  for (uint32_t k = run_starts[u]; k < run_starts[u + 1]; ++k) {
-    const uint32_t node = run_nodes[k];
-    s += iw[node % np] * jac[node / np];
-  }
+  const long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / RUN_LANES;
+  const bool in = r < T.count;
+  const double s =
+      position_weight(N, run_starts, run_nodes, np, jac, in ? T.rows[r] : 0u, in);
+  if (!in || threadIdx.x % RUN_LANES != 0) return;
   records[2 * r] = make_double2(T.pos[3 * r], T.pos[3 * r + 1]);
   records[2 * r + 1] = make_double2(T.pos[3 * r + 2], s);
 }
@@ -1143,16 +1150,29 @@ int prt_mesh_build_positions(prt_mesh *m, const prt_mesh_desc *d) {
 
 // ------------------------------------------- pieces shared with deposit_tc.cu
 
+int prt_node_weights(const double *iw, int np, double *scratch, NodeWeights *out, cudaStream_t s) {
+  std::memset(out, 0, sizeof(*out));
+  if (np <= PRT_NODE_WEIGHTS) {
+    std::memcpy(out->w, iw, sizeof(double) * (size_t)np);
+    return PRT_OK;
+  }
+  PRT_CHECK_CUDA(
+      cudaMemcpyAsync(scratch, iw, sizeof(double) * (size_t)np, cudaMemcpyHostToDevice, s));
+  out->more = scratch;
+  return PRT_OK;
+}
+
 int prt_dep_position_weights(const prt_mesh *mesh, prt_workspace *ws, const double *iw,
                              double *W, cudaStream_t s) {
   int rc;
   double *iwd = (double *)ws_buffer(ws, PRT_WS_DEP_STATS,
                                     sizeof(double) * (64 + mesh->dev.Np + 10 * STATS_BLOCKS), &rc);
   if (!iwd) return rc;
-  PRT_CHECK_CUDA(cudaMemcpyAsync(iwd, iw, sizeof(double) * mesh->dev.Np, cudaMemcpyHostToDevice, s));
+  NodeWeights N;
+  if ((rc = prt_node_weights(iw, mesh->dev.Np, iwd, &N, s))) return rc;
   const PositionSet &PS = mesh->positions;
-  position_weights_kernel<<<prt_grid_blocks(PS.count, 256), 256, 0, s>>>(
-      PS.count, PS.run_starts, PS.run_nodes, mesh->dev.Np, iwd, mesh->dev.jacobians, W);
+  position_weights_kernel<<<prt_grid_blocks(RUN_LANES * PS.count, 256), 256, 0, s>>>(
+      PS.count, PS.run_starts, PS.run_nodes, mesh->dev.Np, N, mesh->dev.jacobians, W);
   PRT_CHECK_CUDA(cudaGetLastError());
   return PRT_OK;
 }
@@ -1252,11 +1272,11 @@ extern "C" int prt_deposit_shape(const prt_mesh *mesh, prt_workspace *ws, int32_
     if (!aux) return rc;
     double *iwd = aux + 16, *partials = aux + 64 + mesh->dev.Np;
     double2 *records = (double2 *)(aux + head);
-    PRT_CHECK_CUDA(cudaMemcpyAsync(iwd, iw, sizeof(double) * mesh->dev.Np,
-                                   cudaMemcpyHostToDevice, s));
+    NodeWeights N;
+    if ((rc = prt_node_weights(iw, mesh->dev.Np, iwd, &N, s))) return rc;
     const TilesDev T = tiles_dev(PS.tiles);
-    weight_records_kernel<<<prt_grid_blocks(PS.count, 256), 256, 0, s>>>(
-        T, PS.run_starts, PS.run_nodes, mesh->dev.Np, iwd, mesh->dev.jacobians, records);
+    weight_records_kernel<<<prt_grid_blocks(RUN_LANES * PS.count, 256), 256, 0, s>>>(
+        T, PS.run_starts, PS.run_nodes, mesh->dev.Np, N, mesh->dev.jacobians, records);
     PRT_CHECK_CUDA(cudaGetLastError());
     {
       ScopedTimer norm_timer(ws, PRT_TIME_DEPOSIT_NORMALIZE, s);

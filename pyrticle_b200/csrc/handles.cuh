@@ -150,6 +150,17 @@ constexpr double PRT_GROUP_TARGET = 24.0;
 void *ws_buffer(prt_workspace *ws, int slot, size_t bytes, int *rc);
 int prt_mesh_build_positions(prt_mesh *m, const prt_mesh_desc *d);
 
+// The integration weights of an element's nodes as a kernel argument: no copy
+// of a few bytes from pageable host memory before the launch. Larger elements'
+// weights (`more`; 64 doubles reach order 5) are copied.
+constexpr int PRT_NODE_WEIGHTS = 64;
+struct NodeWeights {
+  double w[PRT_NODE_WEIGHTS];
+  const double *more;  // np > PRT_NODE_WEIGHTS: in device memory
+};
+// `scratch`: device memory for np weights, read only where np is too large
+int prt_node_weights(const double *iw, int np, double *scratch, NodeWeights *out, cudaStream_t s);
+
 // Shared pieces of the shape deposition (deposit.cu) used by the
 // tensor-core form (deposit_tc.cu).
 // W[u] = sum over the nodes at position u of w_i |J_e| (device; iw a HOST [Np]).
