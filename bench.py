@@ -641,7 +641,7 @@ def grid_bench(args, torch):
             "speedup_mixed_vs_fp64": ms64 / ms,
             "fp64": {"value": n * args.steps / (ms64 * 1e-3), "ms_per_step": ms64 / args.steps,
                      "kernel_ms_per_step": k64,
-                     "roofline": {"bound": "fp64", "kernel": "deposit_grid_kernel (FP64)",
+                     "roofline": {"bound": "fp64", "kernel": "deposit_blocks_kernel over the brick points (FP64)",
                                   "achieved": achieved64, "peak": fp64, "unit": "TFLOP/s",
                                   "frac": achieved64 / fp64, "traffic": None,
                                   "peak_source": "cuBLAS DGEMM 8192^3 measured in this run",
