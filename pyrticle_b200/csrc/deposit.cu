@@ -494,8 +494,8 @@ __global__ void __launch_bounds__(32 * BW, 3)
     }
     X.c[d] = 0.5 * (lo + hi);
     X.h[d] = 0.5 * (hi - lo) + 1e-5 * S.radius;
-    X.mid[d] = have ? (float)(T.boxes[6 * t + d] - X.c[d]) : 0;
-    X.hf[d] = have ? (float)(T.boxes[6 * t + 3 + d] + 1e-5 * S.radius) : -1e30f;
+    X.mid[d] = have ? (float)((T.boxes[6 * t + d] - X.c[d]) * S.inv_radius) : 0;
+    X.hf[d] = have ? near_half(T.boxes[6 * t + 3 + d], X.h[d], S.inv_radius) : -1e30f;
   }
   stage_begin(stage);
   DepositTargets<PER, ALPHA2, COUNT> D;

@@ -124,11 +124,17 @@ __device__ __forceinline__ void reduce_groups(double (&v)[N][PER]) {
   }
 }
 
-// 4 radius^2 for the choice of entries near a box, with a margin above FP32
-// rounding (the choice only decides what is evaluated).
-__device__ __forceinline__ float near_limit(double radius) {
-  const float r = (float)(radius * (1 + 1e-5));
-  return 4.0f * r * r;
+// The choice of entries near a warp's box runs in FP32 on coordinates relative
+// to the block's centre in units of the radius; it only decides what is
+// evaluated. NEAR_LIMIT is (2 radius)^2 with a margin for the rounding of what
+// is of the order of the radius. The rounding of the entry, of the box's
+// centre and half extent and of their differences grows with the block's half
+// extent H instead: at most 2^-24 (5 H + 2) together, which near_half adds to
+// the box. (Without the second part, pairs close to the radius were left out
+// from some 150 radii on.)
+constexpr float NEAR_LIMIT = 4.0f * (1 + 1e-5f) * (1 + 1e-5f);
+__device__ __forceinline__ float near_half(double half, double block_half, double inv_radius) {
+  return (float)((half + 4e-7 * block_half) * inv_radius + 1e-5);
 }
 
 // ------------------------------------------------ four tiles per block
@@ -144,7 +150,7 @@ template <int NV>
 struct BlockStage {
   static constexpr int W = 2 + (NV + 1) / 2, RAW = (3 + NV + 1) / 2, STAGES = 3;
   double2 e[STAGES][W][CHUNK_N + 1];
-  float4 w[STAGES][CHUNK_N];  // the entries' positions, for the choice
+  float4 w[STAGES][CHUNK_N];  // the entries' positions over the radius, for the choice
   uint32_t cum[CHUNK_N + 1];  // sources before the segment
   uint32_t start[CHUNK_N];    // its first record
   double shift[CHUNK_N][3];   // from a record's position to the block's frame
@@ -195,15 +201,16 @@ __device__ __forceinline__ void stage_begin(BlockStage<NV> &S) {
 // Evaluates the `total` sources of the present segments (S.cum, S.start,
 // S.shift; written before a barrier) against the block's tiles:
 // op(w0, w1, w2, e, v) on every lane with its group's entry. mid, hf: this
-// warp's tile box in the block's frame, grown by the FP32 margin; a warp
-// without a tile passes hf < 0 with a magnitude that keeps everything out.
+// warp's tile box in the block's frame in units of the radius, grown by the
+// FP32 margin (near_half); a warp without a tile passes hf < 0 with a magnitude
+// that keeps everything out.
 // SHARE: the warps have the same tile and take 32 of a chunk's entries each.
 // Returns the entries evaluated (per warp). Ends with a barrier.
 template <int PER, int NV, bool SHARE, class Op>
 __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV> &S,
                                                       const double2 *__restrict__ records,
                                                       uint32_t total, const float mid[3],
-                                                      const float hf[3], float rc4,
+                                                      const float hf[3],
                                                       double inv_radius, Op &&op) {
   using ST = BlockStage<NV>;
   constexpr int LANES = 32 / PER;
@@ -252,7 +259,8 @@ __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV> &S,
       }
       const double w0 = v[0] + S.shift[seg0][0], w1 = v[1] + S.shift[seg0][1],
                    w2 = v[2] + S.shift[seg0][2];
-      S.w[st][tid] = make_float4((float)w0, (float)w1, (float)w2, 0);
+      S.w[st][tid] = make_float4((float)(w0 * inv_radius), (float)(w1 * inv_radius),
+                                 (float)(w2 * inv_radius), 0);
       S.e[st][0][tid] = make_double2(w0, w1);
       S.e[st][1][tid] = make_double2(w2, -(w0 * w0 + w1 * w1 + w2 * w2) * inv_radius);
 #pragma unroll
@@ -275,7 +283,7 @@ __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV> &S,
       const float d0 = fabsf(w.x - mid[0]) - hf[0], d1 = fabsf(w.y - mid[1]) - hf[1],
                   d2 = fabsf(w.z - mid[2]) - hf[2];
       const float e0 = d0 + fabsf(d0), e1 = d1 + fabsf(d1), e2 = d2 + fabsf(d2);
-      const bool in = e0 * e0 + e1 * e1 + e2 * e2 <= rc4;
+      const bool in = e0 * e0 + e1 * e1 + e2 * e2 <= NEAR_LIMIT;
       const unsigned bal = __ballot_sync(0xffffffffu, in);
       if (in) list[n + __popc(bal & ((1u << lane) - 1u))] = (uint8_t)(32 * q + lane);
       n += __popc(bal);
@@ -307,7 +315,8 @@ __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV> &S,
 }
 
 // The boxes of a block's tiles: the block's centre c and half extents, and
-// this warp's tile box in the block's frame (mid, hf with the FP32 margin).
+// this warp's tile box in the block's frame over the radius (mid, hf with the
+// FP32 margin).
 struct BlockBox {
   double c[3], h[3];
   float mid[3], hf[3];
@@ -322,7 +331,6 @@ __device__ __forceinline__ uint32_t evaluate_particles(BlockStage<NV> &S, const 
                                                        Op &&op) {
   const int tid = threadIdx.x;
   const double rr = radius * (1 + 1e-5), rr2 = rr * rr;
-  const float rc4 = near_limit(radius);
   int ulo[3], uhi[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -403,7 +411,7 @@ __device__ __forceinline__ uint32_t evaluate_particles(BlockStage<NV> &S, const 
     if (tid == 0) S.cum[CHUNK_N] = total;
     __syncthreads();
     evaluated += evaluate_segments<PER, NV, SHARE>(
-        S, reinterpret_cast<const double2 *>(P.payload), total, X.mid, X.hf, rc4, inv_radius, op);
+        S, reinterpret_cast<const double2 *>(P.payload), total, X.mid, X.hf, inv_radius, op);
   }
   return evaluated;
 }
@@ -444,7 +452,6 @@ __device__ __forceinline__ void evaluate_positions(BlockStage<NV> &S, TileRows &
                                                    double radius, double inv_radius, Op &&op) {
   const int tid = threadIdx.x;
   const double rr = radius * (1 + 1e-5), rr2 = rr * rr;
-  const float rc4 = near_limit(radius);
   int lo_img[3], hi_img[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -515,7 +522,7 @@ __device__ __forceinline__ void evaluate_positions(BlockStage<NV> &S, TileRows &
             for (int d = 0; d < 3; ++d) S.shift[tid][d] = -c[d];
             if (tid == 0) S.cum[CHUNK_N] = total;
             __syncthreads();
-            evaluate_segments<PER, NV, SHARE>(S, records, total, X.mid, X.hf, rc4, inv_radius, op);
+            evaluate_segments<PER, NV, SHARE>(S, records, total, X.mid, X.hf, inv_radius, op);
           }
           __syncthreads();
         }
@@ -587,8 +594,8 @@ __device__ __forceinline__ bool load_particles(ParticleTargets<PER> &D, BlockBox
     X.c[d] = any ? 0.5 * (bl + bh) : 0;
     X.h[d] = any ? 0.5 * (bh - bl) + 1e-5 * S.radius : 0;
     const bool have = lo[d] <= hi[d];
-    X.mid[d] = have ? (float)(0.5 * (lo[d] + hi[d]) - X.c[d]) : 0;
-    X.hf[d] = have ? (float)(0.5 * (hi[d] - lo[d]) + 1e-5 * S.radius) : -1e30f;
+    X.mid[d] = have ? (float)((0.5 * (lo[d] + hi[d]) - X.c[d]) * S.inv_radius) : 0;
+    X.hf[d] = have ? near_half(0.5 * (hi[d] - lo[d]), X.h[d], S.inv_radius) : -1e30f;
   }
 #pragma unroll
   for (int h = 0; h < PER; ++h) {

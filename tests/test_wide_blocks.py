@@ -1,0 +1,103 @@
+"""The FP64 pair sums where the points of a block lie thousands of shape radii
+apart (few particles in a long beam line, a mesh that is coarse against the
+radius): a particle near every node of a thin box 5,000 radii long, whose nodes
+are several radii apart, so that every particle has exactly one position within
+the radius."""
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from pyrticle_b200 import _lib, meshgen  # noqa: E402
+from pyrticle_b200.cloud import PicMethod  # noqa: E402
+from pyrticle_b200.deposition.shape import NormalizedShapeFunctionDepositor  # noqa: E402
+from pyrticle_b200.discretization import Discretization  # noqa: E402
+from pyrticle_b200.pusher import MonomialParticlePusher  # noqa: E402
+from pyrticle_b200.tools import PolynomialShapeFunction  # noqa: E402
+from pyrticle_b200.units import SIUnitsWithNaturalConstants as U  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+
+F64 = torch.float64
+RADIUS = 9.9998e-6
+BOX = (1e-4, 1.2e-4, 0.47)
+
+
+def setup(n, lo, hi, alpha=2, seed=0):
+    """The method, and n particles at lo to hi radii from nodes of their own:
+    positions x [3, n]. Displaced along the box, so that those at the ends of
+    a block are out of its box by just that."""
+    mesh = meshgen.box_mesh((1, 1, 64), (0, 0, 0), BOX, seed=7)
+    m = PicMethod(Discretization(mesh, 2), U, NormalizedShapeFunctionDepositor(),
+                  MonomialParticlePusher(), 3, 3)
+    m.depositor.set_shape_function(None, PolynomialShapeFunction(RADIUS, 3, alpha))
+    nodes = np.ascontiguousarray(m.discretization.nodes)
+    _, first = np.unique(np.round(nodes / 1e-9).astype(np.int64), axis=0, return_index=True)
+    rng = np.random.default_rng(seed)
+    pick = np.sort(rng.permutation(first)[:n])
+    away = np.zeros((len(pick), 3))
+    away[:, 2] = rng.uniform(lo, hi, len(pick)) * RADIUS * rng.choice([-1, 1], len(pick))
+    x = torch.as_tensor((nodes[pick] + away).T.copy(), device="cuda")
+    return m, torch.as_tensor(nodes, device="cuda"), x
+
+
+def pairs(m, nodes, x):
+    """x_u - x_p and r^2 of all (node, particle) pairs, by differences."""
+    d = nodes.T[:, :, None] - x[:, None, :]
+    return d, (d * d).sum(0)
+
+
+def deposit(m, mode, x, q, stats=None):
+    rho = torch.empty((len(m.discretization),), dtype=F64, device="cuda")
+    _lib.check(m.lib.prt_deposit_shape(
+        m.mesh_data.handle, m.workspace, mode, m.depositor._shape_desc(),
+        _lib.ptr(m.depositor.integral_weights), x.shape[1], x.data_ptr(), q.data_ptr(), None,
+        None, rho.data_ptr(), None, 0, C.byref(stats) if stats else None, C.c_void_p(0)))
+    m.check_status()
+    return rho
+
+
+def test_deposited_pairs_near_the_rim_count():
+    """At 0.99999 to 0.999999 radii a - r^2/a is at least 2e-6 a, beyond the
+    rounding of the form (H^2 2^-53 a = 1e-9 a for a block of half extent H =
+    2,700 radii), which is 2 x 1e-9 / 2e-6 of the weight."""
+    m, nodes, x = setup(10_000, 0.99999, 0.999999)
+    q = torch.ones(x.shape[1], dtype=F64, device="cuda")
+    _, r2 = pairs(m, nodes, x)
+    t = torch.clamp(RADIUS - r2 / RADIUS, min=0)
+    want = m.depositor.shape_function.normalizer * (t * t).sum(1)
+    assert bool((want > 0).all())
+    rho = deposit(m, _lib.DEPOSIT_PLAIN, x, q)
+    assert float(((rho - want) / want).abs().max()) <= 1e-2
+
+
+def average(m, x, fields, ordered):
+    """The forces on unit charges at rest, [3, n]."""
+    n = x.shape[1]
+    q = torch.ones(n, dtype=F64, device="cuda")
+    v = torch.zeros_like(x)
+    out = torch.full_like(x, 7.0)
+    ptrs = (C.c_void_p * 6)(*[fields[k].data_ptr() for k in range(6)])
+    _lib.check(m.lib.prt_average_forces_ordered(
+        m.mesh_data.handle, m.workspace, m.depositor._shape_desc(),
+        _lib.ptr(m.depositor.integral_weights), n, x.data_ptr(), q.data_ptr(), v.data_ptr(), None,
+        ptrs, out.data_ptr(), None, None, ordered, C.c_void_p(0)))
+    return out
+
+
+def test_averaged_pairs_near_the_rim_count():
+    """32 particles at each of 600 nodes, a warp's worth, in a store without a
+    spatial order that is taken in its own: blocks as long as the box. With one
+    position within the radius the average is the field there."""
+    m, nodes, x = setup(600, 0.99999, 0.999999)
+    perm = torch.as_tensor(np.random.default_rng(5).permutation(600), device="cuda")
+    x = x[:, perm].repeat_interleave(32, 1).contiguous()
+    # E_x = 1 at every node: no position left out, whatever its weight's rounding
+    fields = torch.zeros((6, len(nodes)), dtype=F64, device="cuda")
+    fields[0] = 1
+    out = average(m, x, fields, 1)
+    assert float((out[0] - 1).abs().max()) <= 1e-14
+    assert bool((out[1:] == 0).all())
