@@ -545,7 +545,7 @@ __global__ void contract_kernel(prt_dep::TilesDev T, long long nn,
 //   dL/dx_p = w sum_u (G0_u + G_u . v_p) dS/dx_p,
 //   dL/dv_p = w sum_u G_u S,   dS/dx_p = alpha (a - r^2/a)^(alpha-1) (2/a) (x_u - x_p),
 // with the particles as targets, in bin order, and the positions as sources
-// (tiles.cuh): 18 FP64 operations per evaluated pair.
+// (tiles.cuh): 17 FP64 operations per evaluated pair.
 constexpr int DEP_ADJ_PER = 4;
 template <bool ALPHA2, bool SHARE>
 __global__ void __launch_bounds__(32 * prt_dep::BW, 3)
@@ -557,7 +557,7 @@ __global__ void __launch_bounds__(32 * prt_dep::BW, 3)
                            double *__restrict__ lx, double *__restrict__ lv) {
   using namespace prt_dep;
   constexpr int PER = DEP_ADJ_PER, LANES = 32 / PER;
-  __shared__ BlockStage<4> stage;
+  __shared__ BlockStage<4, true> stage;
   __shared__ TileRows rows;
   __shared__ double boxes[BW][6];
   BlockBox X;
@@ -572,28 +572,29 @@ __global__ void __launch_bounds__(32 * prt_dep::BW, 3)
 #pragma unroll
     for (int k = 0; k < 6; ++k) acc[k][h] = 0;
   }
-  const double mha = -0.5 * S.radius;  // x_u - x_p = w + V (-a/2), V = 2 (x_p - c) / a
+  const double radius2 = S.radius * S.radius;
   evaluate_positions<PER, 4, SHARE>(
       stage, rows, T, B, records, M, X, S.radius, S.inv_radius,
-      [&](double w0, double w1, double w2, double e, const double *g) {
+      [&](double w0, double w1, double w2, const double *g) {
 #pragma unroll
         for (int h = 0; h < PER; ++h) {
-          const double tr =
-              fma(D.V[0][h], w0, fma(D.V[1][h], w1, fma(D.V[2][h], w2, D.B[h] + e)));
-          // pm = t^(alpha - 1), sv = t^alpha for t > 0
+          const double d0 = w0 - D.p[0][h], d1 = w1 - D.p[1][h], d2 = w2 - D.p[2][h];
+          const double t = inside(radius2, d0, d1, d2);
+          // pm = t^(alpha - 1), sv = t^alpha for t > 0 (ALPHA2: by a and a^2 more)
           double pm, sv;
           if (ALPHA2) {
-            pm = tr > 0 ? tr : 0.0;
+            pm = t > 0 ? t : 0.0;
             sv = pm * pm;
           } else {
-            pm = tr > 0 ? pow(tr, S.alpha - 1.0) : 0.0;
-            sv = pm * tr;
+            const double ta = t * S.inv_radius;
+            pm = t > 0 ? pow(ta, S.alpha - 1.0) : 0.0;
+            sv = pm * ta;
           }
           const double hd =
               pm * fma(g[2], vv[1][h], fma(g[1], vv[0][h], fma(g[3], vv[2][h], g[0])));
-          acc[0][h] = fma(hd, fma(D.V[0][h], mha, w0), acc[0][h]);
-          acc[1][h] = fma(hd, fma(D.V[1][h], mha, w1), acc[1][h]);
-          acc[2][h] = fma(hd, fma(D.V[2][h], mha, w2), acc[2][h]);
+          acc[0][h] = fma(hd, d0, acc[0][h]);
+          acc[1][h] = fma(hd, d1, acc[1][h]);
+          acc[2][h] = fma(hd, d2, acc[2][h]);
           acc[3][h] = fma(g[1], sv, acc[3][h]);
           acc[4][h] = fma(g[2], sv, acc[4][h]);
           acc[5][h] = fma(g[3], sv, acc[5][h]);
@@ -609,11 +610,12 @@ __global__ void __launch_bounds__(32 * prt_dep::BW, 3)
   for (int h = 0; h < PER; ++h) {
     if (h != grp || !D.live[h]) continue;
     const long long i = D.id[h];
-    const double w = q[i] * normalizer, wx = w * S.alpha * (2.0 * S.inv_radius);
+    const double w = q[i] * normalizer, wv = w * direct_scale<ALPHA2>(S);
+    const double wx = w * S.alpha * (2.0 * S.inv_radius) * (ALPHA2 ? S.inv_radius : 1.0);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       lx[d * n + i] += wx * acc[d][0];
-      if (lv) lv[d * n + i] += w * acc[3 + d][0];
+      if (lv) lv[d * n + i] += wv * acc[3 + d][0];
     }
   }
 }

@@ -33,7 +33,7 @@ __global__ void average_records_kernel(TilesDev T, int np, const uint32_t *__res
                                        const __grid_constant__ NodeWeights N,
                                        const double *__restrict__ jac, Fields6 F,
                                        double2 *__restrict__ records) {
-  constexpr int NV = AVG_NV<SQUARES>, RAW = BlockStage<NV>::RAW;
+  constexpr int NV = AVG_NV<SQUARES>, RAW = BlockStage<NV, true>::RAW;
   __shared__ double shared[PRT_NODE_WEIGHTS];
   const double *iw = stage_node_weights(N, np, shared);
   const long long r = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / RUN_LANES;
@@ -69,7 +69,7 @@ __global__ void average_records_kernel(TilesDev T, int np, const uint32_t *__res
 
 template <bool SQUARES>
 struct AverageShared {
-  BlockStage<AVG_NV<SQUARES>> stage;
+  BlockStage<AVG_NV<SQUARES>, true> stage;
   TileRows rows;
   double boxes[BW][6];
 };
@@ -98,14 +98,14 @@ __global__ void __launch_bounds__(32 * BW, 3)
   for (int k = 0; k < NV; ++k)
 #pragma unroll
     for (int h = 0; h < PER; ++h) sum[k][h] = 0;
+  const double radius2 = S.radius * S.radius;
   evaluate_positions<PER, NV, SHARE>(
       A.stage, A.rows, T, B, records, M, X, S.radius, S.inv_radius,
-      [&](double w0, double w1, double w2, double e, const double *g) {
+      [&](double w0, double w1, double w2, const double *g) {
 #pragma unroll
         for (int h = 0; h < PER; ++h) {
-          const double tr =
-              fma(D.V[0][h], w0, fma(D.V[1][h], w1, fma(D.V[2][h], w2, D.B[h] + e)));
-          const double sw = shape_power<ALPHA2>(tr, S.alpha);
+          const double sw = direct_power<ALPHA2>(
+              inside(radius2, w0 - D.p[0][h], w1 - D.p[1][h], w2 - D.p[2][h]), S);
 #pragma unroll
           for (int k = 0; k < NV; ++k) sum[k][h] = fma(sw, g[k], sum[k][h]);
         }
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(32 * BW, 3)
   if (i < 0) return;
   double acc[NV];
 #pragma unroll
-  for (int k = 0; k < NV; ++k) acc[k] = normalizer * sum[k][0];
+  for (int k = 0; k < NV; ++k) acc[k] = normalizer * direct_scale<ALPHA2>(S) * sum[k][0];
   const double charge = q[i];
   double f[3] = {0, 0, 0}, ef[6] = {0, 0, 0, 0, 0, 0}, sde = 0, sdb = 0;
   const double den = charge * acc[0];  // the reconstructed charge
@@ -221,7 +221,7 @@ int average_forces(const prt_mesh *mesh, prt_workspace *ws, const prt_shape_func
   const PositionSet &PS = mesh->positions;
   const int np = mesh->dev.Np;
   int rc;
-  const size_t rec = BlockStage<NV>::RAW * (size_t)PS.count;
+  const size_t rec = BlockStage<NV, true>::RAW * (size_t)PS.count;
   double2 *records =
       (double2 *)ws_buffer(ws, PRT_WS_AVERAGE, sizeof(double2) * rec + sizeof(double) * np, &rc);
   if (!records) return rc;

@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(32 * BW, 3)
                           unsigned long long *__restrict__ counters,
                           const uint32_t *__restrict__ order) {
   constexpr int PER = BLOCK_PER, LANES = 32 / PER;
-  __shared__ BlockStage<4> stage;
+  __shared__ BlockStage<4, false> stage;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int tg = lane % LANES, grp = lane / LANES;
   const long long blk = order ? (long long)order[blockIdx.x] : (long long)blockIdx.x;
@@ -724,8 +724,8 @@ __global__ void weight_records_kernel(TilesDev T, const uint32_t *__restrict__ r
 // positions within the radius; scale = q / integral, or 0 with a warning for
 // a zero integral (the reference skips such a particle). Targets are 32
 // particles per warp in bin order (close together whatever the store's order),
-// sources the positions of the tiles near them (tiles.cuh): six FP64
-// operations per evaluated pair. hits_out: the positions within the radius
+// sources the positions of the tiles near them (tiles.cuh): eight
+// FP64 operations per evaluated pair. hits_out: the positions within the radius
 // (-1 for a dead particle).
 constexpr int NORM_PER = 4;  // (8: 10% slower at 1M particles, spills)
 template <bool ALPHA2, bool SHARE>
@@ -737,7 +737,7 @@ __global__ void __launch_bounds__(32 * BW, 3)
                      double *__restrict__ scale_out, double *__restrict__ hits_out,
                      DevStatus *st) {
   constexpr int PER = NORM_PER, LANES = 32 / PER;
-  __shared__ BlockStage<1> stage;
+  __shared__ BlockStage<1, true> stage;
   __shared__ TileRows rows;
   __shared__ double boxes[BW][6];
   const int lane = threadIdx.x & 31;
@@ -752,16 +752,16 @@ __global__ void __launch_bounds__(32 * BW, 3)
     sum[0][h] = 0;
     hits[h] = 0;
   }
+  const double radius2 = S.radius * S.radius;
   if (any)
     evaluate_positions<PER, 1, SHARE>(
         stage, rows, T, B, records, M, X, S.radius, S.inv_radius,
-        [&](double w0, double w1, double w2, double e, const double *v) {
+        [&](double w0, double w1, double w2, const double *v) {
 #pragma unroll
           for (int h = 0; h < PER; ++h) {
-            const double tr =
-                fma(D.V[0][h], w0, fma(D.V[1][h], w1, fma(D.V[2][h], w2, D.B[h] + e)));
-            sum[0][h] = fma(shape_power<ALPHA2>(tr, S.alpha), v[0], sum[0][h]);
-            hits[h] += __double2hiint(tr) >= 0;
+            const double t = inside(radius2, w0 - D.p[0][h], w1 - D.p[1][h], w2 - D.p[2][h]);
+            sum[0][h] = fma(direct_power<ALPHA2>(t, S), v[0], sum[0][h]);
+            hits[h] += __double2hiint(t) >= 0;
           }
         });
 #pragma unroll
@@ -782,7 +782,7 @@ __global__ void __launch_bounds__(32 * BW, 3)
       hits_out[i] = -1;
       continue;
     }
-    const double integral = normalizer * sum[0][0];
+    const double integral = normalizer * direct_scale<ALPHA2>(S) * sum[0][0];
     if (integral == 0) {
       scale_out[i] = 0;
       record_warning(st, PRT_WARN_ZERO_MASS, i);

@@ -11,9 +11,18 @@
 // then picks the chunk's entries near its own tile (a ballot per 32, an index
 // list) and evaluates those.
 //
-// With u the target and w the source relative to the block's centre,
+// Positions as targets (the depositions): with u the target and w the source
+// relative to the block's centre,
 //   a - r^2/a = (a - |u|^2/a) - |w|^2/a + (2/a) u.w = B + e + V.w,
-// three multiply-adds and an add per pair.
+// three multiply-adds and an add per pair. Its rounding error grows with the
+// square of the block's half extent H, about (H/a)^2 2^-53 a; a mesh's tiles
+// are compact. Particles as targets (DIRECT) may lie far apart in a block (few
+// particles in a long beam line), so these sums take the differences,
+//   a^2 - r^2 = a^2 - |w - u|^2,
+// three subtractions and three multiply-adds, and the powers of 1/a at the end:
+// the error is a few 2^-53 a^2 whatever the block. (By the expansion, 3,000
+// particles 30 radii apart on average had a deposition adjoint with a median
+// relative error of 3.5e-12, by differences 1.2e-13.)
 //
 // Lane layout: PER targets per lane, so 32/PER lanes cover the tile and PER
 // groups of lanes take different sources at the same time. One source per
@@ -94,6 +103,11 @@ int launch_deposit_tiles(prt_workspace *ws, const TileSet &T, const uint32_t *ru
                          const BinGrid &G, const DepParticles &P, const ShapeParams &S,
                          double *const out[4], unsigned long long *counters, cudaStream_t s);
 
+// a^2 - |d|^2.
+__device__ __forceinline__ double inside(double radius2, double d0, double d1, double d2) {
+  return fma(-d0, d0, fma(-d1, d1, fma(-d2, d2, radius2)));
+}
+
 // The weight (t)^alpha for t > 0, else 0.
 template <bool ALPHA2>
 __device__ __forceinline__ double shape_power(double t, double alpha) {
@@ -102,6 +116,17 @@ __device__ __forceinline__ double shape_power(double t, double alpha) {
     return r * r;
   }
   return t > 0 ? pow(t, alpha) : 0.0;
+}
+
+// The same from t = a^2 - r^2, up to a factor direct_scale: (t / a)^alpha.
+template <bool ALPHA2>
+__device__ __forceinline__ double direct_power(double t, const ShapeWeight &S) {
+  if (ALPHA2) return shape_power<true>(t, 2);
+  return t > 0 ? pow(t * S.inv_radius, S.alpha) : 0.0;
+}
+template <bool ALPHA2>
+__device__ __forceinline__ double direct_scale(const ShapeWeight &S) {
+  return ALPHA2 ? S.inv_radius * S.inv_radius : 1.0;
 }
 
 // Adds the lanes' partial sums of the groups: v[N][PER] per lane (PER targets,
@@ -145,15 +170,16 @@ constexpr int CHUNK_N = 32 * BW;
 // Staging of one block: three chunks of entries, W 16-byte words each
 // ((w0, w1), (w2, e), values), word by word; entry CHUNK_N lies beyond every
 // radius. A record (x, y, z, values) is copied to the same place and moved
-// into the block's frame there by the thread that copied it.
-template <int NV>
+// into the block's frame there by the thread that copied it. DIRECT: the
+// entries are the records, moved by a whole period at most.
+template <int NV, bool DIRECT>
 struct BlockStage {
-  static constexpr int W = 2 + (NV + 1) / 2, RAW = (3 + NV + 1) / 2, STAGES = 3;
+  static constexpr int RAW = (3 + NV + 1) / 2, W = DIRECT ? RAW : 2 + (NV + 1) / 2, STAGES = 3;
   double2 e[STAGES][W][CHUNK_N + 1];
   float4 w[STAGES][CHUNK_N];  // the entries' positions over the radius, for the choice
   uint32_t cum[CHUNK_N + 1];  // sources before the segment
   uint32_t start[CHUNK_N];    // its first record
-  double shift[CHUNK_N][3];   // from a record's position to the block's frame
+  double shift[DIRECT ? 1 : CHUNK_N][3];  // from a record's position to the block's frame
   uint32_t wsum[BW];
   uint8_t list[BW][CHUNK_N + 32];
 };
@@ -189,30 +215,42 @@ __device__ __forceinline__ void copy16_async(void *dst, const void *src) {
                : "memory");
 }
 
-template <int NV>
-__device__ __forceinline__ void stage_begin(BlockStage<NV> &S) {
-  using ST = BlockStage<NV>;
+// A coordinate beyond every radius of what is in the mesh, whose square and
+// whose distance's square from its opposite are finite.
+constexpr double FAR = 1e150;
+
+template <int NV, bool DIRECT>
+__device__ __forceinline__ void stage_begin(BlockStage<NV, DIRECT> &S) {
+  using ST = BlockStage<NV, DIRECT>;
   if (threadIdx.x < ST::STAGES * ST::W) {
     const int st = threadIdx.x / ST::W, w = threadIdx.x % ST::W;
-    S.e[st][w][CHUNK_N] = make_double2(0, w == 1 ? -1e300 : 0);
+    S.e[st][w][CHUNK_N] = DIRECT ? make_double2(w < 2 ? FAR : 0, w < 1 ? FAR : 0)
+                                 : make_double2(0, w == 1 ? -1e300 : 0);
   }
 }
 
-// Evaluates the `total` sources of the present segments (S.cum, S.start,
-// S.shift; written before a barrier) against the block's tiles:
-// op(w0, w1, w2, e, v) on every lane with its group's entry. mid, hf: this
-// warp's tile box in the block's frame in units of the radius, grown by the
-// FP32 margin (near_half); a warp without a tile passes hf < 0 with a magnitude
+// The boxes of a block's tiles: the block's centre c and half extents, and
+// this warp's tile box in the block's frame over the radius (mid, hf with the
+// FP32 margin, near_half); a warp without a tile has hf < 0 with a magnitude
 // that keeps everything out.
+struct BlockBox {
+  double c[3], h[3];
+  float mid[3], hf[3];
+};
+
+// Evaluates the `total` sources of the present segments (S.cum, S.start and
+// the shifts to the block's frame S.shift, or DIRECT `shift` for all; written
+// before a barrier) against the block's tiles: op(w0, w1, w2, e, v), DIRECT
+// op(x, y, z, v), on every lane with its group's entry.
 // SHARE: the warps have the same tile and take 32 of a chunk's entries each.
 // Returns the entries evaluated (per warp). Ends with a barrier.
-template <int PER, int NV, bool SHARE, class Op>
-__device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV> &S,
+template <int PER, int NV, bool SHARE, bool DIRECT, class Op>
+__device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV, DIRECT> &S,
                                                       const double2 *__restrict__ records,
-                                                      uint32_t total, const float mid[3],
-                                                      const float hf[3],
-                                                      double inv_radius, Op &&op) {
-  using ST = BlockStage<NV>;
+                                                      uint32_t total, const BlockBox &X,
+                                                      const double *shift, double inv_radius,
+                                                      Op &&op) {
+  using ST = BlockStage<NV, DIRECT>;
   constexpr int LANES = 32 / PER;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, grp = lane / LANES;
   uint8_t *list = S.list[wid];
@@ -250,23 +288,33 @@ __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV> &S,
     const int st = k % ST::STAGES;
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     if (k < mine) {
-      double v[2 * ST::RAW];
+      if constexpr (DIRECT) {
+        const double2 t0 = S.e[st][0][tid], t1 = S.e[st][1][tid];
+        const double w0 = t0.x + shift[0], w1 = t0.y + shift[1], w2 = t1.x + shift[2];
+        S.w[st][tid] = make_float4((float)((w0 - X.c[0]) * inv_radius),
+                                   (float)((w1 - X.c[1]) * inv_radius),
+                                   (float)((w2 - X.c[2]) * inv_radius), 0);
+        S.e[st][0][tid] = make_double2(w0, w1);
+        S.e[st][1][tid] = make_double2(w2, t1.y);
+      } else {
+        double v[2 * ST::RAW];
 #pragma unroll
-      for (int w = 0; w < ST::RAW; ++w) {
-        const double2 t = S.e[st][w][tid];
-        v[2 * w] = t.x;
-        v[2 * w + 1] = t.y;
+        for (int w = 0; w < ST::RAW; ++w) {
+          const double2 t = S.e[st][w][tid];
+          v[2 * w] = t.x;
+          v[2 * w + 1] = t.y;
+        }
+        const double w0 = v[0] + S.shift[seg0][0], w1 = v[1] + S.shift[seg0][1],
+                     w2 = v[2] + S.shift[seg0][2];
+        S.w[st][tid] = make_float4((float)(w0 * inv_radius), (float)(w1 * inv_radius),
+                                   (float)(w2 * inv_radius), 0);
+        S.e[st][0][tid] = make_double2(w0, w1);
+        S.e[st][1][tid] = make_double2(w2, -(w0 * w0 + w1 * w1 + w2 * w2) * inv_radius);
+#pragma unroll
+        for (int w = 2; w < ST::W; ++w)
+          S.e[st][w][tid] =
+              make_double2(v[2 * w - 1], 2 * w < 3 + NV ? v[2 * w < 2 * ST::RAW ? 2 * w : 0] : 0.0);
       }
-      const double w0 = v[0] + S.shift[seg0][0], w1 = v[1] + S.shift[seg0][1],
-                   w2 = v[2] + S.shift[seg0][2];
-      S.w[st][tid] = make_float4((float)(w0 * inv_radius), (float)(w1 * inv_radius),
-                                 (float)(w2 * inv_radius), 0);
-      S.e[st][0][tid] = make_double2(w0, w1);
-      S.e[st][1][tid] = make_double2(w2, -(w0 * w0 + w1 * w1 + w2 * w2) * inv_radius);
-#pragma unroll
-      for (int w = 2; w < ST::W; ++w)
-        S.e[st][w][tid] =
-            make_double2(v[2 * w - 1], 2 * w < 3 + NV ? v[2 * w < 2 * ST::RAW ? 2 * w : 0] : 0.0);
     } else {
       S.w[st][tid] = make_float4(1e30f, 0, 0, 0);
     }
@@ -280,8 +328,8 @@ __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV> &S,
     for (int q = 0; q < BW; ++q) {
       if (SHARE && q != wid) continue;
       const float4 w = S.w[st][32 * q + lane];
-      const float d0 = fabsf(w.x - mid[0]) - hf[0], d1 = fabsf(w.y - mid[1]) - hf[1],
-                  d2 = fabsf(w.z - mid[2]) - hf[2];
+      const float d0 = fabsf(w.x - X.mid[0]) - X.hf[0], d1 = fabsf(w.y - X.mid[1]) - X.hf[1],
+                  d2 = fabsf(w.z - X.mid[2]) - X.hf[2];
       const float e0 = d0 + fabsf(d0), e1 = d1 + fabsf(d1), e2 = d2 + fabsf(d2);
       const bool in = e0 * e0 + e1 * e1 + e2 * e2 <= NEAR_LIMIT;
       const unsigned bal = __ballot_sync(0xffffffffu, in);
@@ -297,15 +345,17 @@ __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV> &S,
     for (int i = 0; i < n; i += PER) {
       const int cur = id;
       id = list[i + PER + grp];
-      const double2 w01 = S.e[st][0][cur], w2e = S.e[st][1][cur];
-      double v[2 * (ST::W - 2)];
+      double v[2 * ST::W];
 #pragma unroll
-      for (int w = 2; w < ST::W; ++w) {
+      for (int w = 0; w < ST::W; ++w) {
         const double2 t = S.e[st][w][cur];
-        v[2 * w - 4] = t.x;
-        v[2 * w - 3] = t.y;
+        v[2 * w] = t.x;
+        v[2 * w + 1] = t.y;
       }
-      op(w01.x, w01.y, w2e.x, w2e.y, v);
+      if constexpr (DIRECT)
+        op(v[0], v[1], v[2], v + 3);
+      else
+        op(v[0], v[1], v[2], v[3], v + 4);
     }
     __syncwarp();
   }
@@ -314,18 +364,10 @@ __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV> &S,
   return evaluated;
 }
 
-// The boxes of a block's tiles: the block's centre c and half extents, and
-// this warp's tile box in the block's frame over the radius (mid, hf with the
-// FP32 margin).
-struct BlockBox {
-  double c[3], h[3];
-  float mid[3], hf[3];
-};
-
 // All particles of the bin rows near the block's box, evaluated against its
 // tiles (evaluate_segments).
 template <int PER, int NV, bool SHARE, class Op>
-__device__ __forceinline__ uint32_t evaluate_particles(BlockStage<NV> &S, const BinGrid &G,
+__device__ __forceinline__ uint32_t evaluate_particles(BlockStage<NV, false> &S, const BinGrid &G,
                                                        const DepParticles &P, const BlockBox &X,
                                                        double radius, double inv_radius,
                                                        Op &&op) {
@@ -410,8 +452,8 @@ __device__ __forceinline__ uint32_t evaluate_particles(BlockStage<NV> &S, const 
     for (int d = 0; d < 3; ++d) S.shift[tid][d] = sh[d];
     if (tid == 0) S.cum[CHUNK_N] = total;
     __syncthreads();
-    evaluated += evaluate_segments<PER, NV, SHARE>(
-        S, reinterpret_cast<const double2 *>(P.payload), total, X.mid, X.hf, inv_radius, op);
+    evaluated += evaluate_segments<PER, NV, SHARE, false>(
+        S, reinterpret_cast<const double2 *>(P.payload), total, X, nullptr, inv_radius, op);
   }
   return evaluated;
 }
@@ -445,7 +487,7 @@ struct TileRows {
 // All positions of the tiles near the block's box (periodic images included),
 // evaluated against its targets: `records` in the tiles' row order.
 template <int PER, int NV, bool SHARE, class Op>
-__device__ __forceinline__ void evaluate_positions(BlockStage<NV> &S, TileRows &Q,
+__device__ __forceinline__ void evaluate_positions(BlockStage<NV, true> &S, TileRows &Q,
                                                    const TilesDev &T, const TileBinsDev &B,
                                                    const double2 *__restrict__ records,
                                                    const DevMesh &M, const BlockBox &X,
@@ -464,10 +506,10 @@ __device__ __forceinline__ void evaluate_positions(BlockStage<NV> &S, TileRows &
   for (int iz = lo_img[2]; iz <= hi_img[2]; ++iz)
     for (int iy = lo_img[1]; iy <= hi_img[1]; ++iy)
       for (int ix = lo_img[0]; ix <= hi_img[0]; ++ix) {
-        // the box moved by whole periods
-        const double c[3] = {X.c[0] + ix * (M.pmax[0] - M.pmin[0]),
-                             X.c[1] + iy * (M.pmax[1] - M.pmin[1]),
-                             X.c[2] + iz * (M.pmax[2] - M.pmin[2])};
+        // the box moved by whole periods, or the positions by their opposite
+        const double shift[3] = {-ix * (M.pmax[0] - M.pmin[0]), -iy * (M.pmax[1] - M.pmin[1]),
+                                 -iz * (M.pmax[2] - M.pmin[2])};
+        const double c[3] = {X.c[0] - shift[0], X.c[1] - shift[1], X.c[2] - shift[2]};
         int b0[3], b1[3];
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -518,11 +560,9 @@ __device__ __forceinline__ void evaluate_positions(BlockStage<NV> &S, TileRows &
             if (total == 0) continue;
             S.cum[tid] = at;
             S.start[tid] = TILE * tile;
-#pragma unroll
-            for (int d = 0; d < 3; ++d) S.shift[tid][d] = -c[d];
             if (tid == 0) S.cum[CHUNK_N] = total;
             __syncthreads();
-            evaluate_segments<PER, NV, SHARE>(S, records, total, X.mid, X.hf, inv_radius, op);
+            evaluate_segments<PER, NV, SHARE, true>(S, records, total, X, shift, inv_radius, op);
           }
           __syncthreads();
         }
@@ -537,7 +577,7 @@ template <int PER>
 struct ParticleTargets {
   long long id[PER];  // store index, -1 for none
   bool live[PER];
-  double V[3][PER], B[PER];
+  double p[3][PER];  // absent and removed particles: beyond every radius
 };
 
 template <int PER, bool SHARE>
@@ -550,8 +590,8 @@ __device__ __forceinline__ bool load_particles(ParticleTargets<PER> &D, BlockBox
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int tg = lane % (32 / PER);
   const long long k0 = 32 * (SHARE ? (long long)blockIdx.x : BW * (long long)blockIdx.x + wid);
-  double p[3][PER], lo[3] = {INFINITY, INFINITY, INFINITY},
-                    hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+  double lo[3] = {INFINITY, INFINITY, INFINITY},
+         hi[3] = {-INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
   for (int h = 0; h < PER; ++h) {
     const long long k = k0 + PER * tg + h;
@@ -559,10 +599,10 @@ __device__ __forceinline__ bool load_particles(ParticleTargets<PER> &D, BlockBox
     D.live[h] = D.id[h] >= 0 && !(el && el[D.id[h]] == PRT_INVALID);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      p[d][h] = D.live[h] ? x[d * n + D.id[h]] : 0;
+      D.p[d][h] = D.live[h] ? x[d * n + D.id[h]] : -FAR;
       if (D.live[h]) {
-        lo[d] = fmin(lo[d], p[d][h]);
-        hi[d] = fmax(hi[d], p[d][h]);
+        lo[d] = fmin(lo[d], D.p[d][h]);
+        hi[d] = fmax(hi[d], D.p[d][h]);
       }
     }
   }
@@ -596,19 +636,6 @@ __device__ __forceinline__ bool load_particles(ParticleTargets<PER> &D, BlockBox
     const bool have = lo[d] <= hi[d];
     X.mid[d] = have ? (float)((0.5 * (lo[d] + hi[d]) - X.c[d]) * S.inv_radius) : 0;
     X.hf[d] = have ? near_half(0.5 * (hi[d] - lo[d]), X.h[d], S.inv_radius) : -1e30f;
-  }
-#pragma unroll
-  for (int h = 0; h < PER; ++h) {
-    double u2 = 0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const double u = p[d][h] - X.c[d];
-      u2 = fma(u, u, u2);
-      D.V[d][h] = 2 * u * S.inv_radius;
-    }
-    // absent and removed particles: never within the radius
-    D.B[h] = D.live[h] ? S.radius - u2 * S.inv_radius : -1e300;
-    if (!D.live[h]) D.V[0][h] = D.V[1][h] = D.V[2][h] = 0;
   }
   return any;
 }

@@ -35,7 +35,11 @@ def setup(n, lo, hi, alpha=2, seed=0):
                   MonomialParticlePusher(), 3, 3)
     m.depositor.set_shape_function(None, PolynomialShapeFunction(RADIUS, 3, alpha))
     nodes = np.ascontiguousarray(m.discretization.nodes)
-    _, first = np.unique(np.round(nodes / 1e-9).astype(np.int64), axis=0, return_index=True)
+    # the nodes at one position, an ulp apart (5e-12 radii here), count as the
+    # first of them, as in the library
+    _, first, which = np.unique(np.round(nodes / 1e-9).astype(np.int64), axis=0,
+                                return_index=True, return_inverse=True)
+    nodes = nodes[first][which.ravel()]
     rng = np.random.default_rng(seed)
     pick = np.sort(rng.permutation(first)[:n])
     away = np.zeros((len(pick), 3))
@@ -101,3 +105,64 @@ def test_averaged_pairs_near_the_rim_count():
     out = average(m, x, fields, 1)
     assert float((out[0] - 1).abs().max()) <= 1e-14
     assert bool((out[1:] == 0).all())
+
+
+@pytest.mark.parametrize("alpha", [2, 3])
+@pytest.mark.parametrize("n,copies", [(33, 1), (600, 1), (600, 32)])
+def test_rounding_does_not_depend_on_the_block(n, copies, alpha):
+    """Particles as targets (normalising integral, average, deposition adjoint)
+    at up to half a radius from their node: by differences the weight is off
+    by some ten roundings (2^-53 each; a power a few more), 4e-15, in blocks a
+    thousand radii long and more. A sum about the block's centre would be off by
+    1e-10 there."""
+    tol = 4e-15
+    m, nodes, x = setup(n, 0.1, 0.5, alpha)
+    rng = np.random.default_rng(2)
+    perm = torch.as_tensor(rng.permutation(n), device="cuda")
+    x = x[:, perm].repeat_interleave(copies, 1).contiguous()
+    n = x.shape[1]
+    x[0] += 1e-7 * torch.as_tensor(rng.uniform(-1, 1, n), device="cuda")
+    q = torch.ones(n, dtype=F64, device="cuda")
+    mesh, sf = m.discretization.mesh, m.depositor.shape_function
+    w = torch.as_tensor(np.outer(mesh.jacobians, m.depositor.integral_weights).ravel(),
+                        device="cuda")
+    G = torch.as_tensor(rng.normal(size=len(nodes)), device="cuda")
+    # the node adjoints of a position are summed first, in ascending order, as in
+    # the library (they may cancel)
+    pos, which = np.unique(nodes.cpu().numpy(), axis=0, return_inverse=True)
+    at_pos = np.zeros(len(pos))
+    np.add.at(at_pos, which.ravel(), G.cpu().numpy())
+    pos, at_pos = (torch.as_tensor(a, device="cuda") for a in (pos, at_pos))
+    integral = torch.zeros(n, dtype=F64, device="cuda")
+    lx_want = torch.zeros((3, n), dtype=F64, device="cuda")
+    for c in range(0, n, 2000):
+        d, r2 = pairs(m, nodes, x[:, c:c + 2000])
+        t = torch.clamp(RADIUS - r2 / RADIUS, min=0)
+        integral[c:c + 2000] = w @ (sf.normalizer * t ** alpha)
+        d, r2 = pairs(m, pos, x[:, c:c + 2000])
+        t = torch.clamp(RADIUS - r2 / RADIUS, min=0)
+        lx_want[:, c:c + 2000] = torch.stack(
+            [at_pos @ (sf.normalizer * alpha * (2 / RADIUS) * t ** (alpha - 1) * d[k])
+             for k in range(3)])
+    stats = _lib.DepositStats()
+    deposit(m, _lib.DEPOSIT_NORMALIZED, x, q, stats)
+    scale = 1 / integral
+    assert stats.norm_count == n
+    assert abs(stats.norm_sum - float(scale.sum())) <= tol * float(scale.abs().sum())
+    assert abs(stats.norm_max / float(scale.max()) - 1) <= 4 * tol
+    fields = torch.zeros((6, len(nodes)), dtype=F64, device="cuda")
+    for ordered in (0, 1):
+        out, sc = torch.zeros_like(x), torch.zeros_like(q)
+        ptrs = (C.c_void_p * 6)(*[fields[k].data_ptr() for k in range(6)])
+        _lib.check(m.lib.prt_average_forces_ordered(
+            m.mesh_data.handle, m.workspace, m.depositor._shape_desc(),
+            _lib.ptr(m.depositor.integral_weights), n, x.data_ptr(), q.data_ptr(),
+            out.data_ptr(), None, ptrs, out.data_ptr(), None, sc.data_ptr(), ordered,
+            C.c_void_p(0)))
+        assert float((sc / scale - 1).abs().max()) <= 4 * tol
+    lx = torch.zeros_like(x)
+    _lib.check(m.lib.prt_deposit_shape_adjoint(
+        m.mesh_data.handle, m.workspace, m.depositor._shape_desc(), n, x.data_ptr(),
+        q.data_ptr(), None, None, G.data_ptr(), None, lx.data_ptr(), None, C.c_void_p(0)))
+    err = torch.linalg.norm(lx - lx_want, dim=0) / torch.linalg.norm(lx_want, dim=0)
+    assert float(err.max()) <= 4 * tol
