@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(32 * prt_dep::BW, 3)
   BlockBox X;
   ParticleTargets<PER> D;
   stage_begin(stage);
-  if (!load_particles<PER, SHARE>(D, X, boxes, n, perm, x, el, S)) return;  // whole block
+  const bool any = load_particles<PER, SHARE>(D, X, boxes, n, perm, x, el, S, B, M);
   double vv[3][PER], acc[6][PER];
 #pragma unroll
   for (int h = 0; h < PER; ++h) {
@@ -573,33 +573,34 @@ __global__ void __launch_bounds__(32 * prt_dep::BW, 3)
     for (int k = 0; k < 6; ++k) acc[k][h] = 0;
   }
   const double radius2 = S.radius * S.radius;
-  evaluate_positions<PER, 4, SHARE>(
-      stage, rows, T, B, records, M, X, S.radius, S.inv_radius,
-      [&](double w0, double w1, double w2, const double *g) {
+  if (any)
+    evaluate_positions<PER, 4, SHARE>(
+        stage, rows, T, B, records, M, X, S.radius, S.inv_radius,
+        [&](double w0, double w1, double w2, const double *g) {
 #pragma unroll
-        for (int h = 0; h < PER; ++h) {
-          const double d0 = w0 - D.p[0][h], d1 = w1 - D.p[1][h], d2 = w2 - D.p[2][h];
-          const double t = inside(radius2, d0, d1, d2);
-          // pm = t^(alpha - 1), sv = t^alpha for t > 0 (ALPHA2: by a and a^2 more)
-          double pm, sv;
-          if (ALPHA2) {
-            pm = t > 0 ? t : 0.0;
-            sv = pm * pm;
-          } else {
-            const double ta = t * S.inv_radius;
-            pm = t > 0 ? pow(ta, S.alpha - 1.0) : 0.0;
-            sv = pm * ta;
+          for (int h = 0; h < PER; ++h) {
+            const double d0 = w0 - D.p[0][h], d1 = w1 - D.p[1][h], d2 = w2 - D.p[2][h];
+            const double t = inside(radius2, d0, d1, d2);
+            // pm = t^(alpha - 1), sv = t^alpha for t > 0 (ALPHA2: by a and a^2 more)
+            double pm, sv;
+            if (ALPHA2) {
+              pm = t > 0 ? t : 0.0;
+              sv = pm * pm;
+            } else {
+              const double ta = t * S.inv_radius;
+              pm = t > 0 ? pow(ta, S.alpha - 1.0) : 0.0;
+              sv = pm * ta;
+            }
+            const double hd =
+                pm * fma(g[2], vv[1][h], fma(g[1], vv[0][h], fma(g[3], vv[2][h], g[0])));
+            acc[0][h] = fma(hd, d0, acc[0][h]);
+            acc[1][h] = fma(hd, d1, acc[1][h]);
+            acc[2][h] = fma(hd, d2, acc[2][h]);
+            acc[3][h] = fma(g[1], sv, acc[3][h]);
+            acc[4][h] = fma(g[2], sv, acc[4][h]);
+            acc[5][h] = fma(g[3], sv, acc[5][h]);
           }
-          const double hd =
-              pm * fma(g[2], vv[1][h], fma(g[1], vv[0][h], fma(g[3], vv[2][h], g[0])));
-          acc[0][h] = fma(hd, d0, acc[0][h]);
-          acc[1][h] = fma(hd, d1, acc[1][h]);
-          acc[2][h] = fma(hd, d2, acc[2][h]);
-          acc[3][h] = fma(g[1], sv, acc[3][h]);
-          acc[4][h] = fma(g[2], sv, acc[4][h]);
-          acc[5][h] = fma(g[3], sv, acc[5][h]);
-        }
-      });
+        });
   reduce_groups<PER, 6>(acc);
   if (SHARE) {
     share_sums<6, PER>(stage, acc);

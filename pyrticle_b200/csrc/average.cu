@@ -92,24 +92,25 @@ __global__ void __launch_bounds__(32 * BW, 3)
   BlockBox X;
   ParticleTargets<PER> D;
   stage_begin(A.stage);
-  if (!load_particles<PER, SHARE>(D, X, A.boxes, n, perm, x, el, S)) return;  // whole block
+  const bool any = load_particles<PER, SHARE>(D, X, A.boxes, n, perm, x, el, S, B, M);
   double sum[NV][PER];
 #pragma unroll
   for (int k = 0; k < NV; ++k)
 #pragma unroll
     for (int h = 0; h < PER; ++h) sum[k][h] = 0;
   const double radius2 = S.radius * S.radius;
-  evaluate_positions<PER, NV, SHARE>(
-      A.stage, A.rows, T, B, records, M, X, S.radius, S.inv_radius,
-      [&](double w0, double w1, double w2, const double *g) {
+  if (any)
+    evaluate_positions<PER, NV, SHARE>(
+        A.stage, A.rows, T, B, records, M, X, S.radius, S.inv_radius,
+        [&](double w0, double w1, double w2, const double *g) {
 #pragma unroll
-        for (int h = 0; h < PER; ++h) {
-          const double sw = direct_power<ALPHA2>(
-              inside(radius2, w0 - D.p[0][h], w1 - D.p[1][h], w2 - D.p[2][h]), S);
+          for (int h = 0; h < PER; ++h) {
+            const double sw = direct_power<ALPHA2>(
+                inside(radius2, w0 - D.p[0][h], w1 - D.p[1][h], w2 - D.p[2][h]), S);
 #pragma unroll
-          for (int k = 0; k < NV; ++k) sum[k][h] = fma(sw, g[k], sum[k][h]);
-        }
-      });
+            for (int k = 0; k < NV; ++k) sum[k][h] = fma(sw, g[k], sum[k][h]);
+          }
+        });
   reduce_groups<PER, NV>(sum);
   if (SHARE) {
     share_sums<NV, PER>(A.stage, sum);

@@ -744,7 +744,7 @@ __global__ void __launch_bounds__(32 * BW, 3)
   BlockBox X;
   ParticleTargets<PER> D;
   stage_begin(stage);
-  const bool any = load_particles<PER, SHARE>(D, X, boxes, n, perm, x, el, S);
+  const bool any = load_particles<PER, SHARE>(D, X, boxes, n, perm, x, el, S, B, M);
   double sum[2][PER];  // the integral, and the hits (exact)
   unsigned hits[PER];
 #pragma unroll
@@ -920,6 +920,7 @@ int prt_build_tiles(const double *points, long long count, const uint32_t *ids, 
     const double ext = hi - lo, w = std::max(sum / std::max<long long>(1, nt), 1e-300);
     TB.dims[a] = ext > 0 ? (int)std::max(1.0, std::min(512.0, std::floor(ext / w))) : 1;
     TB.origin[a] = lo;
+    TB.extent[a] = ext;
     TB.inv_w[a] = ext;
   }
   for (;;) {  // (thin or few tiles: no more than some bins per tile)

@@ -42,7 +42,7 @@ struct TileSet {
   // the tiles by the uniform bin of their centre (bins about a tile wide),
   // where asked for: the searches for the tiles near some particles
   struct {
-    double origin[3], inv_w[3], max_half[3];
+    double origin[3], extent[3], inv_w[3], max_half[3];
     int dims[3];
     const uint32_t *starts = nullptr;  // [nbins + 1]
     const uint32_t *tiles = nullptr;   // [tiles], bin order

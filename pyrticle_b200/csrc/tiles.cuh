@@ -461,7 +461,7 @@ __device__ __forceinline__ uint32_t evaluate_particles(BlockStage<NV, false> &S,
 // ------------------------------------------- particles as the targets
 
 struct TileBinsDev {
-  double origin[3], inv_w[3], max_half[3];
+  double origin[3], extent[3], inv_w[3], max_half[3];
   int dims[3];
   const uint32_t *__restrict__ starts, *__restrict__ tiles;
 };
@@ -470,6 +470,7 @@ inline TileBinsDev tile_bins_dev(const TileSet &T) {
   TileBinsDev B;
   for (int d = 0; d < 3; ++d) {
     B.origin[d] = T.bins.origin[d];
+    B.extent[d] = T.bins.extent[d];
     B.inv_w[d] = T.bins.inv_w[d];
     B.max_half[d] = T.bins.max_half[d];
     B.dims[d] = T.bins.dims[d];
@@ -571,13 +572,16 @@ __device__ __forceinline__ void evaluate_positions(BlockStage<NV, true> &S, Tile
 
 // The particles of a warp's lanes as targets: lane (tg, .) holds PER of the 32
 // from k0 (bin order with `perm`, else store order), and the block's and the
-// warp's boxes around the live ones. SHARE: all warps have the same 32.
-// Returns whether the block has a live particle at all.
+// warp's boxes around those within reach of a position. Particles that are not
+// (removed, or outside the mesh by more than the radius and a period, or at no
+// finite place) have zero sums and no part in the boxes: one at infinity would
+// take its whole block's frame there. SHARE: all warps have the same 32.
+// Returns whether the block has a particle within reach at all.
 template <int PER>
 struct ParticleTargets {
   long long id[PER];  // store index, -1 for none
   bool live[PER];
-  double p[3][PER];  // absent and removed particles: beyond every radius
+  double p[3][PER];  // out of reach: beyond every radius
 };
 
 template <int PER, bool SHARE>
@@ -586,7 +590,8 @@ __device__ __forceinline__ bool load_particles(ParticleTargets<PER> &D, BlockBox
                                                const uint32_t *__restrict__ perm,
                                                const double *__restrict__ x,
                                                const uint32_t *__restrict__ el,
-                                               const ShapeWeight &S) {
+                                               const ShapeWeight &S, const TileBinsDev &B,
+                                               const DevMesh &M) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int tg = lane % (32 / PER);
   const long long k0 = 32 * (SHARE ? (long long)blockIdx.x : BW * (long long)blockIdx.x + wid);
@@ -597,12 +602,21 @@ __device__ __forceinline__ bool load_particles(ParticleTargets<PER> &D, BlockBox
     const long long k = k0 + PER * tg + h;
     D.id[h] = k < n ? (perm ? (long long)perm[k] : k) : -1;
     D.live[h] = D.id[h] >= 0 && !(el && el[D.id[h]] == PRT_INVALID);
+    bool near = D.live[h];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      D.p[d][h] = D.live[h] ? x[d * n + D.id[h]] : -FAR;
-      if (D.live[h]) {
+      D.p[d][h] = D.live[h] ? x[d * n + D.id[h]] : 0;
+      const double reach = B.max_half[d] + S.radius * (1 + 1e-5) + (M.pmax[d] - M.pmin[d]);
+      const double from = D.p[d][h] - B.origin[d];
+      near = near && from >= -reach && from <= B.extent[d] + reach;  // (false for a NaN)
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      if (near) {
         lo[d] = fmin(lo[d], D.p[d][h]);
         hi[d] = fmax(hi[d], D.p[d][h]);
+      } else {
+        D.p[d][h] = -FAR;
       }
     }
   }

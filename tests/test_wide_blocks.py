@@ -166,3 +166,49 @@ def test_rounding_does_not_depend_on_the_block(n, copies, alpha):
         q.data_ptr(), None, None, G.data_ptr(), None, lx.data_ptr(), None, C.c_void_p(0)))
     err = torch.linalg.norm(lx - lx_want, dim=0) / torch.linalg.norm(lx_want, dim=0)
     assert float(err.max()) <= 4 * tol
+
+
+@pytest.mark.parametrize("where", [np.inf, -np.inf, np.nan, 1e30, 5.0])
+@pytest.mark.parametrize("copies", [1, 600])
+def test_a_particle_out_of_reach_takes_nothing_from_its_block(where, copies):
+    """Every fifth particle is far outside of the mesh, or at no finite place:
+    it has no position within the radius, and the others, with one each, have
+    their values to the last bit."""
+    m, nodes, good = setup(33, 0.1, 0.5)
+    good = good.repeat(1, copies)
+    n = good.shape[1] * 5 // 4
+    x = torch.empty((3, n), dtype=F64, device="cuda")
+    live = torch.arange(n, device="cuda") % 5 != 4
+    x[:, live] = good[:, :int(live.sum())]
+    x[:, ~live] = torch.tensor([5e-5, where, 0.2], dtype=F64, device="cuda")[:, None]
+    rng = np.random.default_rng(1)
+    G = torch.as_tensor(rng.normal(size=len(nodes)), device="cuda")
+    fields = torch.as_tensor(rng.normal(size=(6, len(nodes))), device="cuda")
+
+    def results(x, ordered):
+        n = x.shape[1]
+        q = torch.ones(n, dtype=F64, device="cuda")
+        lx, f, sc = torch.zeros_like(x), torch.zeros_like(x), torch.zeros_like(q)
+        v = torch.zeros_like(x)
+        ptrs = (C.c_void_p * 6)(*[fields[k].data_ptr() for k in range(6)])
+        _lib.check(m.lib.prt_average_forces_ordered(
+            m.mesh_data.handle, m.workspace, m.depositor._shape_desc(),
+            _lib.ptr(m.depositor.integral_weights), n, x.data_ptr(), q.data_ptr(), v.data_ptr(),
+            None, ptrs, f.data_ptr(), None, sc.data_ptr(), ordered, C.c_void_p(0)))
+        _lib.check(m.lib.prt_deposit_shape_adjoint(
+            m.mesh_data.handle, m.workspace, m.depositor._shape_desc(), n, x.data_ptr(),
+            q.data_ptr(), None, None, G.data_ptr(), None, lx.data_ptr(), None, C.c_void_p(0)))
+        stats = _lib.DepositStats()
+        rho = deposit(m, _lib.DEPOSIT_NORMALIZED, x, q, stats)
+        return lx, f, sc, rho, stats
+
+    for ordered in (0, 1):
+        want = results(x[:, live].contiguous(), ordered)
+        with pytest.warns(UserWarning):  # zero mass, no average
+            got = results(x, ordered)
+        for a, b in zip(got[:3], want[:3]):
+            assert torch.equal(a[..., live], b)
+            assert bool((a[..., ~live] == 0).all())
+        for name in ("norm_count", "norm_min", "norm_max", "el_sum"):
+            assert getattr(got[4], name) == getattr(want[4], name)
+        assert float((got[3] - want[3]).abs().max()) <= 1e-14 * float(want[3].abs().max())
