@@ -876,12 +876,8 @@ extern "C" int prt_deposit_shape_adjoint(const prt_mesh *mesh, prt_workspace *ws
   contract_kernel<<<prt_grid_blocks(PS.count, 256), 256, 0, s>>>(
       T, nn, PS.run_starts, PS.run_nodes, grad_rho, grad_j, records);
   PRT_CHECK_CUDA(cudaGetLastError());
-  prt_dep::BinGrid G;
-  const uint32_t *perm, *starts;
-  if (!prt_dep::choose_bins(mesh, mesh->box_lo, mesh->box_hi,
-                            shape.radius * prt_dep::BIN_FRACTION, 0.0, G, &rc))
-    return rc;
-  if ((rc = prt_dep::bin_particles(ws, G, n, x, el, &perm, &starts, s))) return rc;
+  const uint32_t *perm;
+  if ((rc = prt_dep::order_particles(mesh, ws, shape.radius, n, x, el, &perm, s))) return rc;
   const double *vv = grad_j ? v : nullptr;
   double *lvv = grad_j ? lam_v : nullptr;
   const bool share = n < prt_dep::SHARE_PARTICLES;

@@ -267,13 +267,9 @@ extern "C" int prt_average_forces_ordered(const prt_mesh *mesh, prt_workspace *w
   int rc;
   // a warp's 32 particles have to lie together: in a store without a spatial
   // order the bins' order is taken
-  const uint32_t *perm = nullptr, *starts;
-  if (!ordered) {
-    BinGrid G;
-    if (!choose_bins(mesh, mesh->box_lo, mesh->box_hi, shape.radius * BIN_FRACTION, 0.0, G, &rc))
-      return rc;
-    if ((rc = bin_particles(ws, G, n, positions, elements, &perm, &starts, s))) return rc;
-  }
+  const uint32_t *perm = nullptr;
+  if (!ordered && (rc = order_particles(mesh, ws, shape.radius, n, positions, elements, &perm, s)))
+    return rc;
   Fields6 F;
   for (int k = 0; k < 6; ++k) F.f[k] = fields[k];
   return vis ? average_forces<true>(mesh, ws, shape, integral_weights, n, positions, charges,

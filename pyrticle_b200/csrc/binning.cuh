@@ -67,6 +67,12 @@ __device__ __forceinline__ int floor_div(int a, int b) {
 int choose_bins(const prt_mesh *m, const double lo[3], const double hi[3], double bin_width,
                 double radius, BinGrid &G, int *rc);
 
+// The store index per particle in the order of bins half a radius wide
+// (removed ones last; workspace scratch), without the bins' starts: the
+// neighbours in it lie together, whatever the store's order.
+int order_particles(const prt_mesh *mesh, prt_workspace *ws, double radius, long long n,
+                    const double *x, const uint32_t *el, const uint32_t **perm, cudaStream_t s);
+
 // Bins and sorts the live particles: the store index per particle in bin order
 // (removed ones last) and the bins' starts (workspace scratch).
 int bin_particles(prt_workspace *ws, const BinGrid &G, long long n, const double *x,

@@ -138,9 +138,10 @@ int choose_bins(const prt_mesh *m, const double box_lo[3], const double box_hi[3
   return 1;
 }
 
-int bin_particles(prt_workspace *ws, const BinGrid &G, long long n, const double *x,
-                  const uint32_t *el, const uint32_t **perm, const uint32_t **bin_starts,
-                  cudaStream_t s) {
+// The particles' indices in bin order, and their sorted bins.
+static int sort_by_bin(prt_workspace *ws, const BinGrid &G, long long n, const double *x,
+                       const uint32_t *el, const uint32_t **perm, const uint32_t **sorted,
+                       cudaStream_t s) {
   int rc;
   uint32_t *keys = (uint32_t *)ws_buffer(ws, PRT_WS_DEP_KEYS, 8 * (size_t)n, &rc);
   if (!keys) return rc;
@@ -158,13 +159,32 @@ int bin_particles(prt_workspace *ws, const BinGrid &G, long long n, const double
   if (!temp) return rc;
   PRT_CHECK_CUDA(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys, keys_out, vals,
                                                  vals_out, (int)n, 0, bits, s));
+  *perm = vals_out;
+  *sorted = keys_out;
+  return PRT_OK;
+}
+
+int order_particles(const prt_mesh *mesh, prt_workspace *ws, double radius, long long n,
+                    const double *x, const uint32_t *el, const uint32_t **perm, cudaStream_t s) {
+  BinGrid G;
+  const uint32_t *sorted;
+  int rc;
+  if (!choose_bins(mesh, mesh->box_lo, mesh->box_hi, radius * BIN_FRACTION, 0.0, G, &rc))
+    return rc;
+  return sort_by_bin(ws, G, n, x, el, perm, &sorted, s);
+}
+
+int bin_particles(prt_workspace *ws, const BinGrid &G, long long n, const double *x,
+                  const uint32_t *el, const uint32_t **perm, const uint32_t **bin_starts,
+                  cudaStream_t s) {
+  int rc;
+  const uint32_t *sorted;
+  if ((rc = sort_by_bin(ws, G, n, x, el, perm, &sorted, s))) return rc;
   uint32_t *starts =
       (uint32_t *)ws_buffer(ws, PRT_WS_DEP_BINSTARTS, 4 * (size_t)(G.nbins + 2), &rc);
   if (!starts) return rc;
-  bin_starts_kernel<<<prt_grid_blocks(G.nbins + 1, 256), 256, 0, s>>>(G.nbins, n, keys_out,
-                                                                      starts);
+  bin_starts_kernel<<<prt_grid_blocks(G.nbins + 1, 256), 256, 0, s>>>(G.nbins, n, sorted, starts);
   PRT_CHECK_CUDA(cudaGetLastError());
-  *perm = vals_out;
   *bin_starts = starts;
   return PRT_OK;
 }

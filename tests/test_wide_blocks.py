@@ -212,3 +212,28 @@ def test_a_particle_out_of_reach_takes_nothing_from_its_block(where, copies):
         for name in ("norm_count", "norm_min", "norm_max", "el_sum"):
             assert getattr(got[4], name) == getattr(want[4], name)
         assert float((got[3] - want[3]).abs().max()) <= 1e-14 * float(want[3].abs().max())
+
+
+@pytest.mark.parametrize("call", ["average", "adjoint"])
+def test_scratch_does_not_grow_with_the_bins(call):
+    """The order of the particles needs no array over the bins, a billion here
+    (a radius of a six-hundredth of the box)."""
+    mesh = meshgen.box_mesh((2, 2, 2), (0, 0, 0), (0.01, 0.012, 0.014), seed=7)
+    m = PicMethod(Discretization(mesh, 2), U, NormalizedShapeFunctionDepositor(),
+                  MonomialParticlePusher(), 3, 3)
+    m.depositor.set_shape_function(None, PolynomialShapeFunction(2e-5, 3, 2))
+    x = torch.full((3, 100), 0.005, dtype=F64, device="cuda")
+    q = torch.ones(100, dtype=F64, device="cuda")
+    G = torch.ones(len(m.discretization), dtype=F64, device="cuda")
+    fields = torch.zeros((6, len(G)), dtype=F64, device="cuda")
+    lx = torch.zeros_like(x)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    if call == "average":
+        average(m, x, fields, 0)
+    else:
+        _lib.check(m.lib.prt_deposit_shape_adjoint(
+            m.mesh_data.handle, m.workspace, m.depositor._shape_desc(), 100, x.data_ptr(),
+            q.data_ptr(), None, None, G.data_ptr(), None, lx.data_ptr(), None, C.c_void_p(0)))
+    torch.cuda.synchronize()
+    assert before - torch.cuda.mem_get_info()[0] < 1 << 28
