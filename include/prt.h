@@ -565,10 +565,13 @@ int prt_average_forces(const prt_mesh *mesh, prt_workspace *ws, prt_shape_functi
                        const uint32_t *elements, const double *const fields[6],
                        double *forces, double *vis, double *scales, void *stream);
 
-/* The same for a store whose neighbours lie together (`ordered` != 0: sorted
- * by prt_sort_by_element, or otherwise compact in runs of 32): it is taken in
- * its own order. With 0, as prt_average_forces does, the particles are put in
- * the order of spatial bins first. */
+/* The same with a choice of order. With `ordered` 0, as prt_average_forces
+ * does, the particles are put in the order of spatial bins first. Else the
+ * store is taken in its own order, which is faster where every run of 128
+ * particles is compact against the radius and slower, by any factor, where one
+ * is not: a store sorted by element stops being so when its particles move on
+ * or wrap around a periodic axis, and is not where the mesh's element numbers
+ * have no spatial order. The results are the same to rounding. */
 int prt_average_forces_ordered(const prt_mesh *mesh, prt_workspace *ws, prt_shape_function shape,
                        const double *integral_weights, int64_t n, const double *positions,
                        const double *charges, const double *velocities,

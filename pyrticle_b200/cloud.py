@@ -141,9 +141,6 @@ class PicState:
         self.x, self.p, self.q, self.m, self.el, self.ids = x, p, q, m, el, ids
         self.kx = None
         self.kp = None
-        # the store was sorted by element and not added to since (neighbours
-        # lie together); a hint for speed only
-        self.element_sorted = False
         self.next_id = int(ids.max().item()) + 1 if ids.numel() else 0
         self.derived_quantity_cache = {}
         self.depositor_state = (method.depositor.make_state(self)
@@ -393,7 +390,6 @@ class PicMethod:
         state.el = torch.cat([state.el, el]).contiguous()
         state.ids = torch.cat([state.ids, ids]).contiguous()
         state.kx = state.kp = None
-        state.element_sorted = False
         self.check_containment(state)
         state.particle_number_shift_signaller.note_change_size(len(state))
         state.derived_quantity_cache.clear()
@@ -487,7 +483,6 @@ class PicMethod:
                        vis_listener=state.vis_listener,
                        pnss=state.particle_number_shift_signaller)
         new.next_id = state.next_id
-        new.element_sorted = state.element_sorted
         _lib.check(self.lib.prt_update_containing_elements(
             self.mesh_data.handle, self.workspace, len(new), new.x.data_ptr(),
             new.p.data_ptr(), new.el.data_ptr(), C.c_void_p(stream_handle())),
@@ -558,7 +553,6 @@ class PicMethod:
             kx.data_ptr() if residuals else None, kp.data_ptr() if residuals else None,
             state.ids.data_ptr(), C.c_void_p(stream_handle())),
             "prt_sort_by_element_of")
-        state.element_sorted = True
         state.derived_quantity_cache.clear()
 
 

@@ -265,8 +265,11 @@ extern "C" int prt_average_forces_ordered(const prt_mesh *mesh, prt_workspace *w
     return PRT_ERR_INVALID_ARGUMENT;
   cudaStream_t s = (cudaStream_t)stream;
   int rc;
-  // a warp's 32 particles have to lie together: in a store without a spatial
-  // order the bins' order is taken
+  // A warp evaluates every position near the box of its 32 particles, so these
+  // have to lie together; the bins' order sees to it whatever the store's.
+  // 100,000 particles, five passes a step: 0.93 ms in the middle of a periodic
+  // beam line and 1.09 with the beam across its ends; in the order of a store
+  // sorted before the step 0.72, but 1.29 as soon as particles wrap.
   const uint32_t *perm = nullptr;
   if (!ordered && (rc = order_particles(mesh, ws, shape.radius, n, positions, elements, &perm, s)))
     return rc;

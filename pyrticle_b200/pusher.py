@@ -188,13 +188,12 @@ class AverageParticlePusher(MonomialParticlePusher):
         visbuf = torch.empty((14, n), dtype=torch.float64, device=state.x.device) if vis else None
         scales = torch.empty((n,), dtype=torch.float64, device=state.x.device) if stats else None
         fptrs = self.field_pointers(field_args if field_args else None)
-        _lib.check(self.lib.prt_average_forces_ordered(
+        _lib.check(self.lib.prt_average_forces(
             m.mesh_data.handle, m.workspace, self._shape_desc(),
             _lib.ptr(self.integral_weights), n, state.x.data_ptr(), state.q.data_ptr(),
             velocities.data_ptr(), state.el.data_ptr(), fptrs, out.data_ptr(),
             visbuf.data_ptr() if vis else None, scales.data_ptr() if stats else None,
-            int(state.element_sorted), C.c_void_p(torch.cuda.current_stream().cuda_stream)),
-            "prt_average_forces_ordered")
+            C.c_void_p(torch.cuda.current_stream().cuda_stream)), "prt_average_forces")
         if stats and state.pusher_state is not None and n:
             sc = scales[scales != 0].cpu().numpy()
             for st in (state.pusher_state.e_normalization_stats,
@@ -236,11 +235,11 @@ class AverageParticlePusher(MonomialParticlePusher):
         _lib.check(self.lib.prt_get_velocities(n, state.p.data_ptr(), state.m.data_ptr(), c,
                                                v.data_ptr(), stream), "prt_get_velocities")
         f = torch.empty_like(state.x)
-        _lib.check(self.lib.prt_average_forces_ordered(
+        _lib.check(self.lib.prt_average_forces(
             m.mesh_data.handle, m.workspace, self._shape_desc(),
             _lib.ptr(self.integral_weights), n, state.x.data_ptr(), state.q.data_ptr(),
-            v.data_ptr(), state.el.data_ptr(), fptrs, f.data_ptr(), None, None,
-            int(state.element_sorted), stream), "prt_average_forces_ordered")
+            v.data_ptr(), state.el.data_ptr(), fptrs, f.data_ptr(), None, None, stream),
+            "prt_average_forces")
         _lib.check(self.lib.prt_lsrk_update(
             m.mesh_data.handle, m.workspace, n, state.x.data_ptr(), state.p.data_ptr(),
             state.m.data_ptr(), state.el.data_ptr(), kx.data_ptr(), kp.data_ptr(),
