@@ -393,17 +393,17 @@ __device__ __forceinline__ uint32_t evaluate_particles(BlockStage<NV, false> &S,
   };
   const int ny = max(0, uhi[1] - ulo[1] + 1), nz = max(0, uhi[2] - ulo[2] + 1);
   const long long nrows = (long long)ny * nz;
-  // a row falls into at most four pieces along a periodic x (a block no wider
-  // than the period, a radius below half), else it is one
-  const int pieces = G.periodic[0] ? 4 : 1;
-  const int turn = CHUNK_N / pieces;
+  // along a periodic x a row is in as many pieces as the block's reach has
+  // periods in it (the points of a brick may be any number of periods apart)
+  const int pieces =
+      G.periodic[0] ? floor_div(uhi[0], G.dims[0]) - floor_div(ulo[0], G.dims[0]) + 1 : 1;
   uint32_t evaluated = 0;
-  for (long long r0 = 0; r0 < nrows; r0 += turn) {
-    const int slot = tid / pieces, piece = tid % pieces;
-    const long long r = r0 + slot;
+  for (long long i0 = 0; i0 < nrows * pieces; i0 += CHUNK_N) {
+    const long long r = (i0 + tid) / pieces;
+    const int piece = (int)(i0 + tid - r * pieces);
     uint32_t start = 0, len = 0;
     double sh[3] = {0, 0, 0};
-    if (slot < turn && r < nrows) {
+    if (r < nrows) {
       const int bz = ulo[2] + (int)(r / ny), by = ulo[1] + (int)(r % ny);
       int wz = bz, wy = by, qz = 0, qy = 0;
       if (G.periodic[2]) {
