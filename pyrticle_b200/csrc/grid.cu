@@ -303,6 +303,7 @@ struct prt_grid {
   mutable double *pt_dev = nullptr;
   // the points cut into tiles, for the FP64 deposition (made on its first call)
   mutable TileSet tiles;
+  mutable bool covered = false;  // every grid-node number is a point's
   mutable std::mutex tiles_mutex;
 };
 
@@ -320,7 +321,7 @@ extern "C" int prt_grid_create(const prt_mesh *mesh, const prt_grid_desc *d, prt
   for (int b = 0; b < d->brick_count; ++b) {
     const prt_brick &B = d->bricks[b];
     for (int a = 0; a < 3; ++a)
-      if (B.dims[a] <= 0 || !(B.stepwidths[a] > 0)) {
+      if (B.dims[a] <= 0 || !(B.stepwidths[a] > 0) || B.start_index < 0) {
         delete g;
         return PRT_ERR_INVALID_ARGUMENT;
       }
@@ -439,6 +440,7 @@ static int grid_tiles(const prt_grid *g) {
   if (g->tiles.tiles) return PRT_OK;
   std::vector<double> P;
   std::vector<uint32_t> ids;
+  std::vector<char> used((size_t)g->grid_nodes, 0);
   for (int b = 0; b < g->brick_count; ++b) {
     const prt_brick &B = g->host_bricks[b];
     long long at = B.start_index;
@@ -450,6 +452,7 @@ static int grid_tiles(const prt_grid *g) {
           brick_point(g, b, idx, p);
           P.insert(P.end(), p, p + 3);
           ids.push_back((uint32_t)at);
+          used[(size_t)at] = 1;
         }
   }
   TileSet T;
@@ -459,6 +462,7 @@ static int grid_tiles(const prt_grid *g) {
     return rc;
   }
   g->tiles = T;
+  g->covered = std::find(used.begin(), used.end(), 0) == used.end();
   return PRT_OK;
 }
 
@@ -542,7 +546,7 @@ extern "C" int prt_deposit_grid(const prt_grid *g, prt_workspace *ws, int32_t we
   if (weights == PRT_GRID_SHAPE) {
     if ((rc = grid_tiles(g))) return rc;
     // numbers that no brick uses stay zero
-    if (g->tiles.count != G_n) {
+    if (!g->covered) {
       if (grid_rho) PRT_CHECK_CUDA(cudaMemsetAsync(grid_rho, 0, G_n * sizeof(double), s));
       if (grid_j) PRT_CHECK_CUDA(cudaMemsetAsync(grid_j, 0, 3 * G_n * sizeof(double), s));
     }

@@ -87,3 +87,16 @@ def test_points_several_periods_apart():
     want = g.want()
     assert bool((want > 0).all())
     assert float((g.rho - want).abs().max() / want.max()) <= 1e-12
+
+
+def test_numbers_that_no_point_has_are_zero():
+    """Two bricks with the same numbers (and points) and a gap of as many: there
+    are as many points as numbers, and yet some numbers have none."""
+    sw, dims = (0.001, 0.002, 0.003), (3, 4, 2)
+    g = Grid([(0, sw, (0, 0, 0), dims), (0, sw, (0, 0, 0), dims),
+              (48, sw, (0.005, 0, 0.001), dims)])
+    _lib.check(g.deposit())
+    g.m.check_status()
+    want = g.want()
+    assert bool((g.rho[24:48] == 0).all())
+    assert float((g.rho - want).abs().max() / want.max()) <= 1e-13
