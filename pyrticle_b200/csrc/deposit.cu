@@ -888,6 +888,52 @@ int upload_vec(const std::vector<T> &v, const T **dst) {
 
 // ------------------------------------------------------------------- tiles
 
+namespace {
+
+// Uploads on a stream of their own, complete when finish() returns: a grid's
+// tiles are made in its first deposition, whose caller's stream may be a
+// non-blocking one (the legacy stream's copies are not ordered before it) or be
+// under capture (neither the allocation nor the copy may become part of that;
+// in the relaxed mode they are made at once).
+class Uploader {
+ public:
+  Uploader() {
+    cudaThreadExchangeStreamCaptureMode(&mode_);
+    error_ = cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking);
+  }
+  ~Uploader() {
+    if (stream_) cudaStreamDestroy(stream_);
+    cudaThreadExchangeStreamCaptureMode(&mode_);
+  }
+  Uploader(const Uploader &) = delete;
+  Uploader &operator=(const Uploader &) = delete;
+  // `v` has to live until finish(); *dst is the caller's in any case
+  template <class T>
+  void copy(const std::vector<T> &v, const T **dst) {
+    T *p = nullptr;
+    if (error_ == cudaSuccess)
+      error_ = cudaMalloc(&p, std::max<size_t>(1, v.size()) * sizeof(T));
+    *dst = p;
+    if (error_ == cudaSuccess && !v.empty())
+      error_ = cudaMemcpyAsync(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, stream_);
+  }
+  int finish() {
+    if (stream_) {
+      const cudaError_t e = cudaStreamSynchronize(stream_);
+      if (error_ == cudaSuccess) error_ = e;
+    }
+    PRT_CHECK_CUDA(error_);
+    return PRT_OK;
+  }
+
+ private:
+  cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+  cudaStream_t stream_ = nullptr;
+  cudaError_t error_ = cudaSuccess;
+};
+
+}  // namespace
+
 int prt_build_tiles(const double *points, long long count, const uint32_t *ids, bool bins,
                     TileSet *out) {
   const int TILE_ = prt_dep::TILE;
@@ -919,11 +965,11 @@ int prt_build_tiles(const double *points, long long count, const uint32_t *ids, 
     for (uint32_t &r : rows) r = ids[r];
   out->tiles = nt;
   out->count = count;
-  int rc;
-  if ((rc = upload_vec(rows, &out->rows))) return rc;
-  if ((rc = upload_vec(pos, &out->pos))) return rc;
-  if ((rc = upload_vec(boxes, &out->boxes))) return rc;
-  if (!bins) return PRT_OK;
+  Uploader up;
+  up.copy(rows, &out->rows);
+  up.copy(pos, &out->pos);
+  up.copy(boxes, &out->boxes);
+  if (!bins) return up.finish();
   // bins about as wide as the tiles' mean extent
   auto &TB = out->bins;
   long long nb = 1;
@@ -966,8 +1012,9 @@ int prt_build_tiles(const double *points, long long count, const uint32_t *ids, 
   for (long long b = 0; b < nb; ++b) starts[b + 1] += starts[b];
   std::vector<uint32_t> fill(starts.begin(), starts.end() - 1);
   for (long long t = 0; t < nt; ++t) order[fill[bin[t]]++] = (uint32_t)t;
-  if ((rc = upload_vec(starts, &TB.starts))) return rc;
-  return upload_vec(order, &TB.tiles);
+  up.copy(starts, &TB.starts);
+  up.copy(order, &TB.tiles);
+  return up.finish();
 }
 
 void prt_free_tiles(TileSet *T) {

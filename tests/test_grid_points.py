@@ -100,3 +100,24 @@ def test_numbers_that_no_point_has_are_zero():
     want = g.want()
     assert bool((g.rho[24:48] == 0).all())
     assert float((g.rho - want).abs().max() / want.max()) <= 1e-13
+
+
+def test_first_call_of_a_grid_under_capture():
+    """A grid's tiles are made in its first FP64 deposition, which may be
+    recorded into a CUDA graph as any other where the workspace is warm."""
+    bricks = [(0, (0.001, 0.001, 0.001), (0, 0, 0), (10, 10, 10))]
+    warm, g = Grid(bricks), Grid(bricks)
+    _lib.check(warm.deposit())
+    torch.cuda.synchronize()
+    g.m.workspace, warm.m.workspace = warm.m.workspace, g.m.workspace
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        rc = g.deposit(torch.cuda.current_stream().cuda_stream)
+    assert rc == _lib.PRT_OK
+    assert bool((g.rho == 7.0).all())  # recorded, not run
+    graph.replay()
+    torch.cuda.synchronize()
+    want = g.want()
+    assert float((g.rho - want).abs().max() / want.max()) <= 1e-13
+    assert torch.equal(g.rho, warm.rho)
+    del graph
