@@ -124,7 +124,7 @@ extern "C" int prt_mesh_create(const prt_mesh_desc *d, prt_mesh **out) {
     D.bin_inv[a] = d->bin_inv_width[a];
     D.bin_dims[a] = d->bin_dims[a];
   }
-  if (rc == PRT_OK) rc = prt_mesh_build_positions(m, d);
+  if (rc == PRT_OK) rc = prt_guarded([&] { return prt_mesh_build_positions(m, d); });
   if (rc != PRT_OK) {
     prt_mesh_destroy(m);
     return rc;

@@ -936,31 +936,11 @@ class Uploader {
 
 int prt_build_tiles(const double *points, long long count, const uint32_t *ids, bool bins,
                     TileSet *out) {
-  const int TILE_ = prt_dep::TILE;
-  std::vector<uint32_t> rows((size_t)count);
-  std::iota(rows.begin(), rows.end(), 0u);
-  // blocks of four tiles first, so that a block's tiles lie together
-  const long long block = prt_dep::BW * TILE_;
-  prt_dep::bisect_parallel(points, rows, (uint32_t)block);
-  for (long long b = 0; b < count; b += block)
-    prt_dep::bisect(points, rows, (uint32_t)b, (uint32_t)std::min(count, b + block), TILE_, 0.0,
-                    nullptr);
-  const long long nt = (count + TILE_ - 1) / TILE_;
-  std::vector<double> pos(3 * (size_t)count), boxes(6 * (size_t)nt);
-  for (long long t = 0; t < nt; ++t) {
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (long long r = t * TILE_; r < std::min<long long>(count, (t + 1) * TILE_); ++r)
-      for (int a = 0; a < 3; ++a) {
-        const double x = points[3 * (size_t)rows[r] + a];
-        pos[3 * (size_t)r + a] = x;
-        lo[a] = std::min(lo[a], x);
-        hi[a] = std::max(hi[a], x);
-      }
-    for (int a = 0; a < 3; ++a) {
-      boxes[6 * (size_t)t + a] = 0.5 * (lo[a] + hi[a]);
-      boxes[6 * (size_t)t + 3 + a] = 0.5 * (hi[a] - lo[a]);
-    }
-  }
+  std::vector<uint32_t> rows;
+  std::vector<double> pos, boxes;
+  prt_dep::cut_tiles(points, (size_t)count, prt_dep::TILE, prt_dep::BW * prt_dep::TILE, rows, pos,
+                     boxes);
+  const long long nt = (long long)boxes.size() / 6;
   if (ids)
     for (uint32_t &r : rows) r = ids[r];
   out->tiles = nt;

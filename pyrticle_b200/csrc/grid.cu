@@ -438,8 +438,14 @@ static void brick_point(const prt_grid *g, int b, const int idx[3], double p[3])
 static int grid_tiles(const prt_grid *g) {
   std::lock_guard<std::mutex> lock(g->tiles_mutex);
   if (g->tiles.tiles) return PRT_OK;
+  long long points = 0;
+  for (const prt_brick &B : g->host_bricks)
+    points += (long long)B.dims[0] * B.dims[1] * B.dims[2];
+  if (std::max(points, g->grid_nodes) > 0xffffffffll) return PRT_ERR_CAPACITY;  // 32-bit rows
   std::vector<double> P;
   std::vector<uint32_t> ids;
+  P.reserve(3 * (size_t)points);
+  ids.reserve((size_t)points);
   std::vector<char> used((size_t)g->grid_nodes, 0);
   for (int b = 0; b < g->brick_count; ++b) {
     const prt_brick &B = g->host_bricks[b];
@@ -456,7 +462,8 @@ static int grid_tiles(const prt_grid *g) {
         }
   }
   TileSet T;
-  const int rc = prt_build_tiles(P.data(), (long long)ids.size(), ids.data(), false, &T);
+  const int rc = prt_guarded(
+      [&] { return prt_build_tiles(P.data(), (long long)ids.size(), ids.data(), false, &T); });
   if (rc) {
     prt_free_tiles(&T);
     return rc;
@@ -544,7 +551,7 @@ extern "C" int prt_deposit_grid(const prt_grid *g, prt_workspace *ws, int32_t we
   DepParticles P;
   if ((rc = stage_particles(ws, G, n, x, q, v, el, nullptr, normalizer, tag, P, s))) return rc;
   if (weights == PRT_GRID_SHAPE) {
-    if ((rc = grid_tiles(g))) return rc;
+    if ((rc = prt_guarded([&] { return grid_tiles(g); }))) return rc;
     // numbers that no brick uses stay zero
     if (!g->covered) {
       if (grid_rho) PRT_CHECK_CUDA(cudaMemsetAsync(grid_rho, 0, G_n * sizeof(double), s));

@@ -147,6 +147,17 @@ constexpr double PRT_GROUP_TARGET = 24.0;
 #define PRT_WIDE_CELL_BITS 1
 #endif
 
+// f(), host work on containers, or PRT_ERR_OUT_OF_MEMORY where that ends with an
+// exception: none passes a C entry.
+template <class F>
+int prt_guarded(F &&f) {
+  try {
+    return f();
+  } catch (...) {
+    return PRT_ERR_OUT_OF_MEMORY;
+  }
+}
+
 void *ws_buffer(prt_workspace *ws, int slot, size_t bytes, int *rc);
 int prt_mesh_build_positions(prt_mesh *m, const prt_mesh_desc *d);
 
