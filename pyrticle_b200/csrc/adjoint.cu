@@ -308,7 +308,9 @@ struct BasisList {
 // with its adjoints in registers: a stage reads 52 bytes of the tape (loaded a
 // stage ahead) where a launch per stage moved 260, and the basis projections
 // are reduced once. Field coefficients interleaved ([E][6][COEF_ROW]), the
-// components of `mask`. Same arithmetic per stage as lsrk_stage_adjoint_kernel.
+// components of `mask`. The derivative of lsrk_stage_adjoint_kernel, equal to
+// rounding (one reciprocal root in place of two roots and divisions, the basis
+// projections summed over a field's value).
 // 300,000 particles, order 3, two basis fields: 24 us a stage, with a launch per
 // stage 100.
 template <int ORDER>
@@ -431,7 +433,10 @@ __global__ void __launch_bounds__(ADJ_BLOCK, ORDER >= 4 ? 3 : 4)
                          : comp == 4 ? gB[1]
                                      : gB[2];
 #pragma unroll
-        for (int k = 0; k < PRT_MAX_FIELD_BASIS; ++k) tb[k] = fma(k == base ? g : 0.0, val, tb[k]);
+        for (int k = 0; k < PRT_MAX_FIELD_BASIS; ++k) {
+          // (a zero times another field's infinity would not be nothing)
+          if (k == base) tb[k] = fma(g, val, tb[k]);
+        }
       }
       double w[3];
       {
