@@ -386,6 +386,19 @@ def run_reference(args):
     print(json.dumps(line), flush=True)
 
 
+def sort_launches(n):
+    """Kernels of one prt_sort_by_element_of without residuals, CUB's not counted:
+    iota, and per group of arrays (x, p, q, m, ids; whole arrays, as many as
+    their rows of n doubles fit 64 MB) a gather and a copy back."""
+    fit = min(15, (64 << 20) // (8 * n))
+    groups, rows = 0, 0
+    for r in (3, 3, 1, 1, 1):
+        if groups == 0 or rows + r > fit:
+            groups, rows = groups + 1, 0
+        rows += r
+    return 1 + 2 * groups
+
+
 def adjoint_bench(torch, scale, hbm_gbs, reps=3, checkpoint_every=10):
     """Differentiable workload (16x16x64 cubes, order 3, 1M electrons, 100
     LSRK4 steps, checkpoint every 10): forward (push + final deposition) and
@@ -999,17 +1012,18 @@ def main():
             "fp64": fp64_block, "speedup_mixed_vs_fp64": ms64 / ms,
             "accuracy_mixed_vs_fp64": accuracy}
     # libprt's own kernels in the timed region of the headline form (CUB's
-    # radix-sort kernels not counted): per sort iota + 5 permutation gathers
-    # (x, p, q, m, ids; the residuals are dead at a step boundary); per step one
-    # kernel for the five RK stages (and one per call for the field
-    # coefficients, not counted); per deposition bin keys, bin starts, payload,
-    # the tile work estimate, charges, charge scale, charge digits, the
-    # deposition pass and the expansion to nodes (9), and with the
-    # normalising depositor position weights, their maximum, scale and
-    # digits, the normalisation pass and the two statistics kernels (7).
-    per_dep = 9 + (7 if args.depositor == "normalized" else 0)
-    line["gpu_launches"] = int(kernel["lsrk_stage"][1] + per_dep * kernel["deposit_gather"][1] +
-                               6 * kernel["sort"][1])
+    # radix-sort kernels not counted): per sort those of sort_launches; per step
+    # the field coefficients (where the step reads them) and the five RK stages;
+    # per deposition velocities, bin keys, bin starts, payload, candidate
+    # positions, charges, charge scale, charge digits, the deposition pass and
+    # the expansion to nodes (10), and with the normalising depositor position
+    # weights, their maximum, scale and digits, the normalisation pass and the
+    # two statistics kernels (7).
+    per_dep = 10 + (7 if args.depositor == "normalized" else 0)
+    per_step = 2 if m._use_coefficients(n, 1) else 1
+    line["gpu_launches"] = int(per_step * kernel["lsrk_stage"][1] +
+                               per_dep * kernel["deposit_gather"][1] +
+                               sort_launches(n) * kernel["sort"][1])
     if e2e:
         line["e2e"] = e2e
     if not args.no_adjoint and world == 1:
