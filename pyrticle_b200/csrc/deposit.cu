@@ -459,6 +459,20 @@ struct DepositTargets {
       if (COUNT) hits[h] += __double2hiint(tr) >= 0;
     }
   }
+  // the same for sources whose values may be infinite or NaN
+  __device__ __forceinline__ void within(double w0, double w1, double w2, double e,
+                                         const double *v) {
+#pragma unroll
+    for (int h = 0; h < PER; ++h) {
+      const double tr = fma(V[0][h], w0, fma(V[1][h], w1, fma(V[2][h], w2, B[h] + e)));
+      const double sw = shape_power<ALPHA2>(tr, alpha);
+      if (tr > 0) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sum[k][h] = fma(v[k], sw, sum[k][h]);
+      }
+      if (COUNT) hits[h] += __double2hiint(tr) >= 0;
+    }
+  }
   // adds the tile's pairs, node pairs and evaluated pairs to counters[0..2]
   __device__ __forceinline__ void count(const TilesDev &T, const uint32_t *run_starts,
                                         long long p0, int npt, int tg,

@@ -108,6 +108,10 @@ __device__ __forceinline__ double inside(double radius2, double d0, double d1, d
   return fma(-d0, d0, fma(-d1, d1, fma(-d2, d2, radius2)));
 }
 
+__device__ __forceinline__ bool not_finite(double v) {
+  return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000;
+}
+
 // The weight (t)^alpha for t > 0, else 0.
 template <bool ALPHA2>
 __device__ __forceinline__ double shape_power(double t, double alpha) {
@@ -243,6 +247,9 @@ struct BlockBox {
 // before a barrier) against the block's tiles: op(w0, w1, w2, e, v), DIRECT
 // op(x, y, z, v), on every lane with its group's entry.
 // SHARE: the warps have the same tile and take 32 of a chunk's entries each.
+// A chunk with an entry whose values are not all finite goes through op.within
+// (not DIRECT), which adds nothing where the weight is zero: a weight of zero
+// times infinity would spoil targets beyond the radius.
 // Returns the entries evaluated (per warp). Ends with a barrier.
 template <int PER, int NV, bool SHARE, bool DIRECT, class Op>
 __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV, DIRECT> &S,
@@ -306,8 +313,11 @@ __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV, DIRECT> &S,
         }
         const double w0 = v[0] + S.shift[seg0][0], w1 = v[1] + S.shift[seg0][1],
                      w2 = v[2] + S.shift[seg0][2];
+        bool odd = false;
+#pragma unroll
+        for (int k = 3; k < 3 + NV; ++k) odd = odd || not_finite(v[k]);
         S.w[st][tid] = make_float4((float)(w0 * inv_radius), (float)(w1 * inv_radius),
-                                   (float)(w2 * inv_radius), 0);
+                                   (float)(w2 * inv_radius), odd ? 1.0f : 0.0f);
         S.e[st][0][tid] = make_double2(w0, w1);
         S.e[st][1][tid] = make_double2(w2, -(w0 * w0 + w1 * w1 + w2 * w2) * inv_radius);
 #pragma unroll
@@ -324,6 +334,7 @@ __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV, DIRECT> &S,
     seg0 = seg1;
     seg1 = seg;
     int n = 0;
+    bool odd = false;
 #pragma unroll
     for (int q = 0; q < BW; ++q) {
       if (SHARE && q != wid) continue;
@@ -335,11 +346,28 @@ __device__ __forceinline__ uint32_t evaluate_segments(BlockStage<NV, DIRECT> &S,
       const unsigned bal = __ballot_sync(0xffffffffu, in);
       if (in) list[n + __popc(bal & ((1u << lane) - 1u))] = (uint8_t)(32 * q + lane);
       n += __popc(bal);
+      if (!DIRECT) odd = odd || (in && w.w != 0);
     }
     // up to a whole turn with entries beyond every radius
     if (lane < PER) list[n + lane] = CHUNK_N;
     __syncwarp();
     evaluated += n;
+    if constexpr (!DIRECT) {
+      if (__any_sync(0xffffffffu, odd)) {
+#pragma unroll 1
+        for (int i = 0; i < n; i += PER) {
+          double v[2 * ST::W];
+#pragma unroll
+          for (int w = 0; w < ST::W; ++w) {
+            const double2 t = S.e[st][w][list[i + grp]];
+            v[2 * w] = t.x;
+            v[2 * w + 1] = t.y;
+          }
+          op.within(v[0], v[1], v[2], v[3], v + 4);
+        }
+        n = 0;
+      }
+    }
     int id = list[grp];
 #pragma unroll 2
     for (int i = 0; i < n; i += PER) {
