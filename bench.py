@@ -164,8 +164,8 @@ def timing_read(m, cat, reset=True):
 # profiles/dram_traffic_config2_16M.md); reported only for that workload.
 MEASURED_TRAFFIC = {
     "config2": {
-        "tc_deposit_kernel<0, 0>": 1486009600 + 119841792,
-        "tc_deposit_kernel<1, 1>": 1075521536 + 520001792,
+        "tc_deposit_kernel<0, 0>": 2381106944 + 134500864,
+        "tc_deposit_kernel<1, 1>": 1426282752 + 771363328,
     }
 }
 
