@@ -371,6 +371,8 @@ extern "C" int prt_grid_create(const prt_mesh *mesh, const prt_grid_desc *d, prt
         rc = PRT_ERR_INVALID_ARGUMENT;
     }
     const size_t tot = d->eog_starts[d->eog_count];
+    for (size_t i = 0; i < tot && !rc; ++i)
+      if (d->eog_grid_nodes[i] >= (uint64_t)gn) rc = PRT_ERR_INVALID_ARGUMENT;
     const size_t mtot = d->eog_matrix_starts[d->eog_count];
     if (!rc) rc = up(&g->eog_elements, d->eog_elements, d->eog_count);
     if (!rc) rc = up(&g->eog_starts, d->eog_starts, d->eog_count + 1);

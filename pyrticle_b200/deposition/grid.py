@@ -174,7 +174,9 @@ def find_points_in_elements(mesh, bricks, el_tolerance, chunk=20000):
         ihi_box = np.minimum(ehi, bhi)
         nonempty = np.all(ilo_box < ihi_box, axis=1)
         lo_i = np.floor((ilo_box - brk.origin) / brk.stepwidths).astype(np.int64)
-        hi_i = np.ceil((ihi_box - brk.origin) / brk.stepwidths).astype(np.int64)
+        # (dims * h / h may round to more than dims: no layer beyond the last)
+        hi_i = np.minimum(np.ceil((ihi_box - brk.origin) / brk.stepwidths).astype(np.int64),
+                          brk.dims)
         ext = np.where(nonempty[:, None], np.maximum(hi_i - lo_i, 0), 0)
         mx = ext.max(axis=0)
 
